@@ -6,8 +6,9 @@ method vectors in shared memory), on the order in which the persistent work queu
 cells and how many it hands out per atomic (the refill chunk), and on how many cells a warp
 integrates at once (32, one per thread; or 1, with species and reactions over the lanes).  The
 tuner times a sample of the caller's own cells under
-  (threads per block, blocks per SM) x (longest-first | index order), then refill chunks on
-  the best of those, then one warp per cell,
+  (threads per block, blocks per SM) x (longest-first | index order), (0, 0) standing for the
+  library's own choice (a group of lanes per cell or one thread per cell, by the batch's size),
+  then refill chunks on the best of those, then one warp per cell,
 keeps the fastest, and records the choice in a versioned JSON file keyed by mechanism, device
 and workload tag, so later runs reuse it without timing.
 """
@@ -18,8 +19,8 @@ import time
 
 from . import lib, check
 
-CACHE_VERSION = 2
-SHAPES = [(256, 1), (224, 1), (192, 1), (160, 1), (128, 1), (128, 2), (96, 2), (64, 2), (64, 3)]
+CACHE_VERSION = 3
+SHAPES = [(0, 0), (256, 1), (224, 1), (192, 1), (160, 1), (128, 1), (128, 2), (96, 2), (64, 2), (64, 3)]
 ORDERS = {"longest-first": 0, "index": 8}
 CHUNKS = [128, 1024]          # refill chunks tried on the best shape (0: exactly the lanes that need a cell)
 WARP_PER_CELL = 16            # GDTK_CHEM_WARP_PER_CELL

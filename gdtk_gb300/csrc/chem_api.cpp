@@ -262,6 +262,12 @@ void run_fast(ReactorObj& r, FastArgs& a, int flags, cudaStream_t s) {
         a.order = r.order.p;
     }
     check(cudaMemsetAsync(r.counter, 0, sizeof(unsigned), s), "cudaMemsetAsync");
+    const int lanes = r.req_block > 0 || r.lane_stats ? 0 : group_lanes(*r.fast, a.total, cuda().sm_count);
+    if (lanes) {
+        check(launch_group(*r.fast, a, lanes, cuda().sm_count, s, &r.last.grid, &r.last.block, &r.last.smem),
+              "chemistry update launch");
+        return;
+    }
     check(launch_fast(*r.fast, a, cuda().sm_count, s, &r.last.grid, &r.last.block, &r.last.smem),
           "chemistry update launch");
     r.last.blocks_per_sm = r.fast->blocks_per_sm;
@@ -501,7 +507,9 @@ int update_cells_with_scratch(int cr_i, int ncell, const double* rho, const doub
         }
         check(cudaMemsetAsync(counter, 0, sizeof(unsigned), s), "cudaMemsetAsync");
         int grid = 0, block = 0, smem = 0;
-        check(launch_fast(*r.fast, a, cuda().sm_count, s, &grid, &block, &smem), "chemistry update launch");
+        const int lanes = r.req_block > 0 ? 0 : group_lanes(*r.fast, a.total, cuda().sm_count);
+        check(lanes ? launch_group(*r.fast, a, lanes, cuda().sm_count, s, &grid, &block, &smem)
+                    : launch_fast(*r.fast, a, cuda().sm_count, s, &grid, &block, &smem), "chemistry update launch");
         return 0;
     });
 }
@@ -856,8 +864,8 @@ int thermochemical_reactor_gas_state_update(int cr_i, int gs_i, double t_interva
         double* d = r.stage.d.p;
         check(cudaMemcpyAsync(d, h.data(), nd * sizeof(double), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
         // ThermochemicalReactor.opCall alone: no retry and no rhou update (gas_cwrap.d:906-921).
-        launch_update(r, 1, d + 0, d + 1, d + 2, d + 3, d + 5, d + 4, r.stage.st.p, t_interval, -1.0e300,
-                      GDTK_CHEM_REFERENCE_ORDER, st, nullptr, nullptr);
+        launch_update(r, 1, d + 0, d + 1, d + 2, d + 3, d + 5, d + 4, r.stage.st.p, t_interval, -1.0e300, 0, st, nullptr,
+                      nullptr);
         int status = 0;
         check(cudaMemcpyAsync(h.data(), d, nd * sizeof(double), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         check(cudaMemcpyAsync(&status, r.stage.st.p, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
@@ -1146,7 +1154,7 @@ int chem_reactor_last_launch(int cr_i, int* grid, int* block, int* smem_bytes, i
 const char* gdtk_last_error(void) { return g_last_error.c_str(); }
 
 int gdtk_exp_host(int n, const double* x, double* y) {
-    static const double tab[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
+    static const uint64_t tab[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
     for (int i = 0; i < n; ++i) y[i] = gdtk_exp(x[i], tab);
     return 0;
 }

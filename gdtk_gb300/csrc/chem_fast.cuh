@@ -43,8 +43,7 @@ namespace gdtk_fast {
 
 using gdtk::gdtk_exp;
 using gdtk::gdtk_div;
-using gdtk::gdtk_div_nr;
-using gdtk::gdtk_add_div;
+using gdtk::gdtk_rcp;
 
 // must match the host's CellBlock / FastArgs (codegen.h)
 struct CellBlock {
@@ -66,7 +65,7 @@ struct CellBlock {
 // launch needs no device-side table and a captured graph replays it exactly.
 struct FastArgs {
     const double* thermo;
-    const double* exp_table;
+    const uint64_t* exp_table;
     int nblocks;
     int total;
     int flags;
@@ -282,13 +281,53 @@ __device__ __forceinline__ double ln_step(double lnT, double x, double T) {
     return log(T);
 }
 
-// *lnT_io: ln T_guess on entry, ln of the returned T on exit.  ysum = sum_i Y_i R_i, added in species order.
+// One Newton correction applied: T, ln T and 1 / T for T + dT; true when |dT| / T < TOL
+// (therm_perf_gas_mix.d:452, with the reciprocal the next iteration needs).
+__device__ __forceinline__ bool newton_advance(double& T, double& lnT, double& rT, double dT) {
+    const double TOL = 1e-10;
+    const double x = dT * rT;   // dT / T of the previous iterate
+    T += dT;
+    lnT = ln_step(lnT, x, T);
+    rT = gdtk_rcp(T);
+    return lt_pos(abs_bits(dT) * rT, TOL);
+}
+#if GDTK_MIX_THERMO
+// f = sum Y_i (h_i - R_i T) and cv = sum Y_i (Cp_i - R_i) from the mixture coefficients ma (and mb, blended by wb)
+__device__ __forceinline__ void mix_f_cv(const double* ma, const double* mb, int ys, double T, double lnT, double rT,
+                                         double rT2, double wb, double ysum, double& f, double& cv) {
+    double H, C;
+    mix_H_Cp(ma, ys, T, lnT, rT, rT2, H, C);
+    if (nonzero(wb)) {
+        double Hb, Cb;
+        mix_H_Cp(mb, ys, T, lnT, rT, rT2, Hb, Cb);
+        H = fma(wb, Hb - H, H);
+        C = fma(wb, Cb - C, C);
+    }
+    f = fma(-ysum, T, H);
+    cv = C - ysum;
+}
+#endif
+// the same as sums over the species
+__device__ __forceinline__ void species_f_cv(const double* TH, const double* YR, int ys, double T, double lnT, double rT,
+                                             double rT2, double& f, double& cv, int& err) {
+#pragma unroll 1
+    for (int i = 0; i < GDTK_NSP; ++i) {
+        double H, Cp;
+        int e = 0;
+        sp_H_Cp(TH, i, T, lnT, rT, rT2, H, Cp, e);
+        if (e) err = e;
+        const double yr = YR[i * ys];
+        f = fma(yr, H - T, f);
+        cv = fma(yr, Cp - 1.0, cv);
+    }
+}
+
+// *lnT_io: ln T_guess on entry, ln of the returned T on exit.  ysum = sum_i Y_i R_i.
 // S: 24 doubles (stride ys) of scratch for the mixture coefficients.
 __device__ __noinline__ double T_from_u(const double* TH, const double* YR, int ys, double* S, double u_tgt,
                                         double T_guess, double ysum, double* lnT_io, int* err, int* iters,
                                         unsigned long long* lst) {
-    const double TOL = 1e-10;
-    double T = T_guess, dT = 0.0, lnT = *lnT_io, rT = gdtk_div(1.0, T);
+    double T = T_guess, dT = 0.0, lnT = *lnT_io, rT = gdtk_rcp(T);
 #if GDTK_MIX_THERMO
     double* ma = S;
     double* mb = S + 12 * ys;
@@ -300,12 +339,7 @@ __device__ __noinline__ double T_from_u(const double* TH, const double* YR, int 
     for (int it = 0; it <= 10; ++it) {
         lane_stat(lst, 4);
         if (it > 0) {
-            const double x = dT * rT;   // dT / T of the previous iterate
-            T += dT;
-            lnT = ln_step(lnT, x, T);
-            // |dT| / T < TOL (therm_perf_gas_mix.d:452) with the reciprocal the next iteration needs
-            rT = gdtk_div(1.0, T);
-            if (lt_pos(abs_bits(dT) * rT, TOL)) { *lnT_io = lnT; return T; }
+            if (newton_advance(T, lnT, rT, dT)) { *lnT_io = lnT; return T; }
             if (it == 10) break;
         }
         const double rT2 = rT * rT;
@@ -315,32 +349,12 @@ __device__ __noinline__ double T_from_u(const double* TH, const double* YR, int 
         double wb = 0.0;
         if (in_mix_range(T) && seg_of(TH, T, sa, sb, wb)) {
             if (sa != seg_a) { mix_coeffs(TH, YR, ys, sa, ma); seg_a = sa; }
-            double H, C;
-            mix_H_Cp(ma, ys, T, lnT, rT, rT2, H, C);
-            if (nonzero(wb)) {
-                if (sb != seg_b) { mix_coeffs(TH, YR, ys, sb, mb); seg_b = sb; }
-                double Hb, Cb;
-                mix_H_Cp(mb, ys, T, lnT, rT, rT2, Hb, Cb);
-                H = fma(wb, Hb - H, H);
-                C = fma(wb, Cb - C, C);
-            }
-            f = fma(-ysum, T, H);
-            cv = C - ysum;
+            if (nonzero(wb) && sb != seg_b) { mix_coeffs(TH, YR, ys, sb, mb); seg_b = sb; }
+            mix_f_cv(ma, mb, ys, T, lnT, rT, rT2, wb, ysum, f, cv);
         } else
 #endif
-        {
-#pragma unroll 1
-            for (int i = 0; i < GDTK_NSP; ++i) {
-                double H, Cp;
-                int e = 0;
-                sp_H_Cp(TH, i, T, lnT, rT, rT2, H, Cp, e);
-                if (e) *err = e;
-                const double yr = YR[i * ys];
-                f = fma(yr, H - T, f);
-                cv = fma(yr, Cp - 1.0, cv);
-            }
-        }
-        dT = -gdtk_div_nr(f - u_tgt, cv);
+            species_f_cv(TH, YR, ys, T, lnT, rT, rT2, f, cv, *err);
+        dT = -gdtk_div(f - u_tgt, cv);
         ++*iters;
     }
     if (gt_pos(abs_bits(dT), 1e-3)) *err = ST_NEWTON;
@@ -382,11 +396,11 @@ __device__ __forceinline__ double sum_pairwise(F d) {
 // G: scratch of GDTK_NSP slots (stride ks); the third-body concentrations of the pressure-dependent
 // rate constants (gen_falloff_M) are read from the GDTK_NFALLOFF slots after it.
 __device__ __noinline__ void rate_constants(const double* TH, double Tq, double lnTq, double* K, int ks,
-                                            const double* etab, double* G, int* err) {
+                                            const uint64_t* etab, double* G, int* err) {
     double T = Tq, lnT = lnTq;   // lnTq = ln Tq
     if (lt_pos(T, GDTK_T_LOWER)) { T = GDTK_T_LOWER; lnT = GDTK_LN_T_LOWER; }
     if (gt_pos(T, GDTK_T_UPPER)) { T = GDTK_T_UPPER; lnT = GDTK_LN_T_UPPER; }
-    const double rT = gdtk_div(1.0, T), rT2 = rT * rT, t1 = lnT + 1.0, t2 = 1.0 - lnT;
+    const double rT = gdtk_rcp(T), rT2 = rT * rT, t1 = lnT + 1.0, t2 = 1.0 - lnT;
     int e = 0;
 #if GDTK_MIX_THERMO
     // every species takes the same curve segment and blend here: choose them once
@@ -410,20 +424,23 @@ __device__ __noinline__ void rate_constants(const double* TH, double Tq, double 
     gen_kc(T, lnT, rT, G, ks, K, ks, etab, G + GDTK_NSP * ks, ks);
 }
 
-// reaction_mechanism.d:161-203 from the rates at c.
+// reaction_mechanism.d:161-203 from the rates at c: one species' time scale, then the limits.
+__device__ __forceinline__ double estimate_of(double c, double q, double L, double min_dt) {
+    if (c > 0.0 && fabs(q - L) > 1.0e-30) {
+        const double dt = (q > 10000.0 * L) ? gdtk_div(c, L + ZERO_EPS) : fabs(gdtk_div(c, q - L));
+        min_dt = fmin(min_dt, dt);
+    }
+    return min_dt;
+}
+__device__ __forceinline__ double estimate_clip(double min_dt) {
+    return fmax(fmin(1.0e-3 * min_dt, 1.0e-10), 1.0e-15);
+}
 __device__ __forceinline__ double estimate_step(const double (&c)[GDTK_NSP], const double (&q)[GDTK_NSP],
                                                 const double (&L)[GDTK_NSP]) {
     double min_dt = 1.0e6;
 #pragma unroll
-    for (int i = 0; i < GDTK_NSP; ++i) {
-        if (c[i] > 0.0 && fabs(q[i] - L[i]) > 1.0e-30) {
-            double dt = (q[i] > 10000.0 * L[i]) ? gdtk_div(c[i], L[i] + ZERO_EPS) : fabs(gdtk_div(c[i], q[i] - L[i]));
-            min_dt = fmin(min_dt, dt);
-        }
-    }
-    double dt_chem = 1.0e-3 * min_dt;
-    dt_chem = fmin(dt_chem, 1.0e-10);
-    return fmax(dt_chem, 1.0e-15);
+    for (int i = 0; i < GDTK_NSP; ++i) min_dt = estimate_of(c[i], q[i], L[i], min_dt);
+    return estimate_clip(min_dt);
 }
 
 // alpha = N/D (chemistry_update.d:599-604) as N(s)/D(s), s = p h, the reference's rational
@@ -437,6 +454,57 @@ __device__ __forceinline__ void alpha_nd(double s, double& N, double& D) {
     D = fma(s, s, N + 180.0);   // s^3 + 12 s^2 + 60 s + 360 = N + s^2 + 180
 }
 
+// The predictor's (q0 = q, pb = p) or corrector's value of a species: y + h (N (q - q0) + D (q0 - pb y)) / (N h pb + D)
+__device__ __forceinline__ double qss_value(double y, double pp, double h, double q, double q0, double pb) {
+    double N, D;
+    alpha_nd(pp * h, N, D);
+    const double num = h * fma(N, q - q0, D * fma(-pb, y, q0));
+    return y + gdtk_div(num, fma(N, h * pb, D));
+}
+__device__ __forceinline__ bool qss_misses(double v, double yp0) {
+    return !lt_pos(v, ZERO_EPS) && ge_nn(abs_bits(v - yp0), fma(GDTK_EPS1, v, GDTK_EPS1 * GDTK_DELTA));
+}
+// sigma = max_i |yc - yp0| / (eps2 (yc + delta)): the largest ratio by comparing cross products (denominators
+// are positive) in a pairwise tree over the species, then one division
+struct Ratio { double num, den; };
+__device__ __forceinline__ Ratio larger_ratio(Ratio a, Ratio b) {   // a unless b's is larger
+    return gt_nn(b.num * a.den, a.num * b.den) ? b : a;
+}
+__device__ __forceinline__ Ratio sigma_leaf(double yc, double yp0) {
+    const double num = abs_bits(yc - yp0);
+    if (lt_pos(yc, ZERO_EPS) || dbits(num) > INF_BITS) return Ratio{0.0, 1.0};   // absent, or NaN
+    return Ratio{num, fma(GDTK_EPS2, yc, GDTK_EPS2 * GDTK_DELTA)};
+}
+template <int LO, int N, typename F>
+__device__ __forceinline__ Ratio tree_max_ratio(F leaf) {   // N a power of two; species beyond GDTK_NSP are absent
+    if constexpr (N == 1) {
+        return leaf(LO);
+    } else {
+        const Ratio a = tree_max_ratio<LO, N / 2>(leaf);
+        if constexpr (LO + N / 2 >= GDTK_NSP) return a;
+        else return larger_ratio(a, tree_max_ratio<LO + N / 2, N / 2>(leaf));
+    }
+}
+constexpr int tree_width(int n) { int p = 1; while (p < n) p *= 2; return p; }
+__device__ __forceinline__ double qss_step(Ratio sg, double h) {
+    const double sigma = gdtk_div(sg.num, sg.den);
+    if (!nonzero(sigma)) return 10.0 * h;   // sigma <= 0 (sigma is >= 0 or NaN)
+    double x = sigma;
+    x = fma(-0.5, gdtk_div(fma(x, x, -sigma), x), x);
+    x = fma(-0.5, gdtk_div(fma(x, x, -sigma), x), x);
+    x = fma(-0.5, gdtk_div(fma(x, x, -sigma), x), x);
+    return h * (gdtk_rcp(x) + 0.005);
+}
+// Y_i of a concentration, below 1e-30 zero
+__device__ __forceinline__ double clipped_massf(double c, double M, double rrho) {
+    const double v = __dmul_rn(__dmul_rn(c, M), rrho);   // not contracted into the sums: the same in every kernel
+    return lt_pos(v, 1.0e-30) ? 0.0 : v;
+}
+// the next step after an accepted one: the suggestion, at most 10% larger, if it grows
+__device__ __forceinline__ double grown_step(double h, double dtS) {
+    return (dbits(dtS) > dbits(h) && dbits(dtS) <= INF_BITS) ? min_pos(dtS, h * 1.1) : h;   // h > 0
+}
+
 // ---------------------------------------------------------------- the kernel
 #if GDTK_METHOD == 0
 // Cash-Karp stage coefficients a[s][j] (stage s + 1 from k_1..k_s), chemistry_update.d:409-412
@@ -446,6 +514,21 @@ __constant__ double RKF_A[5][5] = {
     {3. / 10., -9. / 10., 6. / 5., 0, 0},
     {-11. / 54., 5. / 2., -70. / 27., 35. / 27., 0},
     {1631. / 55296., 175. / 512., 575. / 13824., 44275. / 110592., 253. / 4096.}};
+// the fifth-order result of a species and its error over the tolerance
+__device__ __forceinline__ void rkf_result(double K1, double K3, double K4, double K5, double K6, double h, double y0,
+                                           double& o, double& e) {
+    const double b51 = 37. / 378., b53 = 250. / 621., b54 = 125. / 594., b56 = 512. / 1771., b41 = 2825. / 27648.,
+                 b43 = 18575. / 48384., b44 = 13525. / 55296., b45 = 277. / 14336., b46 = 1.0 / 4.0;
+    o = fma(h, fma(b56, K6, fma(b54, K4, fma(b53, K3, b51 * K1))), y0);
+    const double o4 = fma(h, fma(b46, K6, fma(b45, K5, fma(b44, K4, fma(b43, K3, b41 * K1)))), y0);
+    e = gdtk_div(o - o4, fma(GDTK_ERRTOL, fmax(fabs(y0), fabs(o)), GDTK_ERRTOL));
+}
+// the step-size factor of the scaled error norm; ok: the step is accepted
+__device__ __forceinline__ double rkf_scale(double errn, const uint64_t* etab, bool& ok) {
+    ok = errn <= 1.0;
+    if (ok) return (errn == 0.0) ? 10.0 : fmin(fmax(0.9 * gdtk_exp(-0.2 * log(errn), etab), 0.2), 10.0);
+    return fmax(0.9 * gdtk_exp(-0.2 * log(errn), etab), 0.2);
+}
 #endif
 // GDTK_VEC (per-thread method vector, doubles) comes from the generator: the method's stage
 // storage, at least nsp + 16 when T(rho, u) uses mixture coefficients
@@ -453,9 +536,9 @@ __constant__ double RKF_A[5][5] = {
 extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_chem_fast(const __grid_constant__ FastArgs a) {
     extern __shared__ double smem[];
     double* TH = smem;                                   // thermo table, nsp * stride
-    double* ETAB = smem + GDTK_NSP * GDTK_TH_STRIDE;     // exp table, GDTK_EXP2_TABLE_SIZE
+    uint64_t* ETAB = reinterpret_cast<uint64_t*>(smem + GDTK_NSP * GDTK_TH_STRIDE);     // exp table, GDTK_EXP2_TABLE_SIZE
     const CellBlock* BLK = a.blocks;
-    double* S = ETAB + GDTK_EXP2_TABLE_SIZE;             // per-thread vectors
+    double* S = smem + GDTK_NSP * GDTK_TH_STRIDE + GDTK_EXP2_TABLE_SIZE;             // per-thread vectors
     for (int k = threadIdx.x; k < GDTK_NSP * GDTK_TH_STRIDE; k += blockDim.x) TH[k] = a.thermo[k];
     for (int k = threadIdx.x; k < GDTK_EXP2_TABLE_SIZE; k += blockDim.x) ETAB[k] = a.exp_table[k];
     __syncthreads();
@@ -528,7 +611,7 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                     } else {
                         have = true;
                         retried = false;
-                        rrho = gdtk_div(1.0, rho);
+                        rrho = gdtk_rcp(rho);
                         n_steps = n_rhs = n_kc = n_newton = n_rej = n_est = 0;
                         phase = -1;
                     }
@@ -585,7 +668,13 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                     cycle = 0;
                     phase = 1;
                 }
-                if (phase == 1) { dtSave = dtS; h = fmin(h, tI - t); attempt = 0; phase = 2; }
+                if (phase == 1) {
+                        dtSave = dtS;
+                        const double left = tI - t;
+                        h = lt_pos(h, left) ? h : left;
+                        attempt = 0;
+                        phase = 2;
+                    }
             }
             double* kv = V + s * GDTK_NSP * ks;
 #pragma unroll
@@ -598,34 +687,16 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                     yn[i] = fma(h, acc, y0[i]);
                 }
             } else {
-                const double b51 = 37. / 378., b53 = 250. / 621., b54 = 125. / 594., b56 = 512. / 1771.,
-                    b41 = 2825. / 27648., b43 = 18575. / 48384., b44 = 13525. / 55296., b45 = 277. / 14336.,
-                    b46 = 1.0 / 4.0;
-                double err2 = 0.0;
-#pragma unroll
-                for (int i = 0; i < GDTK_NSP; ++i) {
-                    double K1 = V[i * ks], K3 = V[(2 * GDTK_NSP + i) * ks], K4 = V[(3 * GDTK_NSP + i) * ks],
-                           K5 = V[(4 * GDTK_NSP + i) * ks], K6 = V[(5 * GDTK_NSP + i) * ks];
-                    double o = fma(h, fma(b56, K6, fma(b54, K4, fma(b53, K3, b51 * K1))), y0[i]);
-                    double o4 = fma(h, fma(b46, K6, fma(b45, K5, fma(b44, K4, fma(b43, K3, b41 * K1)))), y0[i]);
-                    double sk = fma(GDTK_ERRTOL, fmax(fabs(y0[i]), fabs(o)), GDTK_ERRTOL);
-                    double e = gdtk_div(o - o4, sk);
-                    err2 = fma(e, e, err2);
+                errn = sqrt(sum_pairwise([&](int i) {
+                    double o, e;
+                    rkf_result(V[i * ks], V[(2 * GDTK_NSP + i) * ks], V[(3 * GDTK_NSP + i) * ks], V[(4 * GDTK_NSP + i) * ks],
+                               V[(5 * GDTK_NSP + i) * ks], h, y0[i], o, e);
                     yn[i] = o;
-                }
-                errn = sqrt(err2 * (1.0 / GDTK_NSP));
+                    return __dmul_rn(e, e);
+                }) * (1.0 / GDTK_NSP));
             }
         }
-        {
-            double scale;
-            if (errn <= 1.0) {
-                scale = (errn == 0.0) ? 10.0 : fmin(fmax(0.9 * gdtk_exp(-0.2 * log(errn), ETAB), 0.2), 10.0);
-                ok = true;
-            } else {
-                scale = fmax(0.9 * gdtk_exp(-0.2 * log(errn), ETAB), 0.2);
-            }
-            dtS = scale * h;
-        }
+        dtS = rkf_scale(errn, ETAB, ok) * h;
 #else
         // alpha-QSS, chemistry_update.d:533-655.  Iteration 0 is the predictor, 1..maxIters the
         // correctors; with q0 = q and p0 = p the corrector formula reduces to the predictor's, so
@@ -655,52 +726,35 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                         cycle = 0;
                         phase = 1;
                     }
-                    if (phase == 1) { dtSave = dtS; h = fmin(h, tI - t); attempt = 0; phase = 2; }
+                    if (phase == 1) {
+                        dtSave = dtS;
+                        const double left = tI - t;
+                        h = lt_pos(h, left) ? h : left;
+                        attempt = 0;
+                        phase = 2;
+                    }
                 }
                 conv = true;
 #pragma unroll
                 for (int i = 0; i < GDTK_NSP; ++i) {
                     const double y = y0[i];
                     const double ci_ = (s == 0) ? y : yn[i];
-                    const double pp = gdtk_div_nr(L[i], ci_ + ZERO_EPS);
-                    double N, D;
-                    alpha_nd(pp * h, N, D);
+                    const double pp = gdtk_div(L[i], ci_ + ZERO_EPS);
                     const double q0 = (s == 0) ? q[i] : Q0[i * ks];
                     const double pb = (s == 0) ? pp : fma(0.5, pp, P0[i * ks]);   // P0 holds p0 / 2
-                    // y + h (N (q - q0) + D (q0 - pb y)) / (N h pb + D)
-                    const double num = h * fma(N, q[i] - q0, D * fma(-pb, y, q0));
-                    const double v = gdtk_add_div(y, num, fma(N, h * pb, D));
+                    const double v = qss_value(y, pp, h, q[i], q0, pb);
                     if (s == 0) {
                         Q0[i * ks] = q[i];
                         P0[i * ks] = 0.5 * pp;
                         YP0[i * ks] = v;
-                    } else if (!lt_pos(v, ZERO_EPS) &&
-                               ge_nn(abs_bits(v - YP0[i * ks]), fma(GDTK_EPS1, v, GDTK_EPS1 * GDTK_DELTA))) {
+                    } else if (qss_misses(v, YP0[i * ks])) {
                         conv = false;
                     }
                     yn[i] = v;
                 }
                 if (s > 0 && conv) break;
             }
-            // sigma = max_i |yc - yp0| / (eps2 (yc + delta)), the largest ratio found by comparing
-            // cross products (denominators are positive), then one division
-            double snum = 0.0, sden = 1.0;
-#pragma unroll
-            for (int i = 0; i < GDTK_NSP; ++i) {
-                double yc = yn[i];
-                if (lt_pos(yc, ZERO_EPS)) continue;
-                const double num = abs_bits(yc - YP0[i * ks]), den = fma(GDTK_EPS2, yc, GDTK_EPS2 * GDTK_DELTA);
-                if (gt_nn(num * sden, snum * den)) { snum = num; sden = den; }
-            }
-            const double sigma = gdtk_div(snum, sden);
-            if (!nonzero(sigma)) dtS = 10.0 * h;   // sigma <= 0 (sigma is >= 0 or NaN)
-            else {
-                double x = sigma;
-                x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-                x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-                x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-                dtS = h * (gdtk_div(1.0, x) + 0.005);
-            }
+            dtS = qss_step(tree_max_ratio<0, tree_width(GDTK_NSP)>([&](int i) { return sigma_leaf(yn[i], YP0[i * ks]); }), h);
             ok = conv;
         }
 #endif
@@ -708,8 +762,7 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
         lane_stat(a.lane_stats, 3);
         if (ok) {   // mass-fraction test (chemistry_update.d:175-185); the Y_i go to V for the thermo update
             double tot = sum_pairwise([&](int i) {
-                double v = yn[i] * GDTK_M[i] * rrho;
-                v = lt_pos(v, 1.0e-30) ? 0.0 : v;
+                const double v = clipped_massf(yn[i], GDTK_M[i], rrho);
                 V[i * ks] = v;
                 return v;
             });
@@ -721,24 +774,21 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
             t += h;
 #pragma unroll
             for (int i = 0; i < GDTK_NSP; ++i) y0[i] = yn[i];
-            double hMax = h * 1.1;
-            if (dtS > h) h = fmin(dtS, hMax);
+            h = grown_step(h, dtS);
 #if GDTK_TIGHT
             {   // chemistry_update.d:265-269; Y_i (from the mass-fraction test) -> Y_i R_i in V, free until the next step
-                double Rm = 0.0;
-#pragma unroll
-                for (int i = 0; i < GDTK_NSP; ++i) {
-                    double yr = V[i * ks] * GDTK_R[i];
+                const double Rm = sum_pairwise([&](int i) {
+                    const double yr = __dmul_rn(V[i * ks], GDTK_R[i]);
                     V[i * ks] = yr;
-                    Rm += yr;
-                }
+                    return yr;
+                });
                 T = T_from_u(TH, V, ks, V + GDTK_NSP * ks, u, T, Rm, &lnT, &err, &n_newton, a.lane_stats);
                 p = rho * Rm * T;
                 need_kc = true;
             }
 #endif
             if (err) fail = err;
-            else if (t >= tI) {
+            else if (ge_pos(t, tI)) {
                 if (cycle == 0) dtSave = dtS;
                 done = true;
             } else {
@@ -766,18 +816,13 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
         }
         if (done) {   // chemistry_update.d:290-325, then fluidfvcell.d:956
             lane_stat(a.lane_stats, 5);
-            auto mf_of = [&](int i) {
-                double v = y0[i] * GDTK_M[i] * rrho;
-                return lt_pos(v, 1.0e-30) ? 0.0 : v;
-            };
-            double rtot = gdtk_div(1.0, sum_pairwise(mf_of));
-            double Rm = 0.0;
-#pragma unroll
-            for (int i = 0; i < GDTK_NSP; ++i) {
-                double yr = mf_of(i) * rtot * GDTK_R[i];
+            auto mf_of = [&](int i) { return clipped_massf(y0[i], GDTK_M[i], rrho); };
+            double rtot = gdtk_rcp(sum_pairwise(mf_of));
+            const double Rm = sum_pairwise([&](int i) {
+                const double yr = __dmul_rn(mf_of(i) * rtot, GDTK_R[i]);
                 V[i * ks] = yr;
-                Rm += yr;
-            }
+                return yr;
+            });
             int st = 0;
             if (a.flags & F_UPDATE_THERMO) {
                 T = T_from_u(TH, V, ks, V + GDTK_NSP * ks, u, T, Rm, &lnT, &st, &n_newton, a.lane_stats);
@@ -828,8 +873,8 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                                                                                      float* key) {
     extern __shared__ double smem[];
     double* TH = smem;
-    double* ETAB = smem + GDTK_NSP * GDTK_TH_STRIDE;
-    double* S = ETAB + GDTK_EXP2_TABLE_SIZE;
+    uint64_t* ETAB = reinterpret_cast<uint64_t*>(smem + GDTK_NSP * GDTK_TH_STRIDE);
+    double* S = smem + GDTK_NSP * GDTK_TH_STRIDE + GDTK_EXP2_TABLE_SIZE;
     for (int k = threadIdx.x; k < GDTK_NSP * GDTK_TH_STRIDE; k += blockDim.x) TH[k] = a.thermo[k];
     for (int k = threadIdx.x; k < GDTK_EXP2_TABLE_SIZE; k += blockDim.x) ETAB[k] = a.exp_table[k];
     __syncthreads();

@@ -1054,10 +1054,10 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
     for (int i = w.lane; i < n; i += 32) {
         const double y = y0[i];
         const double qi = q[i];
-        const double pi = gdtk_div_nr(L[i], y + ZERO_EPS);
+        const double pi = gdtk_div(L[i], y + ZERO_EPS);
         double N, D;
         w_alpha_nd(pi * h, N, D);
-        const double v = gdtk_add_div(y, h * (D * fma(-pi, y, qi)), fma(N, h * pi, D));
+        const double v = y + gdtk_div(h * (D * fma(-pi, y, qi)), fma(N, h * pi, D));
         q0[i] = qi; p0[i] = 0.5 * pi; yp[i] = v; yp0[i] = v;
     }
     __syncwarp();
@@ -1068,11 +1068,11 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
         bool conv = true;
         for (int i = w.lane; i < n; i += 32) {
             const double y = y0[i];
-            const double pp = gdtk_div_nr(L[i], yp[i] + ZERO_EPS);
+            const double pp = gdtk_div(L[i], yp[i] + ZERO_EPS);
             double N, D;
             w_alpha_nd(pp * h, N, D);
             const double pb = fma(0.5, pp, p0[i]);
-            const double yc = gdtk_add_div(y, h * fma(N, q[i] - q0[i], D * fma(-pb, y, q0[i])), fma(N, h * pb, D));
+            const double yc = y + gdtk_div(h * fma(N, q[i] - q0[i], D * fma(-pb, y, q0[i])), fma(N, h * pb, D));
             yp[i] = yc;
             if (!(yc < ZERO_EPS)) {
                 const double test = fabs(yc - yp0[i]);
@@ -1099,10 +1099,10 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
     if (sigma <= 0.0) h_new = 10.0 * h;
     else {
         double x = sigma;
-        x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-        x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-        x = x - 0.5 * gdtk_div_nr(x * x - sigma, x);
-        h_new = h * (gdtk_div_nr(1.0, x) + 0.005);
+        x = x - 0.5 * gdtk_div(x * x - sigma, x);
+        x = x - 0.5 * gdtk_div(x * x - sigma, x);
+        x = x - 0.5 * gdtk_div(x * x - sigma, x);
+        h_new = h * (gdtk_rcp(x) + 0.005);
     }
     hSuggest = h_new;
     if (converged)

@@ -26,6 +26,7 @@
 #include <mutex>
 #include <sstream>
 #include <stdexcept>
+#include <tuple>
 #include <sys/stat.h>
 #include <unistd.h>
 
@@ -38,10 +39,12 @@ namespace gdtk {
 
 extern const char* const kFastCuhSource;
 extern const char* const kFastExpSource;
+extern const char* const kGroupCuhSource;
 
 namespace {
 
 constexpr double R_universal = 8.31451;
+constexpr int kGroupBlock = 512;   // most threads of a block of the kernel with a group of lanes per cell
 
 std::string lit(double v) {   // exact double literal
     char buf[64];
@@ -169,42 +172,79 @@ std::string arrhenius_expr(double A, double n, double C) {
     return e.empty() ? std::string("0.0") : "gdtk_exp(" + e + ", etab)";
 }
 
-// Forward rate constant of a pressure-dependent reaction (rate_constant.d:155-160, 258-287,
-// 338-350) as statements ending in `kf`, from the third-body concentration `Mc`.  log10 and
-// pow(10, x) are written as ln x / ln 10 and exp(x ln 10).
-std::string pressure_dependent_code(const RateConstHost& f) {
-    std::ostringstream o;
-    o << "    const double kinf = " << arrhenius_expr(f.A, f.n, f.C) << ";\n";
-    o << "    const double k0 = " << arrhenius_expr(f.A0, f.n0, f.C0) << ";\n";
-    o << "    const double klh = k0 * kinf * Mc / fma(k0, Mc, kinf);\n";
-    if (f.model == RATE_LH) {
-        o << "    const double kf = klh;\n";
-    } else if (f.model == RATE_TROE) {
-        const double INV_LN10 = 1.0 / std::log(10.0);
-        o << "    const double pr = k0 * Mc / kinf;\n";
-        o << "    const double lpr = log(fmax(pr, 1.0e-30)) * " << lit(INV_LN10) << ";\n";
-        if (f.troe_flags & TROE_FCENT) {
-            const double lfc = std::log10(std::max(f.Fcent, 1.0e-30));
-            o << "    const double lfc = " << lit(lfc) << ", cc = " << lit(-0.4 - 0.67 * lfc)
-              << ", nn = " << lit(0.75 - 1.27 * lfc) << ";\n";
-        } else {
-            o << "    double fcent = " << lit(1.0 - f.a) << " * gdtk_exp(" << lit(-1.0 / f.T3) << " * T, etab);\n";
-            if (f.troe_flags & TROE_T1)
-                o << "    fcent = fma(" << lit(f.a) << ", gdtk_exp(" << lit(-1.0 / f.T1) << " * T, etab), fcent);\n";
-            if (f.troe_flags & TROE_T2) o << "    fcent += gdtk_exp(" << lit(-f.T2) << " * rT, etab);\n";
-            o << "    const double lfc = log(fmax(fcent, 1.0e-30)) * " << lit(INV_LN10) << ";\n";
-            o << "    const double cc = fma(-0.67, lfc, -0.4), nn = fma(-1.27, lfc, 0.75);\n";
-        }
-        o << "    const double numer = lpr + cc;\n";
-        o << "    const double frac = numer / fma(-0.14, numer, nn);\n";
-        o << "    const double kf = gdtk_exp(lfc / fma(frac, frac, 1.0) * " << lit(std::log(10.0)) << ", etab) * klh;\n";
-    } else {   // Yungster-Rabinowitz: a, b, c in a, T1, T2
-        o << "    const double pr = k0 * Mc / kinf;\n";
-        o << "    const double lpr = log(pr);\n";
-        o << "    const double fc = fma(" << lit(f.a) << ", gdtk_exp(" << lit(-f.T1) << " * rT, etab), " << lit(1.0 - f.a)
-          << " * gdtk_exp(" << lit(-f.T2) << " * rT, etab));\n";
-        o << "    const double kf = kinf * (pr / (1.0 + pr)) * fc / fma(lpr, lpr, 1.0);\n";
+// Rate constants of the pressure-dependent reactions (rate_constant.d:155-160, 258-287, 338-350), from the
+// third-body concentration Mc, as one function over a table: log10 and pow(10, x) are written as
+// ln x / ln 10 and exp(x ln 10), and k_b = k_f / K_c.
+const char* const kFalloffSource = R"(
+struct FallRec { double lnA, n, mC, A, lnA0, n0, mC0, A0, lfc, a, x1, x2, x3; int model, flags, pw, pw0, np, nusum, idx, pad;
+                 int sp[8]; double nu[8]; };
+__device__ __forceinline__ double fall_arrhenius(double lnA, double n, double mC, double A, int pw, double T, double lnT, double rT,
+                                                 const uint64_t* etab) {
+  if (pw == 98) return 0.0;
+  if (pw == 99) return gdtk_exp(fma(mC, rT, fma(n, lnT, lnA)), etab);
+  const double b = pw > 0 ? T : rT;
+  double k = A;
+  for (int m = 0; m < abs(pw); ++m) k *= b;
+  return k;
+}
+__device__ __noinline__ void falloff_rates(const FallRec& R, double T, double lnT, double rT, double Mc, const double* g, int gs,
+                                           const uint64_t* etab, double& kf, double& kb) {
+  const double INV_LN10 = 0x1.bcb7b1526e50ep-2, LN10 = 0x1.26bb1bbb55516p+1;
+  const double kinf = fall_arrhenius(R.lnA, R.n, R.mC, R.A, R.pw, T, lnT, rT, etab);
+  const double k0 = fall_arrhenius(R.lnA0, R.n0, R.mC0, R.A0, R.pw0, T, lnT, rT, etab);
+  if (R.model == 4) {   // Yungster-Rabinowitz
+    const double pr = gdtk_div(k0 * Mc, kinf), lpr = log(pr);
+    const double fc = fma(R.a, gdtk_exp(R.x1 * rT, etab), (1.0 - R.a) * gdtk_exp(R.x2 * rT, etab));
+    kf = gdtk_div(__dmul_rn(kinf * gdtk_div(pr, 1.0 + pr), fc), fma(lpr, lpr, 1.0));
+  } else {
+    kf = gdtk_div(k0 * kinf * Mc, fma(k0, Mc, kinf));
+    if (R.model == 3) {   // Troe
+      const double lpr = log(fmax(gdtk_div(k0 * Mc, kinf), 1.0e-30)) * INV_LN10;
+      double lfc = R.lfc;
+      if (!(R.flags & 1)) {
+        double fcent = (1.0 - R.a) * gdtk_exp(R.x3 * T, etab);
+        if (R.flags & 2) fcent = fma(R.a, gdtk_exp(R.x1 * T, etab), fcent);
+        if (R.flags & 4) fcent += gdtk_exp(R.x2 * rT, etab);
+        lfc = log(fmax(fcent, 1.0e-30)) * INV_LN10;
+      }
+      const double numer = lpr + fma(-0.67, lfc, -0.4);
+      const double frac = gdtk_div(numer, fma(-0.14, numer, fma(-1.27, lfc, 0.75)));
+      kf *= gdtk_exp(gdtk_div(lfc, fma(frac, frac, 1.0)) * LN10, etab);
     }
+  }
+  double dg = 0.0;
+  for (int k = 0; k < R.np; ++k) dg = fma(R.nu[k], g[R.sp[k] * gs], dg);
+  kb = kf * gdtk_exp(-fma((double)R.nusum, GDTK_LN_PATM_R - lnT, -dg), etab);
+}
+)";
+
+// A row of GDTK_FALL_TAB.
+std::string falloff_record(const ReactionHost& r, int ir) {
+    const RateConstHost& f = r.frc;
+    auto power = [](double A, double n, double C) {
+        if (C == 0.0 && n == std::floor(n) && std::fabs(n) <= 4) return (int)n;
+        return A <= 0.0 ? 98 : 99;
+    };
+    auto ln = [](double A) { return A > 0.0 ? std::log(A) : 0.0; };
+    const bool troe = f.model == RATE_TROE, given = f.troe_flags & TROE_FCENT;
+    auto inv = [](double x) { return x != 0.0 ? -1.0 / x : 0.0; };
+    std::ostringstream o, sp, nu;
+    int np = 0, nusum = 0;
+    for (auto& pp : participants(r)) {
+        if (pp.nu == 0) continue;
+        sp << (np ? ", " : "") << pp.isp;
+        nu << (np ? ", " : "") << lit((double)pp.nu);
+        nusum += pp.nu;
+        ++np;
+    }
+    if (np == 0) { sp << "0"; nu << "0.0"; }
+    o << "  {" << lit(ln(f.A)) << ", " << lit(f.n) << ", " << lit(-f.C) << ", " << lit(f.A) << ", " << lit(ln(f.A0)) << ", "
+      << lit(f.n0) << ", " << lit(-f.C0) << ", " << lit(f.A0) << ", "
+      << lit(troe && given ? std::log10(std::max(f.Fcent, 1.0e-30)) : 0.0) << ", " << lit(f.a) << ", "
+      << lit(troe ? inv(f.T1) : -f.T1) << ", " << lit(-f.T2) << ", " << lit(troe ? inv(f.T3) : 0.0) << ", "
+      << (f.model == RATE_LH ? 2 : troe ? 3 : 4) << ", " << f.troe_flags << ", " << power(f.A, f.n, f.C) << ", "
+      << power(f.A0, f.n0, f.C0) << ", " << np << ", " << nusum << ", " << ir << ", 0, {" << sp.str() << "}, {" << nu.str()
+      << "}},\n";
     return o.str();
 }
 
@@ -279,6 +319,32 @@ int g_unroll() { return env_int("GDTK_G_UNROLL", 1); }
 int rhs_fence() {
     const char* e = std::getenv("GDTK_RHS_FENCE");
     return (e && *e) ? std::max(0, std::atoi(e)) : 4;
+}
+
+// A sum over the species as the zero-padded pairwise tree of chem_fast.cuh's sum_pairwise.
+std::string tree_sum(const std::vector<std::string>& leaf, int lo, int n) {
+    if (n == 1) return leaf[lo];
+    const std::string a = tree_sum(leaf, lo, n / 2);
+    std::string b;
+    if (lo + n / 2 < (int)leaf.size()) b = tree_sum(leaf, lo + n / 2, n / 2);
+    if (a.empty() || b.empty()) return a.empty() ? b : a;
+    return "(" + a + " + " + b + ")";
+}
+
+// Whether the kernel with a group of lanes per cell (chem_group.cuh) takes the mechanism: every reaction in
+// its tables, and no code form asked for that only the one-thread-per-cell kernel has.
+bool group_kernel_takes(const MechanismHost& mh, size_t n_table, size_t n_falloff) {
+    for (const char* e : {"GDTK_KC_UNROLLED", "GDTK_KB_EXP", "GDTK_PHASE_CLOCKS"}) {
+        const char* v = std::getenv(e);
+        if (v && v[0] == '1') return false;
+    }
+    if (n_table + n_falloff != mh.reactions.size()) return false;
+    for (auto& r : mh.reactions)
+        for (auto* side : {&r.reac, &r.prod}) {
+            if (side->size() > 4) return false;
+            for (auto& x : *side) if (x.second < 1 || x.second > 7) return false;
+        }
+    return true;
 }
 
 bool mix_thermo_range(const GasModelHost& gm, double& tlo, double& thi) {
@@ -373,7 +439,154 @@ int fast_vec_doubles(const GasModelHost& gm, const MechanismHost& mh) {
     return std::max(vec, (any_kb_products(gm, mh) ? 3 * nsp : nsp) + nfall);
 }
 
-std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh, int block, int min_blocks) {
+// The tables of chem_group.cuh: rate-constant records, tick-rate records (both sorted so that the lanes of a
+// round take the same path), and the q and L sums as tasks, dealt whole to 4, 8, 16 or 32 lanes, longest first.
+std::string group_tables(const GasModelHost& gm, const MechanismHost& mh, const std::vector<int>& table_rx,
+                         const std::vector<bool>& kbp, const std::vector<std::vector<std::pair<int, double>>>& sets,
+                         const std::vector<int>& set_of, GroupShape& shape) {
+    const int nsp = gm.n_species(), nr = (int)mh.reactions.size();
+    std::ostringstream o;
+    auto high = [](double v) {
+        uint64_t b;
+        std::memcpy(&b, &v, 8);
+        return (unsigned)(b >> 32);
+    };
+    int nfall = 0;
+    for (auto& r : mh.reactions) nfall += r.frc.pressure_dependent() ? 1 : 0;
+    bool any = false;
+    for (int ir : table_rx) any = any || kbp[ir];
+    o << "#define GDTK_ANY_KBP " << (any ? 1 : 0) << "\n#define GDTK_NKC " << table_rx.size() << "\n#define GDTK_NSETS "
+      << sets.size() << "\n#define GDTK_GRP_BLOCK " << kGroupBlock << "\n";
+    // GRP_CELL of chem_group.cuh (checked there)
+    const int nsets = (int)sets.size();
+    shape.cell_doubles = (4 * nsp + 2 * nr + std::max(2 * nr, std::max(3 * nsp + nfall, nsp + 24)) + nsets +
+                          (mh.method == METHOD_RKF ? 6 : 3) * nsp) | 1;
+    // rate constants, by path
+    struct Kc { int ir, mode, pw, np, nusum; std::vector<Part> parts; };
+    std::vector<Kc> kc;
+    for (int ir : table_rx) {
+        const ReactionHost& r = mh.reactions[ir];
+        Kc k{ir, 0, 99, 0, 0, {}};
+        for (auto& pp : participants(r))
+            if (pp.nu) { k.parts.push_back(pp); k.nusum += pp.nu; }
+        k.np = (int)k.parts.size();
+        k.mode = r.frc.model == RATE_ARRHENIUS ? (r.brc.model == RATE_FROM_EQ ? 0 : 1) : 2;
+        if (k.mode == 0 && kbp[ir]) k.mode = 3;
+        std::string e;
+        if (power_arrhenius(r.frc, e)) k.pw = (int)r.frc.n;
+        kc.push_back(k);
+    }
+    auto kc_key = [](const Kc& k) { return std::make_tuple(k.mode, k.mode == 3 && k.pw != 99, k.np, std::abs(k.nusum)); };
+    std::stable_sort(kc.begin(), kc.end(), [&](const Kc& a, const Kc& b) { return kc_key(a) < kc_key(b); });
+    o << "struct GrpKc { double lnA, n, mC, lnAb, nb, mCb, A; int mode, np, nusum, idx, pw, nusumh; int nuh[8]; signed char sp[8], "
+         "anu[8]; };\n__device__ const GrpKc GRP_KC[" << std::max<size_t>(kc.size(), 1) << "] = {\n";
+    auto lnA = [](const RateConstHost& rc) { return rc.A > 0.0 ? std::log(rc.A) : -1.0e300; };
+    for (auto& k : kc) {
+        const ReactionHost& r = mh.reactions[k.ir];
+        o << "  {" << lit(lnA(r.frc)) << ", " << lit(r.frc.n) << ", " << lit(-r.frc.C) << ", " << lit(lnA(r.brc)) << ", "
+          << lit(r.brc.n) << ", " << lit(-r.brc.C) << ", " << lit(r.frc.A) << ", " << k.mode << ", " << k.np << ", " << k.nusum
+          << ", " << k.ir << ", " << k.pw << ", (int)" << high((double)k.nusum) << "u, {";
+        for (int j = 0; j < k.np; ++j) o << (j ? ", " : "") << "(int)" << high((double)k.parts[j].nu) << "u";
+        o << (k.np ? "}, {" : "0}, {");
+        for (int j = 0; j < k.np; ++j) o << (j ? ", " : "") << k.parts[j].isp;
+        o << (k.np ? "}, {" : "0}, {");
+        for (int j = 0; j < k.np; ++j) o << (j ? ", " : "") << k.parts[j].nu;
+        o << (k.np ? "}},\n" : "0}},\n");
+    }
+    if (kc.empty()) o << "  {}\n";
+    o << "};\n";
+    // tick rates, by the number of factors
+    std::vector<int> order(nr);
+    for (int i = 0; i < nr; ++i) order[i] = i;
+    auto rx_key = [&](int ir) {
+        const ReactionHost& r = mh.reactions[ir];
+        return std::make_tuple(!r.collider, r.reac.size(), r.prod.size());
+    };
+    std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return rx_key(a) < rx_key(b); });
+    o << "__device__ const __align__(16) uint4 GRP_RX[" << nr << "] = {\n";
+    for (int ir : order) {
+        const ReactionHost& r = mh.reactions[ir];
+        unsigned sp[2] = {0, 0}, co = (unsigned)r.reac.size() | (unsigned)r.prod.size() << 3;
+        int side = 0;
+        for (auto* v : {&r.reac, &r.prod}) {
+            for (size_t k = 0; k < v->size(); ++k) {
+                sp[side] |= (unsigned)(*v)[k].first << (8 * k);
+                co |= (unsigned)(*v)[k].second << (6 + 12 * side + 3 * k);
+            }
+            ++side;
+        }
+        o << "  {" << sp[0] << "u, " << sp[1] << "u, " << co << "u, "
+          << ((unsigned)ir | (unsigned)(r.collider ? set_of[ir] + 1 : 0) << 16) << "u},\n";
+    }
+    o << "};\n__device__ const double GRP_EFF[" << std::max<size_t>(sets.size(), 1) * nsp << "] = {";
+    for (auto& st : sets) {
+        std::vector<double> e(nsp, 0.0);
+        for (auto& x : st) e[x.first] = x.second;
+        for (double v : e) o << lit(v) << ", ";
+    }
+    if (sets.empty()) o << "0.0";
+    o << "};\n";
+    if (nfall) {
+        o << "__device__ const double GRP_FALL_EFF[" << nfall * nsp << "] = {";
+        for (auto& r : mh.reactions) {
+            if (!r.frc.pressure_dependent()) continue;
+            std::vector<double> e(nsp, 0.0);
+            for (auto& x : r.eff) e[x.first] = x.second;
+            for (double v : e) o << lit(v) << ", ";
+        }
+        o << "};\n";
+    }
+    // q and L: q gets nu w_f (nu > 0) or -nu w_b, L gets nu w_b or -nu w_f (reaction_mechanism.d:82-96)
+    std::vector<std::vector<std::pair<int, int>>> task(2 * nsp);
+    for (int ir = 0; ir < nr; ++ir)
+        for (auto& pp : participants(mh.reactions[ir])) {
+            if (pp.nu == 0) continue;
+            task[2 * pp.isp].push_back({pp.nu > 0 ? ir : nr + ir, std::abs(pp.nu)});
+            task[2 * pp.isp + 1].push_back({pp.nu > 0 ? nr + ir : ir, std::abs(pp.nu)});
+        }
+    size_t n_ent = 0;
+    for (auto& t : task) n_ent += t.size();
+    o << "__device__ const __align__(16) uint2 GRP_ENT[" << std::max<size_t>(n_ent, 1) << "] = {";
+    for (auto& t : task)
+        for (auto& e : t) o << "{" << e.first << "u, " << high((double)e.second) << "u}, ";
+    if (!n_ent) o << "{0u, 0u}";
+    o << "};\n__device__ const __align__(16) int GRP_TASK[" << ((2 * nsp + 1 + 1) & ~1) << "] = {0";
+    size_t at = 0;
+    for (auto& t : task) o << ", " << (at += t.size());
+    o << "};\n";
+    std::vector<int> by_length(2 * nsp);
+    for (int t = 0; t < 2 * nsp; ++t) by_length[t] = t;
+    std::stable_sort(by_length.begin(), by_length.end(), [&](int a, int b) { return task[a].size() > task[b].size(); });
+    std::ostringstream starts, tasks;
+    for (int lanes : {4, 8, 16, 32}) {
+        std::vector<std::vector<int>> of(lanes);
+        std::vector<size_t> load(lanes, 0);
+        for (int t : by_length) {
+            const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            of[l].push_back(t);
+            load[l] += task[t].size() + 1;
+        }
+        int n = 0;
+        for (int l = 0; l < 33; ++l) {
+            starts << (starts.tellp() > 0 ? ", " : "") << n;
+            if (l < lanes) {
+                for (int t : of[l]) tasks << (tasks.tellp() > 0 ? ", " : "") << t;
+                n += (int)of[l].size();
+            }
+        }
+    }
+    o << "__device__ const __align__(16) int GRP_LANE_START[132] = {" << starts.str() << "};\n";
+    o << "__device__ const __align__(16) int GRP_LANE_TASK[" << 8 * nsp << "] = {" << tasks.str() << "};\n";
+    // the staged tables (GRP_TABLES of chem_group.cuh, checked there)
+    shape.table_doubles = 2 * nr + nsp * 120 + GDTK_EXP2_TABLE_SIZE + std::max(nsets, 1) * nsp +
+                          16 * (int)std::max<size_t>(kc.size(), 1) + (int)std::max<size_t>(n_ent, 1) + (2 * nsp + 2) / 2 + 66 +
+                          4 * nsp;
+    o << "#define GDTK_GRP_CELL " << shape.cell_doubles << "\n#define GDTK_GRP_TABLES " << shape.table_doubles << "\n";
+    return o.str();
+}
+
+std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh, int block, int min_blocks,
+                                 GroupShape* group_shape) {
     if (gm.n_species() > GDTK_MAX_SPECIES || (int)mh.reactions.size() > GDTK_MAX_REACTIONS)
         throw std::runtime_error("the mechanism-specialised kernel takes up to " + std::to_string(GDTK_MAX_SPECIES) +
                                  " species and " + std::to_string(GDTK_MAX_REACTIONS) +
@@ -411,7 +624,7 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
     arr("GDTK_M", [&](int i) { return gm.M[i]; });
     arr("GDTK_RM", [&](int i) { return 1.0 / gm.M[i]; });
     arr("GDTK_R", [&](int i) { return R_universal / gm.M[i]; });
-    o << "namespace gdtk_fast {\nusing gdtk::gdtk_exp;\nusing gdtk::gdtk_div_nr;\n";
+    o << "namespace gdtk_fast {\nusing gdtk::gdtk_exp;\nusing gdtk::gdtk_div;\nusing gdtk::gdtk_rcp;\n";
 
     // ---- third-body concentrations of the pressure-dependent rate constants (rate_constant.d:114-121),
     // from the concentrations at which the rate constants are evaluated
@@ -421,9 +634,9 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
     for (int ir = 0; ir < nr; ++ir) {
         const ReactionHost& r = mh.reactions[ir];
         if (!r.frc.pressure_dependent()) continue;
-        o << "  Mv[" << nfall << " * ms] = 0.0";
-        for (auto& e : r.eff) o << " + " << lit(e.second) << " * c[" << e.first << "]";
-        o << ";\n";
+        o << "  { double m = 0.0;";
+        for (auto& e : r.eff) o << " m = fma(" << lit(e.second) << ", c[" << e.first << "], m);";
+        o << " Mv[" << nfall << " * ms] = m; }\n";
         ++nfall;
     }
     o << "}\n#define GDTK_NFALLOFF " << nfall << "\n";
@@ -481,8 +694,16 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         }
         o << "};\n";
     }
+    o << "#define GDTK_LN_PATM_R " << lit(std::log(101325.0 / R_universal)) << "\n";
+    o << "#define GDTK_R_PATM " << lit(R_universal / 101325.0) << "\n#define GDTK_PATM_R " << lit(101325.0 / R_universal) << "\n";
+    if (nfall) {
+        o << kFalloffSource << "__device__ const FallRec GDTK_FALL_TAB[" << nfall << "] = {\n";
+        for (int ir = 0; ir < nr; ++ir)
+            if (mh.reactions[ir].frc.pressure_dependent()) o << falloff_record(mh.reactions[ir], ir);
+        o << "};\n";
+    }
     o << "__device__ __forceinline__ void gen_kc(double T, double lnT, double rT, const double* g, int gs, double* K, "
-         "int ks, const double* etab, const double* Mv, int ms) {\n";
+         "int ks, const uint64_t* etab, const double* Mv, int ms) {\n";
     o << "  (void)T; (void)Mv; (void)ms;\n";
     if (any_kbp) {   // E_i = exp(G_i / R T) and its reciprocal, after G/RT and the falloff concentrations
         o << "  const double* E = g + (" << nsp << " + " << nfall << ") * gs;\n";
@@ -491,7 +712,7 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         o << "  for (int i = 0; i < " << nsp << "; ++i) {\n";
         o << "    const double e = gdtk_exp(g[i * gs], etab);\n";
         o << "    const_cast<double*>(E)[i * gs] = e;\n";
-        o << "    const_cast<double*>(Ei)[i * gs] = gdtk_div_nr(1.0, e);\n  }\n";
+        o << "    const_cast<double*>(Ei)[i * gs] = gdtk_rcp(e);\n  }\n";
         o << "  const double cf = T * " << lit(R_universal / 101325.0) << ", rcf = rT * " << lit(101325.0 / R_universal)
           << ";   // R T / P_atm and its reciprocal\n";
     }
@@ -535,37 +756,28 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         if (all_kbp) o << "#endif\n";
         o << "  }\n";
     }
-    int ifall = 0;
+    if (nfall) {
+        o << "#pragma unroll 1\n  for (int f = 0; f < " << nfall << "; ++f) {\n    double kf, kb;\n";
+        o << "    falloff_rates(GDTK_FALL_TAB[f], T, lnT, rT, Mv[f * ms], g, gs, etab, kf, kb);\n";
+        o << "    K[GDTK_FALL_TAB[f].idx * ks] = kf;\n    K[(" << nr << " + GDTK_FALL_TAB[f].idx) * ks] = kb;\n  }\n";
+    }
     for (int ir = 0; ir < nr; ++ir) {
         const ReactionHost& r = mh.reactions[ir];
-        if (std::find(table_rx.begin(), table_rx.end(), ir) != table_rx.end()) continue;
+        if (r.frc.pressure_dependent() || std::find(table_rx.begin(), table_rx.end(), ir) != table_rx.end()) continue;
         auto parts = participants(r);
         if (ir > 0 && ir % 4 == 0) o << "  asm volatile(\"\" ::: \"memory\");\n";
-        std::ostringstream dg;   // sum nu * G/RT
+        std::string dgs = "0.0";   // sum nu * G/RT
         int nusum = 0;
         for (auto& p : parts) {
             if (p.nu == 0) continue;
             nusum += p.nu;
-            std::string term = "g[" + std::to_string(p.isp) + " * gs]";
-            if (dg.tellp() == 0) {
-                if (p.nu == 1) dg << term;
-                else dg << lit((double)p.nu) << " * " << term;
-            } else {
-                if (p.nu == 1) dg << " + " << term;
-                else if (p.nu == -1) dg << " - " << term;
-                else dg << " + " << lit((double)p.nu) << " * " << term;
-            }
+            dgs = "fma(" + lit((double)p.nu) + ", g[" + std::to_string(p.isp) + " * gs], " + dgs + ")";
         }
-        std::string dgs = dg.tellp() == 0 ? std::string("0.0") : dg.str();
         // ln K_c = -sum(nu G/RT) + sum(nu) ln(P_atm / R T)   (reaction.d:26-52)
         std::string lnKc = "(-(" + dgs + ")" +
                            (nusum ? " + " + lit((double)nusum) + " * (" + lit(std::log(101325.0 / R_universal)) + " - lnT)" : std::string("")) + ")";
         o << "  { // " << (r.equation.empty() ? std::string("reaction") : r.equation) << "\n";
-        if (r.frc.pressure_dependent()) {   // backward from K_c (checked when the mechanism is read)
-            o << "    const double Mc = Mv[" << ifall++ << " * ms];\n";
-            o << pressure_dependent_code(r.frc);
-            o << "    const double kb = kf * gdtk_exp(-" << lnKc << ", etab);\n";
-        } else if (r.frc.simple()) {
+        if (r.frc.simple()) {
             std::string pw;
             if (power_arrhenius(r.frc, pw)) {
                 o << "    const double kf = " << pw << ";\n";
@@ -609,19 +821,15 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         set_of[ir] = f;
     }
     for (size_t s = 0; s < sets.size(); ++s) {
-        o << "  double M" << s << " = 0.0;\n";
-        bool first = true;
+        std::vector<std::string> leaf(nsp);
         for (auto& e : sets[s]) {
-            std::string cc = "c[" + std::to_string(e.first) + "]";
-            if (first) {
-                o << "  M" << s << " = " << (e.second == 1.0 ? cc : lit(e.second) + " * " + cc) << ";\n";
-                first = false;
-            } else if (e.second == 1.0) {
-                o << "  M" << s << " += " << cc << ";\n";
-            } else {
-                o << "  M" << s << " = fma(" << lit(e.second) << ", " << cc << ", M" << s << ");\n";
-            }
+            const std::string cc = "c[" + std::to_string(e.first) + "]";
+            leaf[e.first] = e.second == 1.0 ? cc : "__dmul_rn(" + lit(e.second) + ", " + cc + ")";
         }
+        int p2 = 1;
+        while (p2 < nsp) p2 *= 2;
+        const std::string sum = tree_sum(leaf, 0, p2);
+        o << "  const double M" << s << " = " << (sum.empty() ? "0.0" : sum) << ";\n";
     }
     std::vector<bool> qset(nsp, false), lset(nsp, false);
     auto acc = [&](std::vector<bool>& set, const char* arr, int isp, int coeff, const char* w) {
@@ -638,8 +846,9 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         if (ir > 0 && rhs_fence() > 0 && ir % rhs_fence() == 0) o << "  asm volatile(\"\" ::: \"memory\");\n";
         o << "  {\n    double wf = K[" << ir << " * ks], wb = K[" << (nr + ir) << " * ks];\n";
         if (r.collider) o << "    wf *= M" << set_of[ir] << "; wb *= M" << set_of[ir] << ";\n";
-        for (auto& x : r.reac) o << "    wf *= " << ipow_expr("c[" + std::to_string(x.first) + "]", x.second) << ";\n";
-        for (auto& x : r.prod) o << "    wb *= " << ipow_expr("c[" + std::to_string(x.first) + "]", x.second) << ";\n";
+        // products that the compiler may not contract into the sums: the same rates in every kernel
+        for (auto& x : r.reac) o << "    wf = __dmul_rn(wf, " << ipow_expr("c[" + std::to_string(x.first) + "]", x.second) << ");\n";
+        for (auto& x : r.prod) o << "    wb = __dmul_rn(wb, " << ipow_expr("c[" + std::to_string(x.first) + "]", x.second) << ");\n";
         for (auto& p : participants(r)) {
             if (p.nu > 0) { acc(qset, "q", p.isp, p.nu, "wf"); acc(lset, "L", p.isp, p.nu, "wb"); }
             else if (p.nu < 0) { acc(qset, "q", p.isp, -p.nu, "wb"); acc(lset, "L", p.isp, -p.nu, "wf"); }
@@ -650,8 +859,15 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         if (!qset[i]) o << "  q[" << i << "] = 0.0;\n";
         if (!lset[i]) o << "  L[" << i << "] = 0.0;\n";
     }
-    o << "}\n}  // namespace gdtk_fast\n";
+    o << "}\n";
+    const bool group = group_kernel_takes(mh, table_rx.size(), (size_t)nfall);
+    o << "#define GDTK_GROUP " << (group ? 1 : 0) << "\n";
+    GroupShape shape;
+    if (group) o << group_tables(gm, mh, table_rx, kbp, sets, set_of, shape);
+    if (group_shape) *group_shape = shape;
+    o << "}  // namespace gdtk_fast\n";
     o << kFastCuhSource;
+    if (group) o << kGroupCuhSource;
     return o.str();
 }
 
@@ -720,6 +936,10 @@ std::string compile_fast_check(const GasModelHost& gm, const MechanismHost& mh, 
     return log + "\ncubin bytes: " + std::to_string(cubin.size()) + "\n";
 }
 
+static size_t group_smem(const GroupShape& g, int block, int lanes) {
+    return (size_t)(g.table_doubles + g.cell_doubles * (block / lanes)) * 8;
+}
+
 FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, int req_block, int req_min_blocks) {
     int dev = 0, major = 0, minor = 0, sms = 0;
     cudaGetDevice(&dev);
@@ -753,9 +973,10 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
     auto k = std::make_unique<FastKernel>();
     k->block = block;
     k->min_blocks = min_blocks;
+    k->method = mh.method;
     k->per_thread_doubles = per_thread;
     k->table_doubles = table;
-    k->source = generate_fast_source(gm, mh, block, min_blocks);
+    k->source = generate_fast_source(gm, mh, block, min_blocks, &k->group);
     std::string key = cubin_cache_key(k->source, major, minor);
     std::string cubin;
     {
@@ -806,8 +1027,21 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
              "cuFuncSetAttribute");
     cu_check(d.occupancy(&k->blocks_per_sm, fn, block, smem_max), "cuOccupancyMaxActiveBlocksPerMultiprocessor");
     if (k->blocks_per_sm < 1) throw std::runtime_error("fast kernel cannot be resident (registers/shared memory)");
+    if (k->group.cell_doubles) {
+        CUfunction gfn;
+        cu_check(d.moduleGetFunction(&gfn, mod, "gdtk_chem_group"), "cuModuleGetFunction");
+        cu_check(d.funcSetAttribute(gfn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)kSmPerBlock),
+                 "cuFuncSetAttribute");
+        // one block per SM: as many warps as its cells' slices fit beside the tables
+        for (int lv = 0; lv < 4; ++lv) {
+            int w = kGroupBlock / 32;
+            while (w > 0 && group_smem(k->group, 32 * w, 4 << lv) > (size_t)kSmPerBlock) --w;
+            k->group_warps[lv] = w;
+        }
+        k->group_function = gfn;
+    }
     std::vector<double> th = fast_thermo_table(gm);
-    static const double etab[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
+    static const uint64_t etab[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
     if (cudaMalloc(&k->d_thermo, th.size() * 8) != cudaSuccess || cudaMalloc(&k->d_exp, sizeof etab) != cudaSuccess)
         throw std::runtime_error("cudaMalloc failed");
     cudaMemcpy(k->d_thermo, th.data(), th.size() * 8, cudaMemcpyHostToDevice);
@@ -829,6 +1063,37 @@ cudaError_t launch_fast(FastKernel& k, FastArgs& a, int sm_count, cudaStream_t s
     size_t smem = (size_t)(k.table_doubles + k.per_thread_doubles * block) * 8;
     void* params[] = {&a};
     CUresult r = driver().launchKernel((CUfunction)k.function, (unsigned)grid, 1, 1, (unsigned)block, 1, 1,
+                                       (unsigned)smem, (CUstream)stream, params, nullptr);
+    if (grid_out) *grid_out = (int)grid;
+    if (block_out) *block_out = block;
+    if (smem_out) *smem_out = (int)smem;
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
+}
+
+int group_lanes(const FastKernel& k, long long total, int sm_count) {
+    if (!k.group_function) return 0;
+    const long long budget = (long long)sm_count * (k.method == METHOD_RKF ? 216 : 1725);
+    for (int lanes = 32; lanes >= 4; lanes /= 2) {
+        const int lv = lanes == 4 ? 0 : lanes == 8 ? 1 : lanes == 16 ? 2 : 3;
+        if (k.group_warps[lv] >= 1 && total * lanes <= budget) return lanes;
+    }
+    return k.method == METHOD_RKF || k.group_warps[0] < 1 ? 0 : 4;
+}
+
+cudaError_t launch_group(FastKernel& k, FastArgs& a, int lanes, int sm_count, cudaStream_t stream, int* grid_out,
+                         int* block_out, int* smem_out) {
+    a.thermo = k.d_thermo;
+    a.exp_table = k.d_exp;
+    int lv = 0;
+    while ((4 << lv) < lanes) ++lv;
+    // one block per SM, so that the tables are staged once per SM; the warps spread over all SMs
+    const long long warps = ((long long)a.total * lanes + 31) / 32;
+    const long long per_sm = std::min<long long>(std::max<long long>((warps + sm_count - 1) / sm_count, 1), k.group_warps[lv]);
+    const int block = 32 * (int)per_sm;
+    const long long grid = std::min<long long>((warps + per_sm - 1) / per_sm, sm_count);
+    const size_t smem = group_smem(k.group, block, lanes);
+    void* params[] = {&a, &lanes};
+    CUresult r = driver().launchKernel((CUfunction)k.group_function, (unsigned)grid, 1, 1, (unsigned)block, 1, 1,
                                        (unsigned)smem, (CUstream)stream, params, nullptr);
     if (grid_out) *grid_out = (int)grid;
     if (block_out) *block_out = block;

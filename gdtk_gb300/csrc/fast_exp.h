@@ -1,17 +1,18 @@
-// fast_exp.h -- exp(x) in FP64 by a table-driven method (shared by device and host code).
+// fast_exp.h -- exp(x) and a / b in FP64 on the integer pipe (shared by device and host code).
 //
-// Method: P. T. P. Tang, "Table-driven implementation of the exponential function in IEEE
-// floating-point arithmetic", ACM TOMS 15(2):144-157, 1989, with N = 256 table entries:
-//   x = (256 m + j) ln2/256 + r,  |r| <= ln2/512,
-//   exp(x) = 2^m * 2^(j/256) * (1 + p(r)),  p(r) = r + r^2 (1/2 + r/6 + r^2/24).
-// The Taylor remainder r^5/120 is below 3.8e-17 (0.17 ulp of 1) on the reduced range, so the
-// degree-4 polynomial suffices; the larger table buys the two multiply-adds that a 64-entry table
-// needs for degree 6.  The reduction uses a two-part ln2/256 (the leading part has 32 significant
-// bits, so k*L1 is exact for every reachable k) and fused multiply-adds; the scale by 2^m is an
-// integer add to the exponent field.  Cost: 9 FP64 operations (1 mul + 8 fma/add), no division.
-// The table 2^(j/256) holds correctly rounded doubles (2 KB); callers pass it in (kernels keep it
-// in shared memory, where lane-divergent indices do not serialise as constant-memory reads would).
-// Accuracy: within 1.3 ulp of the exact value on [-745.13, 709.78] (three quarters correctly
+// GB300 issues one FP64 warp instruction every 19 cycles per SM (76 cycles for each of the four
+// sub-partitions when all are busy, 64 when one warp runs alone) and runs 32-bit integer and FP32
+// instructions beside it at 1 to 4 cycles: 16 32 x 32 + 64-bit multiply-adds hide behind one FP64 FMA.
+// So both functions work on 64-bit fixed-point numbers, with no FP64 instruction in the common case.
+//
+// exp, after the table method of P. T. P. Tang, "Table-driven implementation of the exponential function in
+// IEEE floating-point arithmetic", ACM TOMS 15(2):144-157, 1989, in base 2:
+//   x log2(e) = k + j/256 + r,  0 <= r < 2^-8,  exp(x) = 2^k 2^(j/256) 2^r,
+// 2^r by its Taylor polynomial of degree 5 (remainder below 2^-60).  The product x log2(e) is kept to 2^-64,
+// the polynomial to about 2^-57, the table to 2^-64; the result is rounded once.
+// The table (2 KB) is passed in: kernels keep it in shared memory, where lane-divergent indices do not
+// serialise as constant-memory reads would.
+// Accuracy: within 0.66 ulp of the exact value for 1 <= |x| <= 708, 1 ulp below (95% and 82% correctly
 // rounded); +inf above, 0 below.
 #pragma once
 #ifndef __CUDACC_RTC__
@@ -19,6 +20,8 @@
 #include <cstring>
 #else
 typedef long long int64_t;
+typedef unsigned long long uint64_t;
+typedef int int32_t;
 typedef unsigned int uint32_t;
 #endif
 
@@ -32,73 +35,73 @@ typedef unsigned int uint32_t;
 
 namespace gdtk {
 
-// 2^(j/256), j = 0..255, correctly rounded.
+// 2^(j/256) 2^63, j = 0..255, rounded to nearest: the significands with their leading bit.
 #define GDTK_EXP2_TABLE_SIZE 256
 #define GDTK_EXP2_TABLE_INIT { \
-    0x1.0000000000000p+0, 0x1.00b1afa5abcbfp+0, 0x1.0163da9fb3335p+0, 0x1.02168143b0281p+0, \
-    0x1.02c9a3e778061p+0, 0x1.037d42e11bbccp+0, 0x1.04315e86e7f85p+0, 0x1.04e5f72f654b1p+0, \
-    0x1.059b0d3158574p+0, 0x1.0650a0e3c1f89p+0, 0x1.0706b29ddf6dep+0, 0x1.07bd42b72a836p+0, \
-    0x1.0874518759bc8p+0, 0x1.092bdf66607e0p+0, 0x1.09e3ecac6f383p+0, 0x1.0a9c79b1f3919p+0, \
-    0x1.0b5586cf9890fp+0, 0x1.0c0f145e46c85p+0, 0x1.0cc922b7247f7p+0, 0x1.0d83b23395decp+0, \
-    0x1.0e3ec32d3d1a2p+0, 0x1.0efa55fdfa9c5p+0, 0x1.0fb66affed31bp+0, 0x1.1073028d7233ep+0, \
-    0x1.11301d0125b51p+0, 0x1.11edbab5e2ab6p+0, 0x1.12abdc06c31ccp+0, 0x1.136a814f204abp+0, \
-    0x1.1429aaea92de0p+0, 0x1.14e95934f312ep+0, 0x1.15a98c8a58e51p+0, 0x1.166a45471c3c2p+0, \
-    0x1.172b83c7d517bp+0, 0x1.17ed48695bbc0p+0, 0x1.18af9388c8deap+0, 0x1.1972658375d2fp+0, \
-    0x1.1a35beb6fcb75p+0, 0x1.1af99f8138a1cp+0, 0x1.1bbe084045cd4p+0, 0x1.1c82f95281c6bp+0, \
-    0x1.1d4873168b9aap+0, 0x1.1e0e75eb44027p+0, 0x1.1ed5022fcd91dp+0, 0x1.1f9c18438ce4dp+0, \
-    0x1.2063b88628cd6p+0, 0x1.212be3578a819p+0, 0x1.21f49917ddc96p+0, 0x1.22bdda27912d1p+0, \
-    0x1.2387a6e756238p+0, 0x1.2451ffb82140ap+0, 0x1.251ce4fb2a63fp+0, 0x1.25e85711ece75p+0, \
-    0x1.26b4565e27cddp+0, 0x1.2780e341ddf29p+0, 0x1.284dfe1f56381p+0, 0x1.291ba7591bb70p+0, \
-    0x1.29e9df51fdee1p+0, 0x1.2ab8a66d10f13p+0, 0x1.2b87fd0dad990p+0, 0x1.2c57e39771b2fp+0, \
-    0x1.2d285a6e4030bp+0, 0x1.2df961f641589p+0, 0x1.2ecafa93e2f56p+0, 0x1.2f9d24abd886bp+0, \
-    0x1.306fe0a31b715p+0, 0x1.31432edeeb2fdp+0, 0x1.32170fc4cd831p+0, 0x1.32eb83ba8ea32p+0, \
-    0x1.33c08b26416ffp+0, 0x1.3496266e3fa2dp+0, 0x1.356c55f929ff1p+0, 0x1.36431a2de883bp+0, \
-    0x1.371a7373aa9cbp+0, 0x1.37f26231e754ap+0, 0x1.38cae6d05d866p+0, 0x1.39a401b7140efp+0, \
-    0x1.3a7db34e59ff7p+0, 0x1.3b57fbfec6cf4p+0, 0x1.3c32dc313a8e5p+0, 0x1.3d0e544ede173p+0, \
-    0x1.3dea64c123422p+0, 0x1.3ec70df1c5175p+0, 0x1.3fa4504ac801cp+0, 0x1.40822c367a024p+0, \
-    0x1.4160a21f72e2ap+0, 0x1.423fb2709468ap+0, 0x1.431f5d950a897p+0, 0x1.43ffa3f84b9d4p+0, \
-    0x1.44e086061892dp+0, 0x1.45c2042a7d232p+0, 0x1.46a41ed1d0057p+0, 0x1.4786d668b3237p+0, \
-    0x1.486a2b5c13cd0p+0, 0x1.494e1e192aed2p+0, 0x1.4a32af0d7d3dep+0, 0x1.4b17dea6db7d7p+0, \
-    0x1.4bfdad5362a27p+0, 0x1.4ce41b817c114p+0, 0x1.4dcb299fddd0dp+0, 0x1.4eb2d81d8abffp+0, \
-    0x1.4f9b2769d2ca7p+0, 0x1.508417f4531eep+0, 0x1.516daa2cf6642p+0, 0x1.5257de83f4eefp+0, \
-    0x1.5342b569d4f82p+0, 0x1.542e2f4f6ad27p+0, 0x1.551a4ca5d920fp+0, 0x1.56070dde910d2p+0, \
-    0x1.56f4736b527dap+0, 0x1.57e27dbe2c4cfp+0, 0x1.58d12d497c7fdp+0, 0x1.59c0827ff07ccp+0, \
-    0x1.5ab07dd485429p+0, 0x1.5ba11fba87a03p+0, 0x1.5c9268a5946b7p+0, 0x1.5d84590998b93p+0, \
-    0x1.5e76f15ad2148p+0, 0x1.5f6a320dceb71p+0, 0x1.605e1b976dc09p+0, 0x1.6152ae6cdf6f4p+0, \
-    0x1.6247eb03a5585p+0, 0x1.633dd1d1929fdp+0, 0x1.6434634ccc320p+0, 0x1.652b9febc8fb7p+0, \
-    0x1.6623882552225p+0, 0x1.671c1c70833f6p+0, 0x1.68155d44ca973p+0, 0x1.690f4b19e9538p+0, \
-    0x1.6a09e667f3bcdp+0, 0x1.6b052fa75173ep+0, 0x1.6c012750bdabfp+0, 0x1.6cfdcddd47645p+0, \
-    0x1.6dfb23c651a2fp+0, 0x1.6ef9298593ae5p+0, 0x1.6ff7df9519484p+0, 0x1.70f7466f42e87p+0, \
-    0x1.71f75e8ec5f74p+0, 0x1.72f8286ead08ap+0, 0x1.73f9a48a58174p+0, 0x1.74fbd35d7cbfdp+0, \
-    0x1.75feb564267c9p+0, 0x1.77024b1ab6e09p+0, 0x1.780694fde5d3fp+0, 0x1.790b938ac1cf6p+0, \
-    0x1.7a11473eb0187p+0, 0x1.7b17b0976cfdbp+0, 0x1.7c1ed0130c132p+0, 0x1.7d26a62ff86f0p+0, \
-    0x1.7e2f336cf4e62p+0, 0x1.7f3878491c491p+0, 0x1.80427543e1a12p+0, 0x1.814d2add106d9p+0, \
-    0x1.82589994cce13p+0, 0x1.8364c1eb941f7p+0, 0x1.8471a4623c7adp+0, 0x1.857f4179f5b21p+0, \
-    0x1.868d99b4492edp+0, 0x1.879cad931a436p+0, 0x1.88ac7d98a6699p+0, 0x1.89bd0a478580fp+0, \
-    0x1.8ace5422aa0dbp+0, 0x1.8be05bad61778p+0, 0x1.8cf3216b5448cp+0, 0x1.8e06a5e0866d9p+0, \
-    0x1.8f1ae99157736p+0, 0x1.902fed0282c8ap+0, 0x1.9145b0b91ffc6p+0, 0x1.925c353aa2fe2p+0, \
-    0x1.93737b0cdc5e5p+0, 0x1.948b82b5f98e5p+0, 0x1.95a44cbc8520fp+0, 0x1.96bdd9a7670b3p+0, \
-    0x1.97d829fde4e50p+0, 0x1.98f33e47a22a2p+0, 0x1.9a0f170ca07bap+0, 0x1.9b2bb4d53fe0dp+0, \
-    0x1.9c49182a3f090p+0, 0x1.9d674194bb8d5p+0, 0x1.9e86319e32323p+0, 0x1.9fa5e8d07f29ep+0, \
-    0x1.a0c667b5de565p+0, 0x1.a1e7aed8eb8bbp+0, 0x1.a309bec4a2d33p+0, 0x1.a42c980460ad8p+0, \
-    0x1.a5503b23e255dp+0, 0x1.a674a8af46052p+0, 0x1.a799e1330b358p+0, 0x1.a8bfe53c12e59p+0, \
-    0x1.a9e6b5579fdbfp+0, 0x1.ab0e521356ebap+0, 0x1.ac36bbfd3f37ap+0, 0x1.ad5ff3a3c2774p+0, \
-    0x1.ae89f995ad3adp+0, 0x1.afb4ce622f2ffp+0, 0x1.b0e07298db666p+0, 0x1.b20ce6c9a8952p+0, \
-    0x1.b33a2b84f15fbp+0, 0x1.b468415b749b1p+0, 0x1.b59728de5593ap+0, 0x1.b6c6e29f1c52ap+0, \
-    0x1.b7f76f2fb5e47p+0, 0x1.b928cf22749e4p+0, 0x1.ba5b030a1064ap+0, 0x1.bb8e0b79a6f1fp+0, \
-    0x1.bcc1e904bc1d2p+0, 0x1.bdf69c3f3a207p+0, 0x1.bf2c25bd71e09p+0, 0x1.c06286141b33dp+0, \
-    0x1.c199bdd85529cp+0, 0x1.c2d1cd9fa652cp+0, 0x1.c40ab5fffd07ap+0, 0x1.c544778fafb22p+0, \
-    0x1.c67f12e57d14bp+0, 0x1.c7ba88988c933p+0, 0x1.c8f6d9406e7b5p+0, 0x1.ca3405751c4dbp+0, \
-    0x1.cb720dcef9069p+0, 0x1.ccb0f2e6d1675p+0, 0x1.cdf0b555dc3fap+0, 0x1.cf3155b5bab74p+0, \
-    0x1.d072d4a07897cp+0, 0x1.d1b532b08c968p+0, 0x1.d2f87080d89f2p+0, 0x1.d43c8eacaa1d6p+0, \
-    0x1.d5818dcfba487p+0, 0x1.d6c76e862e6d3p+0, 0x1.d80e316c98398p+0, 0x1.d955d71ff6075p+0, \
-    0x1.da9e603db3285p+0, 0x1.dbe7cd63a8315p+0, 0x1.dd321f301b460p+0, 0x1.de7d5641c0658p+0, \
-    0x1.dfc97337b9b5fp+0, 0x1.e11676b197d17p+0, 0x1.e264614f5a129p+0, 0x1.e3b333b16ee12p+0, \
-    0x1.e502ee78b3ff6p+0, 0x1.e653924676d76p+0, 0x1.e7a51fbc74c83p+0, 0x1.e8f7977cdb740p+0, \
-    0x1.ea4afa2a490dap+0, 0x1.eb9f4867cca6ep+0, 0x1.ecf482d8e67f1p+0, 0x1.ee4aaa2188510p+0, \
-    0x1.efa1bee615a27p+0, 0x1.f0f9c1cb6412ap+0, 0x1.f252b376bba97p+0, 0x1.f3ac948dd7274p+0, \
-    0x1.f50765b6e4540p+0, 0x1.f6632798844f8p+0, 0x1.f7bfdad9cbe14p+0, 0x1.f91d802243c89p+0, \
-    0x1.fa7c1819e90d8p+0, 0x1.fbdba3692d514p+0, 0x1.fd3c22b8f71f1p+0, 0x1.fe9d96b2a23d9p+0, \
+    0x8000000000000000ull, 0x8058d7d2d5e5f6b1ull, 0x80b1ed4fd999ab6cull, 0x810b40a1d81406d4ull, \
+    0x8164d1f3bc030773ull, 0x81bea1708dde6056ull, 0x8218af4373fc25ecull, 0x8272fb97b2a5894cull, \
+    0x82cd8698ac2ba1d7ull, 0x83285071e0fc4547ull, 0x8383594eefb6ee37ull, 0x83dea15b9541b132ull, \
+    0x843a28c3acde4046ull, 0x8495efb3303efd30ull, 0x84f1f656379c1a29ull, 0x854e3cd8f9c8c95dull, \
+    0x85aac367cc487b15ull, 0x86078a2f23642a9full, 0x8664915b923fba04ull, 0x86c1d919caef5c88ull, \
+    0x871f61969e8d1010ull, 0x877d2afefd4e256cull, 0x87db357ff698d792ull, 0x88398146b919f1d4ull, \
+    0x88980e8092da8527ull, 0x88f6dd5af155ac6bull, 0x8955ee03618e5fddull, 0x89b540a7902557a4ull, \
+    0x8a14d575496efd9aull, 0x8a74ac9a79896e47ull, 0x8ad4c6452c728924ull, 0x8b3522a38e1e1032ull, \
+    0x8b95c1e3ea8bd6e7ull, 0x8bf6a434adde0085ull, 0x8c57c9c4646f4ddeull, 0x8cb932c1bae97a95ull, \
+    0x8d1adf5b7e5ba9e6ull, 0x8d7ccfc09c50e2f8ull, 0x8ddf042022e69cd6ull, 0x8e417ca940e35a01ull, \
+    0x8ea4398b45cd53c0ull, 0x8f073af5a2013520ull, 0x8f6a8117e6c8e5c4ull, 0x8fce0c21c6726481ull, \
+    0x9031dc431466b1dcull, 0x9095f1abc540ca6bull, 0x90fa4c8beee4b12bull, 0x915eed13c89689d3ull, \
+    0x91c3d373ab11c336ull, 0x9228ffdc10a051adull, 0x928e727d9531f9acull, 0x92f42b88f673aa7cull, \
+    0x935a2b2f13e6e92cull, 0x93c071a0eef94bc1ull, 0x9426ff0fab1c04b6ull, 0x948dd3ac8ddb7ed3ull, \
+    0x94f4efa8fef70961ull, 0x955c5336887894d5ull, 0x95c3fe86d6cc7fefull, 0x962bf1cbb8d97560ull, \
+    0x96942d3720185a00ull, 0x96fcb0fb20ac4ba3ull, 0x97657d49f17ab08eull, 0x97ce9255ec4357abull, \
+    0x9837f0518db8a96full, 0x98a1976f7597e996ull, 0x990b87e266c189aaull, 0x9975c1dd47518c77ull, \
+    0x99e0459320b7fa65ull, 0x9a4b13371fd166caull, 0x9ab62afc94ff864aull, 0x9b218d16f441d63dull, \
+    0x9b8d39b9d54e5539ull, 0x9bf93118f3aa4cc1ull, 0x9c6573682ec32c2dull, 0x9cd200db8a0774cbull, \
+    0x9d3ed9a72cffb751ull, 0x9dabfdff6367a2aaull, 0x9e196e189d472420ull, 0x9e872a276f0b98ffull, \
+    0x9ef5326091a111aeull, 0x9f6386f8e28ba651ull, 0x9fd228256400dd06ull, 0xa041161b3d0121beull, \
+    0xa0b0510fb9714fc2ull, 0xa11fd9384a344cf7ull, 0xa18faeca8544b6e4ull, 0xa1ffd1fc25cea188ull, \
+    0xa27043030c496819ull, 0xa2e102153e918f9eull, 0xa3520f68e802bb93ull, 0xa3c36b345991b47cull, \
+    0xa43515ae09e6809eull, 0xa4a70f0c95768ec5ull, 0xa5195786be9ef339ull, 0xa58bef536dbeb6eeull, \
+    0xa5fed6a9b15138eaull, 0xa6720dc0be08a20cull, 0xa6e594cfeee86b1eull, 0xa7596c0ec55ff55bull, \
+    0xa7cd93b4e965356aull, 0xa8420bfa298f70d1ull, 0xa8b6d5167b320e09ull, 0xa92bef41fa77771bull, \
+    0xa9a15ab4ea7c0ef8ull, 0xaa1717a7b5693979ull, 0xaa8d2652ec907629ull, 0xab0386ef48868de1ull, \
+    0xab7a39b5a93ed337ull, 0xabf13edf162675e9ull, 0xac6896a4be3fe929ull, 0xace0413ff83e5d04ull, \
+    0xad583eea42a14ac6ull, 0xadd08fdd43d01491ull, 0xae493452ca35b80eull, 0xaec22c84cc5c9465ull, \
+    0xaf3b78ad690a4375ull, 0xafb51906e75b8661ull, 0xb02f0dcbb6e04584ull, 0xb0a957366fb7a3c9ull, \
+    0xb123f581d2ac2590ull, 0xb19ee8e8c94feb09ull, 0xb21a31a66618fe3bull, 0xb295cff5e47db4a4ull, \
+    0xb311c412a9112489ull, 0xb38e0e38419fae18ull, 0xb40aaea2654b9841ull, 0xb487a58cf4a9c180ull, \
+    0xb504f333f9de6484ull, 0xb58297d3a8b9f0d2ull, 0xb60093a85ed5f76cull, 0xb67ee6eea3b22b8full, \
+    0xb6fd91e328d17791ull, 0xb77c94c2c9d725e9ull, 0xb7fbefca8ca41e7cull, 0xb87ba337a1743834ull, \
+    0xb8fbaf4762fb9ee9ull, 0xb97c143756844dbfull, 0xb9fcd2452c0b9debull, 0xba7de9aebe5fea09ull, \
+    0xbaff5ab2133e45fbull, 0xbb81258d5b704b6full, 0xbc034a7ef2e9fb0dull, 0xbc85c9c560e7b269ull, \
+    0xbd08a39f580c36bfull, 0xbd8bd84bb67ed483ull, 0xbe0f6809860993e2ull, 0xbe935317fc378238ull, \
+    0xbf1799b67a731083ull, 0xbf9c3c248e2486f8ull, 0xc0213aa1f0d08db0ull, 0xc0a6956e8836ca8dull, \
+    0xc12c4cca66709456ull, 0xc1b260f5ca0fbb33ull, 0xc238d2311e3d6673ull, 0xc2bfa0bcfad907c9ull, \
+    0xc346ccda24976407ull, 0xc3ce56c98d21b15dull, 0xc4563ecc5334cb33ull, 0xc4de8523c2c07baaull, \
+    0xc5672a115506daddull, 0xc5f02dd6b0bbc3d9ull, 0xc67990b5aa245f79ull, 0xc70352f04336c51eull, \
+    0xc78d74c8abb9b15dull, 0xc817f681416452b2ull, 0xc8a2d85c8ffe2c45ull, 0xc92e1a9d517f0eccull, \
+    0xc9b9bd866e2f27a3ull, 0xca45c15afcc72624ull, 0xcad2265e4290774eull, 0xcb5eecd3b38597c9ull, \
+    0xcbec14fef2727c5dull, 0xcc799f23d11510e5ull, 0xcd078b86503dcdd2ull, 0xcd95da6a9ff06445ull, \
+    0xce248c151f8480e4ull, 0xceb3a0ca5dc6a55dull, 0xcf4318cf191918c1ull, 0xcfd2f4683f94eeb5ull, \
+    0xd06333daef2b2595ull, 0xd0f3d76c75c5db8dull, 0xd184df6251699ac6ull, 0xd2164c023056bcabull, \
+    0xd2a81d91f12ae45aull, 0xd33a5457a3029054ull, 0xd3ccf099859ac379ull, 0xd45ff29e0972c561ull, \
+    0xd4f35aabcfedfa1full, 0xd5872909ab75d18aull, 0xd61b5dfe9f9bce07ull, 0xd6aff9d1e13ba2feull, \
+    0xd744fccad69d6af4ull, 0xd7da67311797f56aull, 0xd870394c6db32c84ull, 0xd9067364d44a929cull, \
+    0xd99d15c278afd7b6ull, 0xda3420adba4d8704ull, 0xdacb946f2ac9cc72ull, 0xdb63714f8e295255ull, \
+    0xdbfbb797daf23755ull, 0xdc9467913a4f1c92ull, 0xdd2d818508324c20ull, 0xddc705bcd378f7f0ull, \
+    0xde60f4825e0e9124ull, 0xdefb4e1f9d1037f2ull, 0xdf9612deb8f04420ull, 0xe031430a0d99e627ull, \
+    0xe0ccdeec2a94e111ull, 0xe168e6cfd3295d23ull, 0xe2055afffe83d369ull, 0xe2a23bc7d7d91226ull, \
+    0xe33f8972be8a5a51ull, 0xe3dd444c46499619ull, 0xe47b6ca0373da88dull, 0xe51a02ba8e26d681ull, \
+    0xe5b906e77c8348a8ull, 0xe658797368b3a717ull, 0xe6f85aaaee1fce22ull, 0xe798aadadd5b9cbfull, \
+    0xe8396a503c4bdc68ull, 0xe8da9958464b42abull, 0xe97c38406c4f8c57ull, 0xea1e4756550eb27bull, \
+    0xeac0c6e7dd24392full, 0xeb63b74317369840ull, 0xec0718b64c1cbddcull, 0xecaaeb8ffb03ab41ull, \
+    0xed4f301ed9942b84ull, 0xedf3e6b1d418a491ull, 0xee990f980da3025bull, 0xef3eab20e032bc6bull, \
+    0xefe4b99bdcdaf5cbull, 0xf08b3b58cbe8b76aull, 0xf13230a7ad094509ull, 0xf1d999d8b7708cc1ull, \
+    0xf281773c59ffb13aull, 0xf329c9233b6bae9cull, 0xf3d28fde3a641a5bull, 0xf47bcbbe6db9fddfull, \
+    0xf5257d152486cc2cull, 0xf5cfa433e6537290ull, 0xf67a416c733f846eull, 0xf7255510c4288239ull, \
+    0xf7d0df730ad13bb9ull, 0xf87ce0e5b2094d9cull, 0xf92959bb5dd4ba74ull, 0xf9d64a46eb939f35ull, \
+    0xfa83b2db722a033aull, 0xfb3193cc4227c3f4ull, 0xfbdfed6ce5f09c49ull, 0xfc8ec01121e447bbull, \
+    0xfd3e0c0cf486c175ull, 0xfdedd1b496a89f35ull, 0xfe9e115c7b8f884cull, 0xff4ecb59511ec8a5ull, \
 }
 
 GDTK_HD int64_t gdtk_bits(double x) {
@@ -130,66 +133,105 @@ GDTK_HD double gdtk_fma(double a, double b, double c) {
 #endif
 }
 
-GDTK_HD double gdtk_exp(double x, const double* tab) {
-    const double INV_L = 0x1.71547652b82fep+8;   // 256 / ln 2
-    const double L1 = 0x1.62e42fee00000p-9;      // ln2/256, leading 32 bits
-    const double L2 = 0x1.a39ef35793c76p-41;     // ln2/256 - L1
-    const double SHIFT = 0x1.8p52;               // round-to-integer shift
-    // |x| < 512 (biased exponent below 1032), tested on the bits: the result is normal and the
-    // scaling below needs no range check.  NaN, infinities and the range ends take the compares.
-    const bool inner = ((gdtk_bits(x) >> 52) & 0x7ff) < 1032;
-    if (!inner) {
-        if (!(x > -745.1332191019412)) return x != x ? x : 0.0;
-        if (x > 709.782712893384) return x * 0x1p1023;   // +inf
+// ---------------------------------------------------------------- 64-bit products on the integer pipe
+GDTK_HD uint64_t gdtk_mul32(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+GDTK_HD uint32_t gdtk_mulhi32(uint32_t a, uint32_t b) {
+#ifdef __CUDA_ARCH__
+    return __umulhi(a, b);
+#else
+    return (uint32_t)(((uint64_t)a * b) >> 32);
+#endif
+}
+// High 64 bits of a b without the lowest partial product's carry: at most 3 below the exact value.
+GDTK_HD uint64_t gdtk_mulhi64(uint64_t a, uint64_t b) {
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+    return gdtk_mul32(ah, bh) + gdtk_mulhi32(ah, bl) + gdtk_mulhi32(al, bh);
+}
+
+GDTK_HD double gdtk_exp(double x, const uint64_t* tab) {
+    const uint64_t b = (uint64_t)gdtk_bits(x);
+    const uint32_t hi = (uint32_t)(b >> 32), e = (hi >> 20) & 0x7ff;
+    if (e >= 1033u) {   // |x| >= 1024, infinite or NaN
+        if ((b & 0x7fffffffffffffffull) > 0x7ff0000000000000ull) return x;
+        return (hi >> 31) ? 0.0 : gdtk_from_bits(0x7ff0000000000000LL);
     }
-    double t = gdtk_fma(x, INV_L, SHIFT);
-    int k = (int)(uint32_t)(gdtk_bits(t) & 0xffffffff);
-    double kd = t - SHIFT;
-    double r = gdtk_fma(-kd, L1, x);
-    r = gdtk_fma(-kd, L2, r);
-    double r2 = r * r;
-    double q = gdtk_fma(1.0 / 24.0, r, 1.0 / 6.0);
-    q = gdtk_fma(q, r, 0.5);
-    double p = gdtk_fma(r2, q, r);
-    double T = tab[k & 255];
-    double y = gdtk_fma(T, p, T);
-    int m = k >> 8;
-    if (inner || (m >= -1020 && m <= 1022)) return gdtk_from_bits(gdtk_bits(y) + ((int64_t)m << 52));
+    // X = |x| 2^54 (bits below are dropped)
+    const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;
+    const uint32_t n = 1032u - e;
+    const uint64_t X = n > 63u ? 0 : m >> n;
+    // |x| log2(e) = k + f: X times log2(e) 2^63 to 96 bits, 2^117 standing for 1
+    const uint32_t xh = (uint32_t)(X >> 32), xl = (uint32_t)X, ch = 0xb8aa3b29u, cl = 0x5c17f0bcu;
+    const uint64_t p0 = gdtk_mul32(xl, cl);
+    const uint64_t p1 = gdtk_mul32(xh, cl) + (p0 >> 32);
+    const uint64_t p2 = gdtk_mul32(xl, ch) + (uint32_t)p1;
+    const uint64_t p3 = gdtk_mul32(xh, ch) + (p1 >> 32) + (p2 >> 32);
+    int k = (int)(p3 >> 53);
+    uint64_t f = (p3 << 11) | ((uint32_t)p2 >> 21);   // fraction, 2^64 standing for 1
+    if (hi >> 31) { k = -k - (f != 0); f = 0 - f; }
+    // 2^(f - j/256) = 1 + 2^-8 u (c1 + u (c2 + u (c3 + u (c4 + u c5)))), u the fraction below j in units of
+    // 2^-8, c_n = (ln 2)^n / n! 2^(-8 (n - 1)); c3..c5 and their products in units of 2^-51, the rest of 2^-64
+    const uint64_t u = f << 8;
+    const uint32_t u32 = (uint32_t)(u >> 32);
+    const uint32_t v = 1907106652u + gdtk_mulhi32(u32, 1290923u + gdtk_mulhi32(u32, 699u));
+    const uint64_t s = (2113054701612ull + gdtk_mulhi32(u32, v)) << 13;
+    const uint64_t q = gdtk_mulhi64(u, 0xb17217f7d1cf79acull + gdtk_mulhi64(u, s));
+    const uint64_t T = tab[(uint32_t)(f >> 56)];
+    const uint64_t M = T + (gdtk_mulhi64(T, q) >> 8);
+    const uint64_t r = (M >> 11) + ((M >> 10) & 1);   // 53 bits, rounded
+    if (k > -1022 && k < 1023) return gdtk_from_bits((int64_t)(r + ((uint64_t)(uint32_t)(k + 1022) << 52)));
+    if (k > 1023) return gdtk_from_bits(0x7ff0000000000000LL);
+    if (k < -1080) return 0.0;
     // near the ends of the range: scale in two exact-power steps (the second may round
     // into the subnormal range, as the true result does)
-    int m1 = m / 2, m2 = m - m1;
-    double s1 = gdtk_from_bits((int64_t)(1023 + m1) << 52);
-    double s2 = gdtk_from_bits((int64_t)(1023 + m2) << 52);
-    return (y * s1) * s2;
+    const double y = gdtk_from_bits((int64_t)(r + ((uint64_t)1022 << 52)));
+    const int m1 = k / 2, m2 = k - m1;
+    return (y * gdtk_from_bits((int64_t)(1023 + m1) << 52)) * gdtk_from_bits((int64_t)(1023 + m2) << 52);
 }
 
 #ifdef __CUDA_ARCH__
 static __device__ __noinline__ double gdtk_div_ieee(double a, double b) { return a / b; }
 #endif
 
-// a / b in FP64 in a few instructions: the hardware's approximate reciprocal y0
-// (rcp.approx.ftz.f64), one cubically convergent Newton-Raphson step y = y0 (1 + e + e^2),
-// e = 1 - b y0, then one correction of the quotient, q = a y + (a - b a y) y, whose remainder
-// term is exact in a fused multiply-add (P. Markstein, "Computation of elementary functions on
-// the IBM RISC System/6000 processor", IBM J. Res. Develop. 34(1):111-119, 1990).  The result is
-// within 1 ulp of the correctly rounded quotient (almost always equal to it) when b and the
-// quotient lie in [2^-999, 2^1001); outside that range, and for zero, infinite or NaN operands,
-// the IEEE division runs instead (one shared out-of-line copy).  Five FMA/multiplies, no branch
-// in the common case; the inline IEEE division is many times larger, and this kernel's loop is
-// limited by instruction fetch.
+// 2^64 / y for y = B / 2^63 in [1, 2), within a few units: the FP32 reciprocal of y's leading 24 bits
+// (rcp.approx.ftz.f32, relative error below 2^-21 in all) as a 32-bit fraction R0, then
+// R = R0 (1 + e + e^2) with e = 1 - y R0, whose error e^3 is below 2^-63.
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ uint64_t gdtk_rcp64(uint64_t B) {
+    float rf;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rf) : "f"(__uint_as_float(0x3f800001u + ((uint32_t)(B >> 40) & 0x7fffffu))));
+    // in [1/2, 1) whatever the approximation's last bit
+    const uint32_t R0 = (min(max(__float_as_uint(rf), 0x3f000000u), 0x3f7fffffu) << 8) | 0x80000000u;
+    const uint64_t T = gdtk_mul32((uint32_t)(B >> 32), R0) + gdtk_mulhi32((uint32_t)B, R0);
+    int64_t E = (int64_t)(0x8000000000000000ull - T);   // e 2^63, below 2^43
+    const int32_t E1 = (int32_t)(E >> 12);
+    E += (int64_t)((uint64_t)((int64_t)E1 * E1) >> 39);
+    const int32_t Eh = (int32_t)(E >> 11);
+    const int64_t c = (int64_t)Eh * (int64_t)(uint64_t)R0 + gdtk_mulhi32(R0, (uint32_t)E << 21);
+    return ((uint64_t)R0 << 32) + (uint64_t)(c >> 20);
+}
+#endif
+
+// a / b within 0.51 ulp (99.9% correctly rounded) on the integer pipe: the 64-bit reciprocal of b's
+// significand times a's, rounded once.  Operands and quotients that are not normal numbers (zero,
+// subnormal, infinite, NaN) take one shared out-of-line IEEE division; a zero numerator over a normal
+// divisor, which the rates of absent species give at every step, does not.
+// An FP64 instruction holds an SM's FP64 pipe for 19 cycles (76 for each of the four sub-partitions'
+// warps), so the reciprocal seed and 4 FP64 operations of a Newton-Raphson division took about 330
+// cycles; this takes about 100 of the integer pipe's, which runs beside it.
 GDTK_HD double gdtk_div(double a, double b) {
 #ifdef __CUDA_ARCH__
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
-    const double q = a * y;
-    const double res = __fma_rn(__fma_rn(-b, q, a), y, q);
-    const unsigned eb = (unsigned)(__double_as_longlong(b) >> 52) & 0x7ffu;
-    const unsigned eq = (unsigned)(__double_as_longlong(res) >> 52) & 0x7ffu;
-    if (eb - 24u < 2000u) {
-        if (eq - 24u < 2000u) return res;
-        if (a == 0.0) return q;   // a signed zero, as a / b
+    const uint64_t ua = (uint64_t)__double_as_longlong(a), ub = (uint64_t)__double_as_longlong(b);
+    const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
+    const uint32_t ea = (ha >> 20) & 0x7ff, eb = (hb >> 20) & 0x7ff;
+    uint64_t q = gdtk_mulhi64((ua << 11) | 0x8000000000000000ull, gdtk_rcp64((ub << 11) | 0x8000000000000000ull));
+    const uint32_t ge = (uint32_t)(q >> 63);      // the significands' quotient is in (1/2, 2), 2^63 standing for 1
+    q <<= 1 - ge;
+    const uint32_t ex = ea - eb + ge + 1021;      // exponent field less the leading bit's 1
+    const uint64_t sign = (uint64_t)((ha ^ hb) & 0x80000000u) << 32;
+    if (eb - 1u < 2046u) {
+        if (ea - 1u < 2046u && ex < 2045u)
+            return __longlong_as_double((long long)(((q >> 11) + ((q >> 10) & 1) + ((uint64_t)ex << 52)) | sign));
+        if ((ua << 1) == 0) return __longlong_as_double((long long)sign);
     }
     return gdtk_div_ieee(a, b);
 #else
@@ -197,44 +239,18 @@ GDTK_HD double gdtk_div(double a, double b) {
 #endif
 }
 
-// a / b within 2 ulp, one FMA cheaper than gdtk_div: the same reciprocal y (the approximation refined by
-// one cubically convergent Newton-Raphson step, within about 1 ulp of 1/b) times a, without the
-// quotient correction.  The same range rules and IEEE fallback as gdtk_div.  The chemistry kernel's
-// divisions need no more: its results are compared with the reference at 1e-8, not bitwise.
-GDTK_HD double gdtk_div_nr(double a, double b) {
+// 1 / b as gdtk_div, without the product.
+GDTK_HD double gdtk_rcp(double b) {
 #ifdef __CUDA_ARCH__
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
-    const double q = a * y;
-    const unsigned eb = (unsigned)(__double_as_longlong(b) >> 52) & 0x7ffu;
-    const unsigned eq = (unsigned)(__double_as_longlong(q) >> 52) & 0x7ffu;
-    if (eb - 24u < 2000u) {
-        if (eq - 24u < 2000u) return q;
-        if (a == 0.0) return q;
-    }
-    return gdtk_div_ieee(a, b);
+    const uint64_t ub = (uint64_t)__double_as_longlong(b);
+    const uint32_t hb = (uint32_t)(ub >> 32), eb = (hb >> 20) & 0x7ff;
+    uint64_t q = gdtk_rcp64((ub << 11) | 0x8000000000000000ull);   // 2^64 / y, in (2^63, 2^64), or 2^64 - few at y = 1
+    if (eb - 1u < 2044u && (ub << 12) != 0)
+        return __longlong_as_double((long long)((q >> 11) + ((q >> 10) & 1) + ((uint64_t)(2044u - eb) << 52)) |
+                                    (long long)((uint64_t)(hb & 0x80000000u) << 32));
+    return gdtk_div_ieee(1.0, b);
 #else
-    return a / b;
-#endif
-}
-
-// c + a / b with the quotient within 2 ulp: the refined reciprocal of gdtk_div_nr, then one fused
-// multiply-add a * (1/b) + c in place of gdtk_div_nr's multiply and a separate add.  The same range
-// rule on b and IEEE fallback as gdtk_div_nr; a zero, infinite or NaN a propagates through the FMA
-// as through a / b.
-GDTK_HD double gdtk_add_div(double c, double a, double b) {
-#ifdef __CUDA_ARCH__
-    double y;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    const double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
-    const unsigned eb = (unsigned)(__double_as_longlong(b) >> 52) & 0x7ffu;
-    if (eb - 24u < 2000u) return __fma_rn(a, y, c);
-    return c + gdtk_div_ieee(a, b);
-#else
-    return c + a / b;
+    return 1.0 / b;
 #endif
 }
 

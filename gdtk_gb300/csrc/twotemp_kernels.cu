@@ -49,9 +49,9 @@ constexpr int MAX_EEM = 64;
 
 // exp by Tang's table method (fast_exp.h, within 1.3 ulp): 9 FP64 operations where the library's takes
 // about 20 FMA slots on this GPU.  The update kernel stages the table in shared memory once per block.
-__device__ const double kExp2Table[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
-__shared__ double s_exp2[GDTK_EXP2_TABLE_SIZE];
-__device__ __forceinline__ double ex(double x) { return gdtk_exp(x, s_exp2); }
+__device__ const uint64_t kExp2Table[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
+__shared__ uint64_t s_exp2[GDTK_EXP2_TABLE_SIZE];
+__device__ __noinline__ double ex(double x) { return gdtk_exp(x, s_exp2); }   // one copy: fetching inlined ones costs more
 
 // NASA-9 Cp, h and s of cea_thermo_curves.d:55-137 (cea_thermo.h's segment choice and blending,
 // cea_coeffs) in Horner form with the reciprocal temperature rT = 1 / T: the reference's divisions by T,
