@@ -319,25 +319,38 @@ void prepare_warp_path(ReactorObj& r, const PackedMech& pm) {
         return 2 * nr + (use_b ? nslot : 0) + j;
     };
     if (2 * nr + 2 * nslot > 0x2000) throw std::runtime_error("too many tick-rate terms for the warp-per-cell gather");
-    // tasks: the q and the L of each species, longest first onto the least-loaded lane (ties: lowest lane)
-    std::vector<int> order(2 * nsp);
-    for (int t = 0; t < 2 * nsp; ++t) order[t] = t;
-    std::stable_sort(order.begin(), order.end(),
-                     [&](int a, int b) { return per[a >> 1].size() > per[b >> 1].size(); });
-    std::vector<std::vector<int>> lane_tasks(32);
+    // tasks: the q and the L of each species; those longer than a lane's share of all entries are split into
+    // equal parts, whose later ones go to partial sums.  Longest first onto the least-loaded lane (ties: lowest)
+    struct Part { int target, isp; bool to_L; size_t lo, hi; };
+    std::vector<Part> parts;
+    std::vector<int> comb;
+    size_t total = 0;
+    for (auto& v : per) total += 2 * v.size();
+    const size_t share = std::max<size_t>(4, (total + 31) / 32);
+    int npart = 0;
+    for (int t = 0; t < 2 * nsp; ++t) {
+        const size_t len = per[t >> 1].size();
+        if (!len) continue;
+        size_t n = (len + share - 1) / share;
+        if (npart + (int)n - 1 > 128) n = 1;
+        if (n > 1) comb.push_back((t >> 1) | (t & 1) << 7 | npart << 8 | (int)(n - 1) << 16);
+        for (size_t k = 0; k < n; ++k)
+            parts.push_back({k == 0 ? t >> 1 : 128 + npart++, t >> 1, (t & 1) != 0, len * k / n, len * (k + 1) / n});
+    }
+    std::stable_sort(parts.begin(), parts.end(), [](const Part& a, const Part& b) { return a.hi - a.lo > b.hi - b.lo; });
+    std::vector<std::vector<int>> lane_parts(32);
     std::vector<size_t> load(32, 0);
-    for (int t : order) {
-        if (per[t >> 1].empty()) continue;
+    for (size_t k = 0; k < parts.size(); ++k) {
         const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        lane_tasks[l].push_back(t);
-        load[l] += per[t >> 1].size();
+        lane_parts[l].push_back((int)k);
+        load[l] += parts[k].hi - parts[k].lo;
     }
     std::vector<int> lane(33, 0), ent;
     for (int l = 0; l < 32; ++l) {
-        for (int t : lane_tasks[l]) {
-            const int isp = t >> 1;
-            const bool to_L = t & 1;
-            for (auto& e : per[isp]) ent.push_back(isp | index(e, to_L) << 8 | (to_L ? 1 : 0) << 21);
+        for (int k : lane_parts[l]) {
+            const Part& t = parts[k];
+            for (size_t j = t.lo; j < t.hi; ++j)
+                ent.push_back(t.target | index(per[t.isp][j], t.to_L) << 8 | (t.to_L ? 1 : 0) << 21);
         }
         lane[l + 1] = (int)ent.size();
     }
@@ -369,10 +382,13 @@ void prepare_warp_path(ReactorObj& r, const PackedMech& pm) {
     t.off_slot = put(slot);
     t.off_lane = put(lane);
     t.off_ent = put(ent);
+    t.off_comb = put(comb);
+    t.ncomb = (int)comb.size();
+    t.npart = npart;
     t.n_smem_ints = (int)all.size();
     t.off_efflen = put(efflen);
     t.off_effidx = put(effidx);
-    r.warp_doubles = chem_warp_doubles(nsp, nr, neff, pm.method, nslot);
+    r.warp_doubles = chem_warp_doubles(nsp, nr, neff, pm.method, nslot, npart);
     r.wt_i.ensure(all.size());
     r.wt_d.ensure(effval.size());
     check(cudaMemcpy(r.wt_i.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy");

@@ -748,20 +748,21 @@ __global__ void order_scatter(const float* key, int n, int* hist, int* order) {
 // consecutive words across lanes), and a species -> (reaction, coefficient) gather whose species are
 // dealt to the lanes longest first, so that the lanes' loops are about equally long.  Rate constants
 // and thermo read the packed mechanism from global memory (they need not fit in shared memory).
-// Every sum the reference takes over species in order (energies, gas constant, mass-fraction total,
-// RKF error norm) is taken by lane 0 in that order from per-species terms the lanes computed, and q, L
-// gather each species' terms in reaction order, the reference-order kernel's summation order.  This
-// translation unit is compiled with FMA contraction and its alpha-QSS step takes the two-division
+// Sums the reference takes over species in order (energies, gas constant, mass-fraction total,
+// RKF error norm) are taken by lane 0 in that order from per-species terms the lanes computed; q and L
+// gather each species' terms in reaction order, a long species' in parts, and third-body sums are spread
+// over lanes.  This translation unit is compiled with FMA contraction and its alpha-QSS step takes the two-division
 // form (w_aqss_step), so values agree with the reference-order kernel to rounding, not bitwise.
 // Minima and maxima (step estimate, sigma) are order-free.
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 struct WarpLayout {
-    int y0, yout, q, L, mf, g, tmp, kf, kb, wf, wb, wsf, wsb, meff, ext, total;
-    __device__ __host__ void make(int nsp, int nr, int neff, int method, int nslot) {
+    int y0, yout, q, L, mf, g, tmp, kf, kb, wf, wb, wsf, wsb, part, meff, ext, total;
+    __device__ __host__ void make(int nsp, int nr, int neff, int method, int nslot, int npart) {
         y0 = 0; yout = nsp; q = 2 * nsp; L = 3 * nsp; mf = 4 * nsp; g = 5 * nsp; tmp = 6 * nsp;
         kf = 8 * nsp; kb = kf + nr; wf = kb + nr; wb = wf + nr; wsf = wb + nr; wsb = wsf + nslot;
-        meff = wsb + nslot;
+        part = wsb + nslot;
+        meff = part + npart;
         ext = meff + (neff > 0 ? neff : 1);
         total = ext + (method == METHOD_RKF ? 7 * nsp : 4 * nsp);
     }
@@ -777,8 +778,11 @@ struct WarpCtx {
     int nslot;
     double* wsf;            // the warp's |nu| w_f and |nu| w_b of each slot
     double* wsb;
+    double* part;           // the warp's partial q and L of split tasks
     int ent_lo, ent_hi;     // this lane's gather entries
-    const int* ent;         // shared: species | index << 8 | L << 21 | source << 22
+    const int* ent;         // shared: target | index << 8 | L << 21
+    const int* comb;        // shared: species | L << 7 | first part << 8 | number of parts << 16, per split task
+    int ncomb;
     const int* efflen;      // global: length of each efficiency list
     const int* effidx;      // global, [k][neff]: species of entry k of each list
     const double* effval;   // global, [k][neff]: its efficiency
@@ -848,11 +852,18 @@ __device__ void w_split_rates(const WarpCtx& w, const double* c, double* q, doub
                               const double* kb, double* wf, double* wb, double* meff) {
     const MechView& m = w.m;
     const int neff = m.neff;
-    for (int s = w.lane; s < neff; s += 32) {   // reaction.d:450-456, in the list's order
-        const int len = w.efflen[s];
+    // third bodies (reaction.d:450-456): the lists spread over all lanes, 2^n lanes to a list
+    int per = 1;
+    while (2 * per * neff <= 32) per *= 2;
+    for (int s0 = 0; s0 < neff; s0 += 32 / per) {
+        const int s = s0 + w.lane / per;
         double term = 0.0;
-        for (int k = 0; k < len; ++k) term += w.effval[k * neff + s] * c[w.effidx[k * neff + s]];
-        meff[s] = term;
+        if (s < neff) {
+            const int len = w.efflen[s];
+            for (int k = w.lane & (per - 1); k < len; k += per) term = fma(w.effval[k * neff + s], c[w.effidx[k * neff + s]], term);
+        }
+        for (int o = 1; o < per; o <<= 1) term += __shfl_xor_sync(FULL_MASK, term, o);
+        if (s < neff && !(w.lane & (per - 1))) meff[s] = term;
     }
     for (int i = w.lane; i < m.nsp; i += 32) { q[i] = 0.0; L[i] = 0.0; }
     __syncwarp();
@@ -875,20 +886,36 @@ __device__ void w_split_rates(const WarpCtx& w, const double* c, double* q, doub
     }
     __syncwarp();
     // q, L: each of this lane's tasks adds its terms in reaction order from 0 (reaction_mechanism.d:82-96);
-    // an entry's index runs over w_f, w_b and the slots' |nu| w_f, |nu| w_b, which lie end to end
+    // an entry's index runs over w_f, w_b and the slots' |nu| w_f, |nu| w_b, which lie end to end.  A task that
+    // is longer than a lane's fair share (a long species of the acetylene model, H, has 187 terms) is split; its later
+    // parts go to w.part and are added below.
     int cur = -1;
     double sum = 0.0;
+    auto flush = [&]() {
+        if (cur & 0x80) w.part[cur & 0x7f] = sum;
+        else ((cur >> 21) ? L : q)[cur & 0x7f] = sum;
+    };
     for (int k = w.ent_lo; k < w.ent_hi; ++k) {
         const int e = w.ent[k];
-        const int key = e & 0x2000ff;   // species and the q / L bit
+        const int key = e & 0x2000ff;   // target and the q / L bit
+        const double v = wf[(e >> 8) & 0x1fff];
         if (key != cur) {
-            if (cur >= 0) ((cur >> 21) ? L : q)[cur & 0xff] = sum;
+            if (cur >= 0) flush();
             cur = key;
-            sum = 0.0;
+            sum = v;
+        } else {
+            sum += v;
         }
-        sum += wf[(e >> 8) & 0x1fff];
     }
-    if (cur >= 0) ((cur >> 21) ? L : q)[cur & 0xff] = sum;
+    if (cur >= 0) flush();
+    __syncwarp();
+    for (int k = w.lane; k < w.ncomb; k += 32) {
+        const int e = w.comb[k], first = (e >> 8) & 0xff, n = e >> 16;
+        double* dst = ((e & 0x80) ? L : q) + (e & 0x7f);
+        double v = *dst;
+        for (int j = 0; j < n; ++j) v += w.part[first + j];
+        *dst = v;
+    }
     __syncwarp();
 }
 
@@ -1031,8 +1058,24 @@ __device__ bool w_rkf_step(const WarpCtx& w, const double* y0, double h, double*
 // alpha = N(s) / D(s), s = p h: chemistry_update.d:599-604's rational function of r = 1 / (p h + eps) with
 // numerator and denominator multiplied by s^3 (no division by s, so the reference's eps, which guards its
 // 1 / (p h), changes nothing above s = 1e-34); s is capped at 1e50, where the ratio is 1 to double precision.
+// a < b of doubles that are >= +0 (or NaN, above all), on the integer pipe: an FP64 compare costs an FMA's slot
+__device__ __forceinline__ bool w_below(double a, double b) {
+    return (unsigned long long)__double_as_longlong(a) < (unsigned long long)__double_as_longlong(b);
+}
+__device__ __forceinline__ bool w_nan(double a) {
+    return (__double_as_longlong(a) & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL;
+}
+// p = L / (c + eps): the sum is c itself above 1e-34
+__device__ __forceinline__ double w_qss_p(double L, double c) {
+    return gdtk_div(L, __double_as_longlong(c) > __double_as_longlong(1.0e-30) ? c : c + ZERO_EPS);
+}
+// yc is no species below eps: negative values and -0 have the sign bit, NaN none below eps
+__device__ __forceinline__ bool w_present(double yc) {
+    const long long b = __double_as_longlong(yc);
+    return b >= __double_as_longlong(ZERO_EPS) || w_nan(yc);
+}
 __device__ __forceinline__ void w_alpha_nd(double s, double& N, double& D) {
-    s = fmin(s, 1.0e50);
+    s = w_below(s, 1.0e50) ? s : 1.0e50;
     N = fma(s, fma(s, 11.0 + s, 60.0), 180.0);
     D = fma(s, s, N + 180.0);   // s^3 + 12 s^2 + 60 s + 360
 }
@@ -1054,7 +1097,7 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
     for (int i = w.lane; i < n; i += 32) {
         const double y = y0[i];
         const double qi = q[i];
-        const double pi = gdtk_div(L[i], y + ZERO_EPS);
+        const double pi = w_qss_p(L[i], y);
         double N, D;
         w_alpha_nd(pi * h, N, D);
         const double v = y + gdtk_div(h * (D * fma(-pi, y, qi)), fma(N, h * pi, D));
@@ -1068,15 +1111,15 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
         bool conv = true;
         for (int i = w.lane; i < n; i += 32) {
             const double y = y0[i];
-            const double pp = gdtk_div(L[i], yp[i] + ZERO_EPS);
+            const double pp = w_qss_p(L[i], yp[i]);
             double N, D;
             w_alpha_nd(pp * h, N, D);
             const double pb = fma(0.5, pp, p0[i]);
             const double yc = y + gdtk_div(h * fma(N, q[i] - q0[i], D * fma(-pb, y, q0[i])), fma(N, h * pb, D));
             yp[i] = yc;
-            if (!(yc < ZERO_EPS)) {
-                const double test = fabs(yc - yp0[i]);
-                if (test >= fma(eps1, yc, eps1 * delta)) conv = false;
+            if (w_present(yc)) {
+                const double test = fabs(yc - yp0[i]), tol = fma(eps1, yc, eps1 * delta);
+                if (!w_below(test, tol) && !w_nan(test)) conv = false;
             }
         }
         __syncwarp();
@@ -1086,11 +1129,12 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
     double snum = 0.0, sden = 1.0;   // this lane's largest |yc - yp0| / (eps2 (yc + delta))
     for (int i = w.lane; i < n; i += 32) {
         const double yc = yp[i];
-        if (yc < ZERO_EPS) continue;
+        if (!w_present(yc)) continue;
         const double num = fabs(yc - yp0[i]), den = fma(eps2, yc, eps2 * delta);
-        if (num * sden > snum * den) { snum = num; sden = den; }
+        const double a = num * sden, b = snum * den;
+        if (w_below(b, a) && !w_nan(a)) { snum = num; sden = den; }
     }
-    double sigma = snum / sden;
+    double sigma = gdtk_div(snum, sden);
     for (int o = 16; o > 0; o >>= 1) {
         const double other = __shfl_xor_sync(FULL_MASK, sigma, o);
         if (other > sigma) sigma = other;
@@ -1134,10 +1178,13 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
     w.effval = tb.eff_val;
     const MechView& m = w.m;
     WarpLayout lay;
-    lay.make(m.nsp, m.nr, m.neff, METHOD, tb.nslot);
+    lay.make(m.nsp, m.nr, m.neff, METHOD, tb.nslot, tb.npart);
     double* S = smem_w + (tb.n_smem_ints + 1) / 2 + (size_t)(threadIdx.x >> 5) * warp_doubles;
     w.wsf = S + lay.wsf;
     w.wsb = S + lay.wsb;
+    w.part = S + lay.part;
+    w.comb = ti + tb.off_comb;
+    w.ncomb = tb.ncomb;
     double *y0 = S + lay.y0, *yout = S + lay.yout, *q = S + lay.q, *L = S + lay.L, *mf = S + lay.mf, *g = S + lay.g,
            *tmp = S + lay.tmp, *kf = S + lay.kf, *kb = S + lay.kb, *wf = S + lay.wf, *wb = S + lay.wb,
            *meff = S + lay.meff, *ext = S + lay.ext;
@@ -1325,9 +1372,9 @@ cudaError_t launch_bucket_order(const float* key, int n, int* order, int* hist, 
 // ---------------------------------------------------------------- host-side launchers
 
 #if GDTK_WARP_TU
-int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot) {
+int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot, int npart) {
     WarpLayout l;
-    l.make(nsp, nr, neff, method, nslot);
+    l.make(nsp, nr, neff, method, nslot, npart);
     return l.total;
 }
 

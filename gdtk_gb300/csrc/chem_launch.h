@@ -64,10 +64,12 @@ cudaError_t launch_gas_service(const GasServiceArgs& a, int sm_count, cudaStream
 //     [off_rxeff + ir]   efficiency list of reaction ir's third body, or -1
 //     [off_slot + j]     scaled tick-rate slot j: reaction | |nu| << 16, for each (reaction, |nu| >= 2) pair
 //     [off_lane + l]     first gather entry of lane l (33 entries)
-//     [off_ent + k]      gather entry: species | index << 8 | (1 for L) << 21, adding element `index` of
+//     [off_ent + k]      gather entry: target | index << 8 | (1 for L) << 21, adding element `index` of
 //                        the warp's w_f[nr], w_b[nr], |nu| w_f[nslot], |nu| w_b[nslot] (end to end) to q or
-//                        L of the species.  The tasks (one species' q, or its L) are dealt whole to the
-//                        lanes, longest first; a task's entries are in ascending reaction order
+//                        L of the species `target`, or to partial sum target - 128.  The tasks (one species' q,
+//                        or its L; those longer than a lane's share in parts) are dealt to the lanes,
+//                        longest first; a task's entries are in ascending reaction order
+//     [off_comb + k]     split task k: species | (1 for L) << 7 | first partial sum << 8 | their number << 16
 //   ints [off_efflen, ...) and doubles, read from global memory:
 //     [off_efflen + s]            length of efficiency list s
 //     [off_effidx + k*neff + s]   species of the k-th entry of list s (transposed: lanes read one list each)
@@ -75,11 +77,11 @@ cudaError_t launch_gas_service(const GasServiceArgs& a, int sm_count, cudaStream
 struct WarpTables {
     const int* gi;
     const double* eff_val;
-    int n_smem_ints, nslot;
-    int off_tstart, off_tmid, off_terms, off_rxeff, off_slot, off_lane, off_ent, off_efflen, off_effidx;
+    int n_smem_ints, nslot, npart, ncomb;
+    int off_tstart, off_tmid, off_terms, off_rxeff, off_slot, off_lane, off_ent, off_comb, off_efflen, off_effidx;
 };
 // Shared-memory doubles of one warp's vectors.
-int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot);
+int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot, int npart);
 cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables& t, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info);
 // Cost buckets of the longest-first ordering: launch_bucket_order's hist scratch holds this many ints.
