@@ -45,7 +45,7 @@ struct GrpTab {
     const double* eff;        // [NSETS][NSP] third-body efficiencies, 0 where absent
     const GrpKc* kc;
     const uint4* rx;
-    const uint2* ent;         // (tick-rate index, high word of the coefficient) of the q and L sums, task by task
+    const unsigned* ent;      // the terms of the q and L sums, task by task: tick-rate index, coefficient (codegen.cpp)
     const int* task;          // first entry of each task (2 NSP + 1); task 2 i is q_i, 2 i + 1 L_i
     const int* lane_start;    // per L (4, 8, 16, 32): first slot of each lane (L + 1)
     const int* lane_task;     // per L: the tasks in lane order
@@ -62,6 +62,17 @@ struct GrpCell {
 };
 
 constexpr unsigned GRP_FULL = 0xffffffffu;
+
+// e c with the roundings of the product, which most efficiencies, 1, do not need
+__device__ __forceinline__ double third_body(double e, double c) { return dbits(e) == dbits(1.0) ? c : __dmul_rn(e, c); }
+// x / 2 for x = 0 or normal x > 0
+__device__ __forceinline__ double half_nn(double x) {
+    return (unsigned long long)((dbits(x) >> 52) - 2) < 0x7fcULL ? __longlong_as_double(dbits(x) - (1LL << 52)) : 0.5 * x;
+}
+
+#if GDTK_METHOD == 0
+__constant__ int GRP_COEF_HI[8] = {0, 0x3ff00000, 0x40000000, 0x40080000, 0x40100000, 0x40140000, 0x40180000, 0x401c0000};
+#endif
 
 // sum over the species of leaf(i), the zero-padded pairwise tree of sum_pairwise; every lane gets it.
 template <int L, typename F>
@@ -172,19 +183,23 @@ __device__ __forceinline__ void grp_rate_constants(const GrpTab& tab, GrpCell& s
                 if (R.pw != 99) {
                     const double b = R.pw > 0 ? T : rT;
                     kf = R.A;
+#pragma unroll 1
                     for (int m = 0; m < abs(R.pw); ++m) kf *= b;
                 } else {
                     kf = gdtk_exp(fma(R.mC, rT, fma(R.n, lnT, R.lnA)), tab.ETAB);
                 }
-                double P = 1.0;
-                const double c = R.nusum > 0 ? cf : rcf;
-                for (int m = 0; m < abs(R.nusum); ++m) P *= c;
+                // P = (R T / P_atm)^sum(nu) prod E^nu from its first factor on
+                double P = R.nusum > 0 ? cf : rcf;
+                bool one = R.nusum == 0;   // no factor yet
+                for (int m = 1; m < abs(R.nusum); ++m) P *= R.nusum > 0 ? cf : rcf;
                 for (int k = 0; k < R.np; ++k) {
                     const int nk = R.anu[k];
                     const double v = (nk > 0 ? E : E + GDTK_NSP)[R.sp[k]];
-                    for (int m = 0; m < abs(nk); ++m) P *= v;
+                    int m = abs(nk);
+                    if (one) { P = v; one = false; --m; }
+                    for (; m > 0; --m) P *= v;
                 }
-                kb = kf * P;
+                kb = one ? kf : kf * P;
             } else
 #endif
             {
@@ -231,6 +246,45 @@ __device__ __forceinline__ double grp_ipow(double x, int n) {   // the order of 
     }
 }
 
+#if GDTK_METHOD != 0
+// The q and L sums of the alpha-QSS right-hand side on the integer pipe: a term takes about 22 cycles there, where
+// an FP64 addition takes 76 of the pipe that bounds the kernel (73% busy on the mixing layer), and the
+// terms do not wait for one another.  The terms, all >= 0, are aligned to the largest with 5 bits below its last
+// and the sum is rounded once, closer to the exact value than the chain of FP64 additions it replaces.
+// 262,147 H2-air cells 400 -> 364 ms, 32,000 with 16 lanes 80.7 -> 72.0.  The tick rates' products stay FP64:
+// on the integer pipe, with its conversions, they took 391 to 517 ms.
+// sum of the entries' W 2^shift (index | shift << 16)
+__device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1, const double* W) {
+    const unsigned* H = reinterpret_cast<const unsigned*>(W) + 1;
+    unsigned mx = 0;
+#pragma unroll 4
+    for (int e = e0; e < e1; ++e) {
+        const unsigned x = ent[e];
+        mx = max(mx, H[2 * (x & 0xffff)] + ((x >> 16) << 20));
+    }
+    if (mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {   // a normal largest term, far from the range's ends
+        const int E6 = (int)(mx >> 20) + 6;
+        uint64_t acc = 0;
+#pragma unroll 4
+        for (int e = e0; e < e1; ++e) {
+            const unsigned x = ent[e];
+            const uint64_t w = (uint64_t)dbits(W[x & 0xffff]);
+            const int we = (int)(w >> 52), d = E6 - we - (int)(x >> 16);
+            if (we != 0 && d < 64) acc += ((w << 11) | 0x8000000000000000ull) >> d;
+        }
+        const int c = __clzll((long long)acc);   // 1..6
+        acc <<= c;
+        return __longlong_as_double((long long)((acc >> 11) + ((acc >> 10) & 1) + ((uint64_t)(unsigned)(E6 - c - 1) << 52)));
+    }
+    double sum = 0.0;
+    for (int e = e0; e < e1; ++e) {
+        const unsigned x = ent[e];
+        sum = fma((double)(1u << (x >> 16)), W[x & 0xffff], sum);
+    }
+    return sum;
+}
+#endif
+
 // q and L of every species at the concentrations c into S[GO_Q..], S[GO_L..] (gen_rhs).
 template <int L>
 __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, const double* c, int gl, bool act) {
@@ -238,7 +292,7 @@ __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, con
 #pragma unroll 1
     for (int m = 0; m < GDTK_NSETS; ++m) {
         const double* ef = tab.eff + m * GDTK_NSP;
-        const double M = grp_sum<L>(gl, [&](int i) { return __dmul_rn(ef[i], c[i]); });
+        const double M = grp_sum<L>(gl, [&](int i) { return third_body(ef[i], c[i]); });
         if (act && gl == 0) S[GO_M + m] = M;
     }
     __syncwarp(GRP_FULL);
@@ -250,12 +304,12 @@ __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, con
             const uint4 x = tab.rx[r];
             const int id = x.w & 0xffff, set = x.w >> 16;
             double wf = K[id], wb = K[GDTK_NR + id];
+            const unsigned nf = x.z & 7, nb = (x.z >> 3) & 7;
             if (set) { const double M = S[GO_M + set - 1]; wf *= M; wb *= M; }
-            const int nf = x.z & 7, nb = (x.z >> 3) & 7;
             unsigned sp = x.x, co = x.z >> 6;
-            for (int k = 0; k < nf; ++k, sp >>= 8, co >>= 3) wf *= grp_ipow(c[sp & 255], co & 7);
+            for (unsigned k = 0; k < nf; ++k, sp >>= 8, co >>= 3) wf *= grp_ipow(c[sp & 255], co & 7);
             sp = x.y; co = x.z >> 18;
-            for (int k = 0; k < nb; ++k, sp >>= 8, co >>= 3) wb *= grp_ipow(c[sp & 255], co & 7);
+            for (unsigned k = 0; k < nb; ++k, sp >>= 8, co >>= 3) wb *= grp_ipow(c[sp & 255], co & 7);
             W[id] = wf;
             W[GDTK_NR + id] = wb;
         }
@@ -268,12 +322,22 @@ __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, con
 #pragma unroll 1
         for (int k = ls[gl]; k < ls[gl + 1]; ++k) {
             const int t = lt[k], e1 = tab.task[t + 1];
+#if GDTK_METHOD == 0
+            int e = tab.task[t];
             double acc = 0.0;
-#pragma unroll 4
-            for (int e = tab.task[t]; e < e1; ++e) {
-                const uint2 x = tab.ent[e];
-                acc = fma(__hiloint2double((int)x.y, 0), W[x.x], acc);
+            if (e < e1) {   // the first term: no sum, and no product by a coefficient of 1
+                const unsigned x = tab.ent[e++];
+                acc = W[x & 0xffff];
+                if (x >> 16 != 1) acc *= __hiloint2double(GRP_COEF_HI[x >> 16], 0);
             }
+#pragma unroll 4
+            for (; e < e1; ++e) {
+                const unsigned x = tab.ent[e];
+                acc = fma(__hiloint2double(GRP_COEF_HI[x >> 16], 0), W[x & 0xffff], acc);
+            }
+#else
+            const double acc = grp_gather(tab.ent, tab.task[t], e1, W);
+#endif
             S[((t & 1) ? GO_L : GO_Q) + (t >> 1)] = acc;
         }
     }
@@ -299,7 +363,16 @@ __device__ __forceinline__ void grp_mix_coeffs(const double* TH, const double* Y
 }
 #endif
 
-// T_from_u for the groups with `act`; YR and the scratch M (24 doubles) in the cell's slice.
+#if GDTK_MIX_THERMO
+// mix_H_Cp's H/R (odd false) or Cp/R (odd true), each in its own roundings: Cp/R starts from 0 T + c
+__device__ __forceinline__ double mix_H_or_Cp(const double* m, bool odd, double T, double lnT, double rT, double rT2) {
+    const double a6 = odd ? 0.0 : m[6], a5 = m[odd ? 11 : 5], a4 = m[odd ? 10 : 4], a3 = m[odd ? 9 : 3], a2 = m[odd ? 8 : 2];
+    const double h0 = odd ? -m[0] : m[0], e = m[odd ? 2 : 7];
+    return fma(T, fma(T, fma(T, fma(T, fma(T, a6, a5), a4), a3), a2), fma(h0, odd ? rT2 : rT, fma(m[1], odd ? rT : lnT, e)));
+}
+#endif
+
+// T_from_u for the groups with `act`; YR and the scratch M (24 doubles or 2 NSP) in the cell's slice.
 template <int L>
 __device__ __forceinline__ double grp_T_from_u(const GrpTab& tab, const double* YR, double* M, double u_tgt, double T_guess,
                                                double ysum, double& lnT_io, int& err, int& iters, int gl, bool act) {
@@ -327,14 +400,45 @@ __device__ __forceinline__ double grp_T_from_u(const GrpTab& tab, const double* 
         if (__any_sync(GRP_FULL, nb)) grp_mix_coeffs<L>(tab.TH, YR, sb, M + 12, gl, nb);
         if (na) seg_a = sa;
         if (nb) seg_b = sb;
-        if (mix) {
-            mix_f_cv(M, M + 12, 1, T, lnT, rT, rT2, wb, ysum, f, cv);
-        } else
+        if (__any_sync(GRP_FULL, mix)) {
+            // H/R on the even lanes and Cp/R on the odd ones: the same polynomial in T with other coefficients
+            const bool odd = gl & 1;
+            double v = 0.0;
+            if (mix) {
+                v = mix_H_or_Cp(M, odd, T, lnT, rT, rT2);
+                if (nonzero(wb)) v = fma(wb, mix_H_or_Cp(M + 12, odd, T, lnT, rT, rT2) - v, v);
+                v = fma(-ysum, odd ? 1.0 : T, v);
+            }
+            const double o = __shfl_xor_sync(GRP_FULL, v, 1);
+            f = odd ? o : v;
+            cv = odd ? v : o;
+        }
+        const bool each = on && !mix;
+#else
+        const bool each = on;
 #endif
-        if (on) {
+        if (__any_sync(GRP_FULL, each)) {   // species by species, over the lanes, into the scratch
             int e = 0;
-            species_f_cv(tab.TH, YR, 1, T, lnT, rT, rT2, f, cv, e);
-            if (e) err = e;
+            if (each)
+                for (int i = gl; i < GDTK_NSP; i += L) {
+                    double tf, tc;
+                    species_terms(tab.TH, i, YR[i], T, lnT, rT, rT2, tf, tc, e);
+                    M[i] = tf;
+                    M[GDTK_NSP + i] = tc;
+                }
+            __syncwarp(GRP_FULL);
+            const double sf = grp_sum<L>(gl, [&](int i) { return M[i]; });
+            const double sc = grp_sum<L>(gl, [&](int i) { return M[GDTK_NSP + i]; });
+#pragma unroll
+            for (int x = 1; x < L; x <<= 1) e |= __shfl_xor_sync(GRP_FULL, e, x);
+            if (each) {
+                f = sf;
+                cv = sc;
+                if (e) err = e;
+            }
+#if GDTK_MIX_THERMO
+            if (each) seg_a = seg_b = -1;   // the coefficients are overwritten
+#endif
         }
         if (on) { dT = -gdtk_div(f - u_tgt, cv); ++iters; }
     }
@@ -345,17 +449,29 @@ __device__ __forceinline__ double grp_T_from_u(const GrpTab& tab, const double* 
 
 // One warp's loop with L lanes per cell.  Returns true when cells are left for twice the lanes.
 template <int L>
-__device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, GrpCell& s, bool& exhausted) {
+__device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, GrpCell& s, bool& exhausted, bool first) {
     const int lane = threadIdx.x & 31, gl = lane & (L - 1), leader0 = lane & ~(L - 1);
     const unsigned gmask = (L == 32 ? GRP_FULL : ((1u << (L & 31)) - 1u)) << leader0;
     while (true) {
         if (!exhausted) {
             const unsigned need = __ballot_sync(GRP_FULL, !s.have && gl == 0);
             if (need) {
-                unsigned base = 0;
-                if (lane == 0) base = atomicAdd(a.counter, (unsigned)__popc(need));
-                base = __shfl_sync(GRP_FULL, base, 0);
-                const unsigned pos = base + __popc(need & ((1u << leader0) - 1u));
+                // The first cells are dealt over the SMs, then the warps, then a warp's groups, so that the longest
+                // lie in different SMs and warps and take a warp's lanes when its shorter ones are done; the
+                // rest come from the counter, at most one atomic per warp.
+                const unsigned warps = gridDim.x * (blockDim.x >> 5), dealt = warps * (32 / L);
+                unsigned pos, next;
+                if (first) {
+                    pos = (lane / L) * warps + (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+                    next = dealt;
+                    first = false;
+                } else {
+                    unsigned base = 0;
+                    if (lane == 0) base = atomicAdd(a.counter, (unsigned)__popc(need));
+                    base = dealt + __shfl_sync(GRP_FULL, base, 0);
+                    pos = base + __popc(need & ((1u << leader0) - 1u));
+                    next = base + __popc(need);
+                }
                 if (!s.have && pos < (unsigned)a.total) {
                     s.g = a.order ? (unsigned)a.order[pos] : pos;
                     int lo = 0, hi = a.nblocks - 1;
@@ -380,7 +496,7 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
                         s.phase = -1;
                     }
                 }
-                exhausted = base + __popc(need) >= (unsigned)a.total;
+                exhausted = next >= (unsigned)a.total;
             }
         }
         const unsigned hm = __ballot_sync(GRP_FULL, s.have);
@@ -401,7 +517,7 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
             if (s.have && s.phase == -1) {
                 const CellBlock& B = a.blocks[s.b];
                 s.T = B.T[s.ci]; s.p = B.p[s.ci]; s.dtS = s.dtS0; s.t = 0.0; s.err = 0;
-                s.lnT = log(s.T);
+                s.lnT = gdtk_log(s.T);
                 for (int i = gl; i < GDTK_NSP; i += L) {
                     const double v = B.massf[(size_t)i * B.ncell + s.ci] * s.rho * GDTK_RM[i];
                     Y0[i] = (v < MIN_MOLES) ? 0.0 : v;
@@ -495,16 +611,17 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
 #pragma unroll 1
                     for (int i = gl; i < GDTK_NSP; i += L) {
                         const double y = Y0[i], q = Q[i];
-                        const double pp = gdtk_div(LO[i], (st == 0 ? y : C[i]) + ZERO_EPS);
-                        const double q0 = st == 0 ? q : Q0[i];
-                        const double pb = st == 0 ? pp : fma(0.5, pp, P0[i]);
-                        const double v = qss_value(y, pp, s.h, q, q0, pb);
+                        double v;
                         if (st == 0) {
+                            const double pp = qss_p(LO[i], y);
+                            v = qss_predict(y, pp, s.h, q);
                             Q0[i] = q;
-                            P0[i] = 0.5 * pp;
+                            P0[i] = half_nn(pp);
                             YP0[i] = v;
-                        } else if (qss_misses(v, YP0[i])) {
-                            cv = false;
+                        } else {
+                            const double pp = qss_p(LO[i], C[i]);
+                            v = qss_value(y, pp, s.h, q, Q0[i], fma(0.5, pp, P0[i]));
+                            if (qss_misses(v, YP0[i])) cv = false;
                         }
                         C[i] = v;
                     }
@@ -559,7 +676,7 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
             }
         } else if (act) {
             ++s.n_rej;
-            s.h /= 10.0;
+            s.h = gdtk_div(s.h, 10.0);
             if (s.err) fail = s.err;
             else if (s.h < H_MIN) fail = ST_H_MIN;
             else if (++s.attempt == GDTK_MAX_ATTEMPTS) fail = ST_MAX_ATTEMPTS;
@@ -675,7 +792,7 @@ extern "C" __global__ void __launch_bounds__(GDTK_GRP_BLOCK) gdtk_chem_group(con
     tab.ETAB = (const uint64_t*)stage(a.exp_table, GDTK_EXP2_TABLE_SIZE * 8);
     tab.eff = (const double*)stage(GRP_EFF, sizeof GRP_EFF);
     tab.kc = (const GrpKc*)stage(GRP_KC, sizeof GRP_KC);
-    tab.ent = (const uint2*)stage(GRP_ENT, sizeof GRP_ENT);
+    tab.ent = (const unsigned*)stage(GRP_ENT, sizeof GRP_ENT);
     tab.task = (const int*)stage(GRP_TASK, sizeof GRP_TASK);
     tab.lane_start = (const int*)stage(GRP_LANE_START, sizeof GRP_LANE_START);
     tab.lane_task = (const int*)stage(GRP_LANE_TASK, sizeof GRP_LANE_TASK);
@@ -684,10 +801,10 @@ extern "C" __global__ void __launch_bounds__(GDTK_GRP_BLOCK) gdtk_chem_group(con
     const int cells = 32 / lanes;   // of a warp
     s.S = q + ((threadIdx.x >> 5) * cells + (threadIdx.x & 31) / lanes) * GRP_CELL;
     bool exhausted = false, left = true;
-    if (lanes == 4) { left = grp_loop<4>(a, tab, s, exhausted); if (left) grp_widen<4>(s); }
-    if (lanes <= 8 && left) { left = grp_loop<8>(a, tab, s, exhausted); if (left) grp_widen<8>(s); }
-    if (lanes <= 16 && left) { left = grp_loop<16>(a, tab, s, exhausted); if (left) grp_widen<16>(s); }
-    if (left) grp_loop<32>(a, tab, s, exhausted);
+    if (lanes == 4) { left = grp_loop<4>(a, tab, s, exhausted, true); if (left) grp_widen<4>(s); }
+    if (lanes <= 8 && left) { left = grp_loop<8>(a, tab, s, exhausted, lanes == 8); if (left) grp_widen<8>(s); }
+    if (lanes <= 16 && left) { left = grp_loop<16>(a, tab, s, exhausted, lanes == 16); if (left) grp_widen<16>(s); }
+    if (left) grp_loop<32>(a, tab, s, exhausted, lanes == 32);
 }
 
 }  // namespace gdtk_fast

@@ -193,19 +193,19 @@ __device__ __noinline__ void falloff_rates(const FallRec& R, double T, double ln
   const double kinf = fall_arrhenius(R.lnA, R.n, R.mC, R.A, R.pw, T, lnT, rT, etab);
   const double k0 = fall_arrhenius(R.lnA0, R.n0, R.mC0, R.A0, R.pw0, T, lnT, rT, etab);
   if (R.model == 4) {   // Yungster-Rabinowitz
-    const double pr = gdtk_div(k0 * Mc, kinf), lpr = log(pr);
+    const double pr = gdtk_div(k0 * Mc, kinf), lpr = gdtk_log(pr);
     const double fc = fma(R.a, gdtk_exp(R.x1 * rT, etab), (1.0 - R.a) * gdtk_exp(R.x2 * rT, etab));
     kf = gdtk_div(__dmul_rn(kinf * gdtk_div(pr, 1.0 + pr), fc), fma(lpr, lpr, 1.0));
   } else {
     kf = gdtk_div(k0 * kinf * Mc, fma(k0, Mc, kinf));
     if (R.model == 3) {   // Troe
-      const double lpr = log(fmax(gdtk_div(k0 * Mc, kinf), 1.0e-30)) * INV_LN10;
+      const double lpr = gdtk_log(fmax(gdtk_div(k0 * Mc, kinf), 1.0e-30)) * INV_LN10;
       double lfc = R.lfc;
       if (!(R.flags & 1)) {
         double fcent = (1.0 - R.a) * gdtk_exp(R.x3 * T, etab);
         if (R.flags & 2) fcent = fma(R.a, gdtk_exp(R.x1 * T, etab), fcent);
         if (R.flags & 4) fcent += gdtk_exp(R.x2 * rT, etab);
-        lfc = log(fmax(fcent, 1.0e-30)) * INV_LN10;
+        lfc = gdtk_log(fmax(fcent, 1.0e-30)) * INV_LN10;
       }
       const double numer = lpr + fma(-0.67, lfc, -0.4);
       const double frac = gdtk_div(numer, fma(-0.14, numer, fma(-1.27, lfc, 0.75)));
@@ -305,7 +305,8 @@ std::vector<double> fast_thermo_table(const GasModelHost& gm) {
 
 // The temperature range where every species takes the same curve segment and blend of
 // cea_thermo_curves.d:150-182 (so that the mixture's H/R is one polynomial there): species curves
-// with at least two segments and equal first three breaks and first blend range.
+// with at least two segments and the same break and blend between the first two, from the highest lower end to the
+// lowest upper end or blend with a third segment.
 // Unroll factors of the rate-constant loops (reaction table, species G/RT): two independent
 // iterations in flight give the FP64 pipe work while one waits on its table loads.
 int env_int(const char* name, int dflt) {
@@ -358,9 +359,7 @@ bool mix_thermo_range(const GasModelHost& gm, double& tlo, double& thi) {
     thi = 1e300;
     for (int i = 0; i < nsp; ++i) {
         const CeaCurveHost& c = gm.curves[i];
-        if (c.nseg < 2 || c0.nseg < 2 || c.breaks[0] != c0.breaks[0] || c.breaks[1] != c0.breaks[1] ||
-            c.breaks[2] != c0.breaks[2] || c.blends[0] != c0.blends[0])
-            return false;
+        if (c.nseg < 2 || c0.nseg < 2 || c.breaks[1] != c0.breaks[1] || c.blends[0] != c0.blends[0]) return false;
         tlo = std::max(tlo, v.sp(i)[SP_TLOW]);
         thi = std::min(thi, v.sp(i)[SP_THIGH]);
         if (c.nseg > 2) thi = std::min(thi, c.breaks[2] - 0.5 * c.blends[1]);
@@ -544,19 +543,35 @@ std::string group_tables(const GasModelHost& gm, const MechanismHost& mh, const 
             task[2 * pp.isp].push_back({pp.nu > 0 ? ir : nr + ir, std::abs(pp.nu)});
             task[2 * pp.isp + 1].push_back({pp.nu > 0 ? nr + ir : ir, std::abs(pp.nu)});
         }
+    // RKF: index | coefficient << 16; alpha-QSS: index | log2 of the coefficient << 16, a coefficient that is no power
+    // of two in several entries
+    std::vector<std::vector<unsigned>> entries(2 * nsp);
     size_t n_ent = 0;
-    for (auto& t : task) n_ent += t.size();
-    o << "__device__ const __align__(16) uint2 GRP_ENT[" << std::max<size_t>(n_ent, 1) << "] = {";
-    for (auto& t : task)
-        for (auto& e : t) o << "{" << e.first << "u, " << high((double)e.second) << "u}, ";
-    if (!n_ent) o << "{0u, 0u}";
+    for (int t = 0; t < 2 * nsp; ++t) {
+        for (auto& e : task[t]) {
+            if (mh.method == METHOD_RKF) entries[t].push_back((unsigned)e.first | (unsigned)e.second << 16);
+            else
+                for (int k = 0; k < 3; ++k)
+                    if (e.second >> k & 1) entries[t].push_back((unsigned)e.first | (unsigned)k << 16);
+        }
+        n_ent += entries[t].size();
+    }
+    const size_t ent_size = (std::max<size_t>(n_ent, 1) + 1) & ~(size_t)1;
+    o << "__device__ const __align__(16) unsigned GRP_ENT[" << ent_size << "] = {0u";
+    {
+        std::ostringstream es;
+        for (auto& t : entries)
+            for (unsigned e : t) es << (es.tellp() > 0 ? ", " : "") << e << "u";
+        if (n_ent) { o.seekp(-2, std::ios_base::end); o << es.str(); }
+    }
     o << "};\n__device__ const __align__(16) int GRP_TASK[" << ((2 * nsp + 1 + 1) & ~1) << "] = {0";
     size_t at = 0;
-    for (auto& t : task) o << ", " << (at += t.size());
+    for (auto& t : entries) o << ", " << (at += t.size());
     o << "};\n";
     std::vector<int> by_length(2 * nsp);
     for (int t = 0; t < 2 * nsp; ++t) by_length[t] = t;
-    std::stable_sort(by_length.begin(), by_length.end(), [&](int a, int b) { return task[a].size() > task[b].size(); });
+    std::stable_sort(by_length.begin(), by_length.end(),
+                     [&](int a, int b) { return entries[a].size() > entries[b].size(); });
     std::ostringstream starts, tasks;
     for (int lanes : {4, 8, 16, 32}) {
         std::vector<std::vector<int>> of(lanes);
@@ -564,7 +579,7 @@ std::string group_tables(const GasModelHost& gm, const MechanismHost& mh, const 
         for (int t : by_length) {
             const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
             of[l].push_back(t);
-            load[l] += task[t].size() + 1;
+            load[l] += entries[t].size() + (mh.method == METHOD_RKF ? 1 : 2);
         }
         int n = 0;
         for (int l = 0; l < 33; ++l) {
@@ -579,7 +594,7 @@ std::string group_tables(const GasModelHost& gm, const MechanismHost& mh, const 
     o << "__device__ const __align__(16) int GRP_LANE_TASK[" << 8 * nsp << "] = {" << tasks.str() << "};\n";
     // the staged tables (GRP_TABLES of chem_group.cuh, checked there)
     shape.table_doubles = 2 * nr + nsp * 120 + GDTK_EXP2_TABLE_SIZE + std::max(nsets, 1) * nsp +
-                          16 * (int)std::max<size_t>(kc.size(), 1) + (int)std::max<size_t>(n_ent, 1) + (2 * nsp + 2) / 2 + 66 +
+                          16 * (int)std::max<size_t>(kc.size(), 1) + (int)ent_size / 2 + (2 * nsp + 2) / 2 + 66 +
                           4 * nsp;
     o << "#define GDTK_GRP_CELL " << shape.cell_doubles << "\n#define GDTK_GRP_TABLES " << shape.table_doubles << "\n";
     return o.str();
@@ -615,6 +630,9 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         const char* pc = std::getenv("GDTK_PHASE_CLOCKS");
         o << "#define GDTK_PHASE_CLOCKS " << ((pc && pc[0] == '1') ? 1 : 0) << "\n";
     }
+    // one copy of exp and the division: fetching an inlined copy at each of some 30 places costs more than the calls
+    // (262,147 H2-air cells 412 -> 393 ms, 9,001 methane cells 429 -> 384 ms), and half the compile time
+    o << "#define GDTK_FN static __device__ __noinline__\n";
     o << kFastExpSource << "\n";
     auto arr = [&](const char* name, std::function<double(int)> f) {
         o << "__constant__ double " << name << "[" << nsp << "] = {";
@@ -624,7 +642,7 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
     arr("GDTK_M", [&](int i) { return gm.M[i]; });
     arr("GDTK_RM", [&](int i) { return 1.0 / gm.M[i]; });
     arr("GDTK_R", [&](int i) { return R_universal / gm.M[i]; });
-    o << "namespace gdtk_fast {\nusing gdtk::gdtk_exp;\nusing gdtk::gdtk_div;\nusing gdtk::gdtk_rcp;\n";
+    o << "namespace gdtk_fast {\nusing gdtk::gdtk_exp;\nusing gdtk::gdtk_div;\nusing gdtk::gdtk_log;\nusing gdtk::gdtk_rcp;\n";
 
     // ---- third-body concentrations of the pressure-dependent rate constants (rate_constant.d:114-121),
     // from the concentrations at which the rate constants are evaluated
@@ -1070,14 +1088,22 @@ cudaError_t launch_fast(FastKernel& k, FastArgs& a, int sm_count, cudaStream_t s
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }
 
+// More lanes shorten a cell's step but spend more FP64 instructions on it (a cell's own scalars and sums are computed
+// by every lane), so the most lanes are taken while the cells, in turns of the resident ones, do not
+// exceed `turns`: measured where two choices cross.  H2-air (13 species; ms with 4 / 8 / 16 / 32 lanes): 1,000 cells
+// 36 / 31 / 29 / 29, 12,000 63 / 52 / 48 / 54, 48,000 108 / 96 / 109 / 179, 262,147 364 / 437 / 575 / 975.  The
+// Runge-Kutta mechanisms are smaller (5 species) and their cells' step counts alike, so that no long tail
+// pays for lanes: 1,000 air cells 2.8 / 2.4 / 2.3 / 2.3, 4,000 2.7 / 2.3 / 2.9 / 3.5, 12,000 3.3 / 3.7 / 5.6 / 9.7;
+// one thread per cell takes 3.9 there and 4.9 at 30,000, where 4 lanes take 6.3.
 int group_lanes(const FastKernel& k, long long total, int sm_count) {
     if (!k.group_function) return 0;
-    const long long budget = (long long)sm_count * (k.method == METHOD_RKF ? 216 : 1725);
-    for (int lanes = 32; lanes >= 4; lanes /= 2) {
-        const int lv = lanes == 4 ? 0 : lanes == 8 ? 1 : lanes == 16 ? 2 : 3;
-        if (k.group_warps[lv] >= 1 && total * lanes <= budget) return lanes;
+    const bool rkf = k.method == METHOD_RKF;
+    const double turns[4] = {rkf ? 0.78 : 1e30, rkf ? 0.65 : 7.0, rkf ? 0.44 : 6.5, rkf ? 0.3 : 1.6};
+    for (int lv = 3; lv >= 0; --lv) {
+        const double resident = (double)sm_count * k.group_warps[lv] * (8 >> lv);
+        if ((double)total <= turns[lv] * resident) return 4 << lv;
     }
-    return k.method == METHOD_RKF || k.group_warps[0] < 1 ? 0 : 4;
+    return 0;
 }
 
 cudaError_t launch_group(FastKernel& k, FastArgs& a, int lanes, int sm_count, cudaStream_t stream, int* grid_out,

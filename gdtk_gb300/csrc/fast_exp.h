@@ -33,6 +33,10 @@ typedef unsigned int uint32_t;
 #endif
 #endif
 
+#ifndef GDTK_FN
+#define GDTK_FN GDTK_HD
+#endif
+
 namespace gdtk {
 
 // 2^(j/256) 2^63, j = 0..255, rounded to nearest: the significands with their leading bit.
@@ -148,7 +152,7 @@ GDTK_HD uint64_t gdtk_mulhi64(uint64_t a, uint64_t b) {
     return gdtk_mul32(ah, bh) + gdtk_mulhi32(ah, bl) + gdtk_mulhi32(al, bh);
 }
 
-GDTK_HD double gdtk_exp(double x, const uint64_t* tab) {
+GDTK_FN double gdtk_exp(double x, const uint64_t* tab) {
     const uint64_t b = (uint64_t)gdtk_bits(x);
     const uint32_t hi = (uint32_t)(b >> 32), e = (hi >> 20) & 0x7ff;
     if (e >= 1033u) {   // |x| >= 1024, infinite or NaN
@@ -218,7 +222,7 @@ __device__ __forceinline__ uint64_t gdtk_rcp64(uint64_t B) {
 // An FP64 instruction holds an SM's FP64 pipe for 19 cycles (76 for each of the four sub-partitions'
 // warps), so the reciprocal seed and 4 FP64 operations of a Newton-Raphson division took about 330
 // cycles; this takes about 100 of the integer pipe's, which runs beside it.
-GDTK_HD double gdtk_div(double a, double b) {
+GDTK_FN double gdtk_div(double a, double b) {
 #ifdef __CUDA_ARCH__
     const uint64_t ua = (uint64_t)__double_as_longlong(a), ub = (uint64_t)__double_as_longlong(b);
     const uint32_t ha = (uint32_t)(ua >> 32), hb = (uint32_t)(ub >> 32);
@@ -253,5 +257,116 @@ GDTK_HD double gdtk_rcp(double b) {
     return 1.0 / b;
 #endif
 }
+
+#ifdef __CUDACC__
+// ln x on the integer pipe, after the same kind of table method (P. T. P. Tang, "Table-driven implementation of the
+// logarithm function in IEEE floating-point arithmetic", ACM TOMS 16(4):378-400, 1990): x = 2^k z with z in
+// [1/sqrt 2, sqrt 2), r = z inv_j - 1 with |r| < 2^-8.9 from a 32-bit reciprocal inv_j of z's interval,
+//   ln x = k ln 2 - ln inv_j + r - r^2 (1/2 - r (1/3 - r (1/4 - r (1/5 - r/6)))),
+// in 64-bit fixed point: 2^-62 for |k| <= 1, 2^-53 beyond, rounded once.  Within 1.2 ulp (99% correctly
+// rounded; 0.13 ulp beyond the half for temperatures).  Within 1/16 of 1, where fixed point would lose
+// relative accuracy, and for operands that are not positive normal numbers, the library's log runs.
+// About 150 cycles of the integer pipe where the library's log takes 2,200 (its FP64 operations).
+struct GdtkLogEntry { uint32_t inv, pad; int64_t L; };   // inv_j 2^31, -ln(inv_j) 2^62
+static __device__ const __align__(16) GdtkLogEntry kGdtkLogTable[256] = {
+    {0x7fc01ff0u, 0u, 8998414665322726ll}, {0x7f411e53u, 0u, 26942739767671375ll}, {0x7ec31843u, 0u, 44817515941805768ll}, {0x7e460adau, 0u, 62623274883990110ll},
+    {0x7dc9f339u, 0u, 80360551694122604ll}, {0x7d4ece90u, 0u, 98029867128141961ll}, {0x7cd49a16u, 0u, 115631744678121797ll}, {0x7c5b5311u, 0u, 133166692686875710ll},
+    {0x7be2f6ceu, 0u, 150635221558767311ll}, {0x7b6b82a7u, 0u, 168037830191025763ll}, {0x7af4f3feu, 0u, 185375016692622223ll}, {0x7a7f4841u, 0u, 202647269157614344ll},
+    {0x7a0a7ce7u, 0u, 219855072001972700ll}, {0x79968f70u, 0u, 236998905667667615ll}, {0x79237d66u, 0u, 254079244056126874ll}, {0x78b1445cu, 0u, 271096556464898743ll},
+    {0x783fe1f0u, 0u, 288051302715514983ll}, {0x77cf53c6u, 0u, 304943944239267715ll}, {0x775f978cu, 0u, 321774934689206548ll}, {0x76f0aafau, 0u, 338544719593703353ll},
+    {0x76828bceu, 0u, 355253745286495101ll}, {0x761537d0u, 0u, 371902449414049796ll}, {0x75a8acd0u, 0u, 388491265257703956ll}, {0x753ce8a5u, 0u, 405020623810608869ll},
+    {0x74d1e92fu, 0u, 421490948844782801ll}, {0x7467ac55u, 0u, 437902661321886349ll}, {0x73fe3007u, 0u, 454256174424373105ll}, {0x7395723bu, 0u, 470551900375692550ll},
+    {0x732d70eeu, 0u, 486790247864139666ll}, {0x72c62a25u, 0u, 502971619415284002ll}, {0x725f9becu, 0u, 519096413519673428ll}, {0x71f9c457u, 0u, 535165021986376158ll},
+    {0x7194a17fu, 0u, 551177836925622749ll}, {0x71303185u, 0u, 567135243310430132ll}, {0x70cc7290u, 0u, 583037623570703728ll}, {0x706962cdu, 0u, 598885357396484511ll},
+    {0x70070070u, 0u, 614678819086588057ll}, {0x6fa549b4u, 0u, 630418377308047487ll}, {0x6f443cd9u, 0u, 646104399795544406ll}, {0x6ee3d826u, 0u, 661737248235284705ll},
+    {0x6e8419e7u, 0u, 677317282996234308ll}, {0x6e25006eu, 0u, 692844860474337203ll}, {0x6dc68a14u, 0u, 708320330385570556ll}, {0x6d68b535u, 0u, 723744045569794039ll},
+    {0x6d0b8037u, 0u, 739116344266583717ll}, {0x6caee980u, 0u, 754437575033772291ll}, {0x6c52ef7fu, 0u, 769708073955014501ll}, {0x6bf790a9u, 0u, 784928171944926363ll},
+    {0x6b9ccb74u, 0u, 800098207313144792ll}, {0x6b429e60u, 0u, 815218502701246718ll}, {0x6ae907efu, 0u, 830289385274817177ll}, {0x6a9006a9u, 0u, 845311176363512741ll},
+    {0x6a37991au, 0u, 860284196426430952ll}, {0x69dfbdd4u, 0u, 875208759732378773ll}, {0x6988736du, 0u, 890085179357474207ll}, {0x6931b880u, 0u, 904913764443615003ll},
+    {0x68db8bacu, 0u, 919694822648866029ll}, {0x6885eb96u, 0u, 934428654758074857ll}, {0x6830d6e5u, 0u, 949115565021521522ll}, {0x67dc4c46u, 0u, 963755850521454019ll},
+    {0x67884a6au, 0u, 978349806266680797ll}, {0x6734d006u, 0u, 992897725060488525ll}, {0x66e1dbd5u, 0u, 1007399892024455381ll}, {0x668f6c92u, 0u, 1021856600462332500ll},
+    {0x663d8100u, 0u, 1036268130385690913ll}, {0x65ec17e3u, 0u, 1050634767090447204ll}, {0x659b3006u, 0u, 1064956784915951354ll}, {0x654ac836u, 0u, 1079234460552435617ll},
+    {0x64fadf43u, 0u, 1093468070267000678ll}, {0x64ab7402u, 0u, 1107657884348286326ll}, {0x645c854bu, 0u, 1121804172405517996ll}, {0x640e11fbu, 0u, 1135907197778666113ll},
+    {0x63c018f0u, 0u, 1149967228381423150ll}, {0x6372990eu, 0u, 1163984522868633405ll}, {0x6325913cu, 0u, 1177959338731095526ll}, {0x62d90063u, 0u, 1191891934979272455ll},
+    {0x628ce570u, 0u, 1205782566509264075ll}, {0x62413f54u, 0u, 1219631483962893425ll}, {0x61f60d03u, 0u, 1233438936393365249ll}, {0x61ab4d73u, 0u, 1247205173980846614ll},
+    {0x6160ff9fu, 0u, 1260930439506910557ll}, {0x61172283u, 0u, 1274614979495676078ll}, {0x60cdb521u, 0u, 1288259029999992381ll}, {0x6084b67bu, 0u, 1301862833462840222ll},
+    {0x603c2597u, 0u, 1315426627317138432ll}, {0x5ff40180u, 0u, 1328950640977984829ll}, {0x5fac4940u, 0u, 1342435112895891728ll}, {0x5f64fbe7u, 0u, 1355880270452327193ll},
+    {0x5f1e1886u, 0u, 1369286344181091286ll}, {0x5ed79e32u, 0u, 1382653559054895200ll}, {0x5e918c01u, 0u, 1395982143060524553ll}, {0x5e4be10fu, 0u, 1409272312604336304ll},
+    {0x5e069c77u, 0u, 1422524292746930707ll}, {0x5dc1bd58u, 0u, 1435738302608003052ll}, {0x5d7d42d5u, 0u, 1448914555220258396ll}, {0x5d392c10u, 0u, 1462053272125995914ll},
+    {0x5cf57831u, 0u, 1475154662741235988ll}, {0x5cb22662u, 0u, 1488218935986329459ll}, {0x5c6f35cdu, 0u, 1501246306170076965ll}, {0x5c2ca5a0u, 0u, 1514236981081322215ll},
+    {0x5bea750du, 0u, 1527191161841090063ll}, {0x5ba8a344u, 0u, 1540109060748009884ll}, {0x5b672f7du, 0u, 1552990871308399167ll}, {0x5b2618ecu, 0u, 1565836804108261702ll},
+    {0x5ae55ecdu, 0u, 1578647050710764020ll}, {0x5aa5005bu, 0u, 1591421810631588989ll}, {0xb4c9f9a5u, 0u, -1592415877503655658ll}, {0xb44aa6e9u, 0u, -1579711499949419975ll},
+    {0xb3cc0706u, 0u, -1567042025113367036ll}, {0xb34e1884u, 0u, -1554407261444135171ll}, {0xb2d0d9efu, 0u, -1541807018798566496ll}, {0xb25449d7u, 0u, -1529241108508507520ll},
+    {0xb1d866d1u, 0u, -1516709344993442917ll}, {0xb15d2f75u, 0u, -1504211542749137499ll}, {0xb0e2a260u, 0u, -1491747519502129740ll}, {0xb068be31u, 0u, -1479317091623858286ll},
+    {0xafef818cu, 0u, -1466920078843777911ll}, {0xaf76eb18u, 0u, -1454556301205324177ll}, {0xaefef982u, 0u, -1442225583825591229ll}, {0xae87ab76u, 0u, -1429927745981102704ll},
+    {0xae10ffa9u, 0u, -1417662616863268482ll}, {0xad9af4d0u, 0u, -1405430021502054851ll}, {0xad2589a3u, 0u, -1393229785513888461ll}, {0xacb0bce1u, 0u, -1381061741516990409ll},
+    {0xac3c8d4au, 0u, -1368925719688238155ll}, {0xabc8f9a0u, 0u, -1356821549370109534ll}, {0xab5600abu, 0u, -1344749065515941710ll}, {0xaae3a136u, 0u, -1332708103976426703ll},
+    {0xaa71da0du, 0u, -1320698498323498847ll}, {0xaa00aa01u, 0u, -1308720086325492472ll}, {0xa9900fe6u, 0u, -1296772706796545879ll}, {0xa9200a92u, 0u, -1284856198021137741ll},
+    {0xa8b098e0u, 0u, -1272970402671574721ll}, {0xa841b9adu, 0u, -1261115162999054144ll}, {0xa7d36bd7u, 0u, -1249290319225144085ll}, {0xa765ae43u, 0u, -1237495719402748713ll},
+    {0xa6f87fd6u, 0u, -1225731208026790920ll}, {0xa68bdf79u, 0u, -1213996632623935117ll}, {0xa61fcc16u, 0u, -1202291838860556536ll}, {0xa5b4449du, 0u, -1190616678846142292ll},
+    {0xa54947fdu, 0u, -1178970999606172190ll}, {0xa4ded52cu, 0u, -1167354656387523200ll}, {0xa474eb1fu, 0u, -1155767499422462819ll}, {0xa40b88d0u, 0u, -1144209383950200553ll},
+    {0xa3a2ad39u, 0u, -1132680161911568359ll}, {0xa33a575au, 0u, -1121179692042153787ll}, {0xa2d28634u, 0u, -1109707831546283239ll}, {0xa26b38c8u, 0u, -1098264434414916872ll},
+    {0xa2046e1fu, 0u, -1086849364987873504ll}, {0xa19e253fu, 0u, -1075462479402497102ll}, {0xa1385d35u, 0u, -1064103642570303542ll}, {0xa0d3150cu, 0u, -1052772712931013228ll},
+    {0xa06e4bd4u, 0u, -1041469554394186731ll}, {0xa00a00a0u, 0u, -1030194032999036460ll}, {0x9fa63284u, 0u, -1018946013524027557ll}, {0x9f42e095u, 0u, -1007725359498178428ll},
+    {0x9ee009eeu, 0u, -996531941863230650ll}, {0x9e7dada9u, 0u, -985365626949627204ll}, {0x9e1bcae3u, 0u, -974226283400373018ll}, {0x9dba60bbu, 0u, -963113780482004585ll},
+    {0x9d596e54u, 0u, -952027991611287314ll}, {0x9cf8f2d1u, 0u, -940968787425622140ll}, {0x9c98ed58u, 0u, -929936041040109964ll}, {0x9c395d10u, 0u, -918929624582666935ll},
+    {0x9bda4124u, 0u, -907949414497436759ll}, {0x9b7b98c0u, 0u, -896995286316408663ll}, {0x9b1d6311u, 0u, -886067114671919769ll}, {0x9abf9f48u, 0u, -875164778638120800ll},
+    {0x9a624c97u, 0u, -864288156465145665ll}, {0x9a056a31u, 0u, -853437125591909928ll}, {0x99a8f74cu, 0u, -842611566236746512ll}, {0x994cf320u, 0u, -831811359659272758ll},
+    {0x98f15ce7u, 0u, -821036388194444172ll}, {0x989633dbu, 0u, -810286531683792990ll}, {0x983b773bu, 0u, -799561676495960865ll}, {0x97e12644u, 0u, -788861702955043965ll},
+    {0x97874039u, 0u, -778186499803412671ll}, {0x972dc45bu, 0u, -767535949774252256ll}, {0x96d4b1efu, 0u, -756909940476813953ll}, {0x967c083bu, 0u, -746308358993170991ll},
+    {0x9623c686u, 0u, -735731091892001635ll}, {0x95cbec1bu, 0u, -725178030747478488ll}, {0x95747844u, 0u, -714649063020117939ll}, {0x951d6a4du, 0u, -704144077559053380ll},
+    {0x94c6c187u, 0u, -693662970179884809ll}, {0x94707d3fu, 0u, -683205627096681164ll}, {0x941a9cc8u, 0u, -672771943391177914ll}, {0x93c51f75u, 0u, -662361811970927450ll},
+    {0x9370049cu, 0u, -651975129155842424ll}, {0x931b4b91u, 0u, -641611785391810809ll}, {0x92c6f3acu, 0u, -631271676438878673ll}, {0x9272fc48u, 0u, -620954701571842368ll},
+    {0x921f64bfu, 0u, -610660756112309651ll}, {0x91cc2c6cu, 0u, -600389735172205242ll}, {0x917952aeu, 0u, -590141539337210897ll}, {0x9126d6e5u, 0u, -579916069063401419ll},
+    {0x90d4b86fu, 0u, -569713218998450277ll}, {0x9082f6b0u, 0u, -559532893150689480ll}, {0x9031910au, 0u, -549374989758582671ll}, {0x8fe086e2u, 0u, -539239410795507244ll},
+    {0x8f8fd7a0u, 0u, -529126062026930318ll}, {0x8f3f82a8u, 0u, -519034839635388937ll}, {0x8eef8766u, 0u, -508965653208050757ll}, {0x8e9fe542u, 0u, -498918402771541270ll},
+    {0x8e509ba8u, 0u, -488892994154381331ll}, {0x8e01aa05u, 0u, -478889333258426590ll}, {0x8db30fc6u, 0u, -468907324134599449ll}, {0x8d64cc5cu, 0u, -458946876753812749ll},
+    {0x8d16df35u, 0u, -449007893447817753ll}, {0x8cc947c5u, 0u, -439090286413124090ll}, {0x8c7c057du, 0u, -429193960221897251ll}, {0x8c2f17d2u, 0u, -419318825479812684ll},
+    {0x8be27e39u, 0u, -409464791044779386ll}, {0x8b963829u, 0u, -399631767960408269ll}, {0x8b4a451au, 0u, -389819667519605085ll}, {0x8afea483u, 0u, -380028397325435527ll},
+    {0x8ab355e0u, 0u, -370257873156179479ll}, {0x8a6858abu, 0u, -360508005163392945ll}, {0x8a1dac60u, 0u, -350778705786029316ll}, {0x89d3507du, 0u, -341069889787707457ll},
+    {0x89894480u, 0u, -331381470296857181ll}, {0x893f87e8u, 0u, -321713360804922057ll}, {0x88f61a37u, 0u, -312065479196750375ll}, {0x88acfaeeu, 0u, -302437739764352437ll},
+    {0x8864298fu, 0u, -292830057212219676ll}, {0x881ba59eu, 0u, -283242348693464148ll}, {0x87d36ea0u, 0u, -273674531823666025ll}, {0x878b841au, 0u, -264126522669600233ll},
+    {0x8743e595u, 0u, -254598243873543112ll}, {0x86fc9296u, 0u, -245089608442271133ll}, {0x86b58aa8u, 0u, -235600540064296469ll}, {0x866ecd53u, 0u, -226130954829062788ll},
+    {0x86285a23u, 0u, -216680775502370960ll}, {0x85e230a3u, 0u, -207249921340665572ll}, {0x859c5060u, 0u, -197838314237982453ll}, {0x8556b8e7u, 0u, -188445874640932310ll},
+    {0x851169c7u, 0u, -179072525676171835ll}, {0x84cc6290u, 0u, -169718191118579122ll}, {0x8487a2d1u, 0u, -160382791260219186ll}, {0x84432a1bu, 0u, -151066249120404785ll},
+    {0x83fef802u, 0u, -141768492566349147ll}, {0x83bb0c18u, 0u, -132489443939024929ll}, {0x837765f0u, 0u, -123229026280115809ll}, {0x83340520u, 0u, -113987167539447640ll},
+    {0x82f0e93du, 0u, -104763792237292842ll}, {0x82ae11deu, 0u, -95558827750151755ll}, {0x826b7e99u, 0u, -86372198026240537ll}, {0x82292f08u, 0u, -77203834120173305ll},
+    {0x81e722c2u, 0u, -68053659461191774ll}, {0x81a55963u, 0u, -58921606748578577ll}, {0x8163d283u, 0u, -49807598933376560ll}, {0x81228dbfu, 0u, -40711568288616261ll},
+    {0x80e18ab3u, 0u, -31633443714015211ll}, {0x80a0c8fbu, 0u, -22573152848700295ll}, {0x80604836u, 0u, -13530628491512705ll}, {0x80200802u, 0u, -4505800079136905ll}};
+static __device__ __noinline__ double gdtk_log(double x) {
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+    const uint32_t e = (uint32_t)(b >> 52);
+    if (e - 1u >= 2046u || b - 0x3fee000000000000ull < 0x3ff1000000000000ull - 0x3fee000000000000ull) return log(x);
+    const uint32_t j = (uint32_t)(b >> 44) & 255u;
+    const int up = j >= 106;                                              // significand above sqrt 2: z is its half
+    const int k = (int)e - 1023 + up;
+    const uint64_t z = ((b << 11) | 0x8000000000000000ull) >> up;         // 2^63
+    const uint32_t inv = kGdtkLogTable[j].inv;
+    const int64_t L = kGdtkLogTable[j].L;
+    const int64_t r = (int64_t)(gdtk_mul32((uint32_t)(z >> 32), inv) + gdtk_mulhi32((uint32_t)z, inv) - 0x4000000000000000ull);   // 2^62
+    const int r32 = (int)(r >> 23);                                       // 2^39
+    int C = 429496730 - (__mulhi(r32, 357913941) >> 7);                   // 2^31: 1/5 - r/6
+    C = 536870912 - (__mulhi(r32, C) >> 7);
+    C = 715827883 - (__mulhi(r32, C) >> 7);                               // 1/3 - r (1/4 - ...)
+    const uint64_t B = 0x2000000000000000ull - (uint64_t)(((int64_t)r32 * C) >> 8);   // 2^62: 1/2 - r C
+    const uint64_t a = (uint64_t)(r < 0 ? -r : r) << 8;                   // 2^70
+    const int64_t s = L + r - (int64_t)(gdtk_mulhi64(gdtk_mulhi64(a, a), B << 2) >> 14);
+    int64_t v;
+    uint32_t scale;
+    if (k + 1u <= 2u) {
+        v = s + (int64_t)k * 0x2c5c85fdf473de6bll;
+        scale = 62;
+    } else {
+        v = (int64_t)k * 0x162e42fefa39efll + (((int64_t)k * 219028) >> 20) + ((s + 256) >> 9);
+        scale = 53;
+    }
+    uint64_t u = (uint64_t)(v < 0 ? -v : v);
+    const int c = __clzll((long long)u);
+    u <<= c;
+    const uint64_t m = (u >> 11) + ((u >> 10) & 1);
+    return __longlong_as_double((long long)((m + ((uint64_t)(1085u - scale - (uint32_t)c) << 52)) |
+                                            (v < 0 ? 0x8000000000000000ull : 0ull)));
+}
+#endif
 
 }  // namespace gdtk
