@@ -142,6 +142,7 @@ struct ReactorObj {
     Staging stage;
     LaunchInfo last{};
     std::unique_ptr<FastKernel> fast;   // mechanism-specialised kernel, compiled on first use
+    bool no_fast = false;               // they cannot be built for this mechanism
     int req_block = 0, req_min_blocks = 0;   // launch shape chosen by chem_reactor_configure
     int refill_chunk = 0;                    // chem_reactor_set_refill_chunk
     unsigned long long* lane_stats = nullptr;   // when set, the fast kernel counts lane occupancy
@@ -247,6 +248,18 @@ const char* status_text(int st) {
     case CELL_CEA_RANGE: return "Coefficients for CEA curve could not be determined.";
     default: return "chemistry update failed";
     }
+}
+
+// Loads the mechanism-specialised kernels; false where they cannot be built (a large mechanism, shared memory).
+bool have_fast(ReactorObj& r) {
+    if (r.fast) return true;
+    if (r.large || r.no_fast) return false;
+    try {
+        r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
+    } catch (std::exception&) {
+        r.no_fast = true;
+    }
+    return !r.no_fast;
 }
 
 // Fast-kernel launch of an assembled FastArgs, longest-first unless GDTK_CHEM_INDEX_ORDER.
@@ -880,8 +893,8 @@ int thermochemical_reactor_gas_state_update(int cr_i, int gs_i, double t_interva
         double* d = r.stage.d.p;
         check(cudaMemcpyAsync(d, h.data(), nd * sizeof(double), cudaMemcpyHostToDevice, st), "cudaMemcpyAsync");
         // ThermochemicalReactor.opCall alone: no retry and no rhou update (gas_cwrap.d:906-921).
-        launch_update(r, 1, d + 0, d + 1, d + 2, d + 3, d + 5, d + 4, r.stage.st.p, t_interval, -1.0e300, 0, st, nullptr,
-                      nullptr);
+        launch_update(r, 1, d + 0, d + 1, d + 2, d + 3, d + 5, d + 4, r.stage.st.p, t_interval, -1.0e300,
+                      r.large || have_fast(r) ? 0 : GDTK_CHEM_REFERENCE_ORDER, st, nullptr, nullptr);
         int status = 0;
         check(cudaMemcpyAsync(h.data(), d, nd * sizeof(double), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
         check(cudaMemcpyAsync(&status, r.stage.st.p, sizeof(int), cudaMemcpyDeviceToHost, st), "cudaMemcpyAsync");
@@ -1055,8 +1068,17 @@ int chem_reactor_source_terms_cells(int cr_i, int ncell, const double* rho, cons
         auto& r = reactor(cr_i);
         require_cuda();
         if (ncell <= 0) return 0;
+        cudaStream_t s = (cudaStream_t)stream;
+        // the mechanism-specialised kernel (600,011 H2-air cells in 1.6 ms, where the reference-order service takes
+        // 15.1); a large mechanism has none, and a capture cannot load one
+        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+        if (!r.large && !r.fast) check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
+        if (capturing == cudaStreamCaptureStatusNone && have_fast(r)) {
+            check(launch_source(*r.fast, ncell, rho, T, massf, source, status, cuda().sm_count, s), "source terms launch");
+            return 0;
+        }
         run_service(r.dev, 2, 1, ncell, const_cast<double*>(rho), nullptr, const_cast<double*>(T), nullptr, massf,
-                    source, nullptr, status, (cudaStream_t)stream);
+                    source, nullptr, status, s);
         return 0;
     });
 }

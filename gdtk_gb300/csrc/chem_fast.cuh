@@ -949,4 +949,42 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
     }
 }
 
+// Species source terms (reaction_mechanism.d:98-105) of n cells, one thread per cell: the rate constants and the
+// right-hand side of the update.  Bound by FP64 issue (about 1,100 operations per H2-air cell).
+extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS)
+    gdtk_chem_source(const double* thermo, const uint64_t* exp_table, int n, const double* rho, const double* T,
+                     const double* massf, double* source, int* status) {
+    extern __shared__ double smem[];
+    double* TH = smem;
+    uint64_t* ETAB = reinterpret_cast<uint64_t*>(smem + GDTK_NSP * GDTK_TH_STRIDE);
+    double* S = smem + GDTK_NSP * GDTK_TH_STRIDE + GDTK_EXP2_TABLE_SIZE;
+    for (int k = threadIdx.x; k < GDTK_NSP * GDTK_TH_STRIDE; k += blockDim.x) TH[k] = thermo[k];
+    for (int k = threadIdx.x; k < GDTK_EXP2_TABLE_SIZE; k += blockDim.x) ETAB[k] = exp_table[k];
+    __syncthreads();
+    const int ks = blockDim.x;
+    double* K = S + threadIdx.x;
+    double* V = K + 2 * GDTK_NR * ks;
+    for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < n; g += gridDim.x * blockDim.x) {
+        const double r = rho[g];
+        int err = 0;
+        if (isnan(r) || r <= 0.0) {
+            err = ST_BAD;
+        } else {
+            double y[GDTK_NSP], q[GDTK_NSP], L[GDTK_NSP];
+#pragma unroll
+            for (int i = 0; i < GDTK_NSP; ++i) {
+                const double v = massf[(size_t)i * n + g] * r * GDTK_RM[i];
+                y[i] = (v < MIN_MOLES) ? 0.0 : v;
+            }
+            const double Tc = T[g];
+            if (GDTK_NFALLOFF) gen_falloff_M(y, V + GDTK_NSP * ks, ks);
+            rate_constants(TH, Tc, gdtk_log(Tc), K, ks, ETAB, V, &err);
+            gen_rhs(y, q, L, K, ks);
+#pragma unroll
+            for (int i = 0; i < GDTK_NSP; ++i) source[(size_t)i * n + g] = (q[i] - L[i]) * GDTK_M[i];
+        }
+        if (status) status[g] = err;
+    }
+}
+
 }  // namespace gdtk_fast

@@ -1038,7 +1038,12 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
     CUfunction cfn;
     cu_check(d.moduleGetFunction(&cfn, mod, "gdtk_chem_cost"), "cuModuleGetFunction");
     k->cost_function = cfn;
+    CUfunction sfn;
+    cu_check(d.moduleGetFunction(&sfn, mod, "gdtk_chem_source"), "cuModuleGetFunction");
+    k->source_function = sfn;
     const size_t smem_max = (size_t)(table + per_thread * block) * 8;
+    cu_check(d.funcSetAttribute(sfn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_max),
+             "cuFuncSetAttribute");
     cu_check(d.funcSetAttribute(fn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_max),
              "cuFuncSetAttribute");
     cu_check(d.funcSetAttribute(cfn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_max),
@@ -1124,6 +1129,21 @@ cudaError_t launch_group(FastKernel& k, FastArgs& a, int lanes, int sm_count, cu
     if (grid_out) *grid_out = (int)grid;
     if (block_out) *block_out = block;
     if (smem_out) *smem_out = (int)smem;
+    return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
+}
+
+cudaError_t launch_source(FastKernel& k, int n, const double* rho, const double* T, const double* massf, double* source,
+                          int* status, int sm_count, cudaStream_t stream) {
+    int block = k.block;
+    while (block > 32 && ((long long)n + block - 1) / block < sm_count) block -= 32;
+    const long long want = ((long long)n + block - 1) / block;
+    const long long grid = std::min<long long>(want, (long long)sm_count * k.blocks_per_sm * (k.block / block));
+    const size_t smem = (size_t)(k.table_doubles + k.per_thread_doubles * block) * 8;
+    const double* thermo = k.d_thermo;
+    const uint64_t* etab = k.d_exp;
+    void* params[] = {&thermo, &etab, &n, &rho, &T, &massf, &source, &status};
+    CUresult r = driver().launchKernel((CUfunction)k.source_function, (unsigned)grid, 1, 1, (unsigned)block, 1, 1,
+                                       (unsigned)smem, (CUstream)stream, params, nullptr);
     return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorLaunchFailure;
 }
 

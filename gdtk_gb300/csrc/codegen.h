@@ -51,6 +51,7 @@ struct FastKernel {
     void* module = nullptr;     // CUmodule
     void* function = nullptr;   // CUfunction
     void* cost_function = nullptr;   // CUfunction of the cost pre-pass
+    void* source_function = nullptr; // CUfunction of the source terms
     int block = 0;              // threads per block the kernel was compiled for
     int min_blocks = 1;
     int method = 0;
@@ -86,6 +87,9 @@ int group_lanes(const FastKernel& k, long long total, int sm_count);
 // Launches the kernel with a group of `lanes` lanes per cell.
 cudaError_t launch_group(FastKernel& k, FastArgs& a, int lanes, int sm_count, cudaStream_t stream, int* grid_out,
                          int* block_out, int* smem_out);
+// Species source terms of n cells.
+cudaError_t launch_source(FastKernel& k, int n, const double* rho, const double* T, const double* massf, double* source,
+                          int* status, int sm_count, cudaStream_t stream);
 // Longest-first visit order: cost pre-pass into key[total], then a bucket sort into order[total]
 // (hist: 257 ints of scratch).  All on `stream`.
 cudaError_t launch_order(FastKernel& k, FastArgs& a, int sm_count, float* key, int* order, int* hist,
