@@ -34,9 +34,10 @@ SOURCES = [
     ("lua_table.cpp", []),
 ]
 HEADERS = ["chem_kernels.cu", "chem_types.h", "chem_launch.h", "cea_thermo.h", "lua_table.h", "mechanism.h", "codegen.h", "fast_exp.h",
-           "chem_fast.cuh", "chem_group.cuh", "mix_thermo.cuh", "api_internal.h", "mlp_launch.h", "surrogate_launch.h", "twotemp.h"]
+           "chem_fast.cuh", "chem_group.cuh", "cea_poly.cuh", "mix_thermo.cuh", "api_internal.h", "mlp_launch.h", "surrogate_launch.h", "twotemp.h"]
 # sources compiled at run time by NVRTC, embedded in the library as string literals
-EMBEDDED = [("kFastCuhSource", "chem_fast.cuh"), ("kFastExpSource", "fast_exp.h"), ("kGroupCuhSource", "chem_group.cuh")]
+EMBEDDED = [("kFastCuhSource", "chem_fast.cuh"), ("kFastExpSource", "fast_exp.h"), ("kGroupCuhSource", "chem_group.cuh"),
+            ("kCeaPolySource", "cea_poly.cuh")]
 
 
 def _write_embedded():

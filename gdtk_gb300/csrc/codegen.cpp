@@ -39,6 +39,7 @@ namespace gdtk {
 
 extern const char* const kFastCuhSource;
 extern const char* const kFastExpSource;
+extern const char* const kCeaPolySource;
 extern const char* const kGroupCuhSource;
 
 namespace {
@@ -633,7 +634,7 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
     // one copy of exp and the division: fetching an inlined copy at each of some 30 places costs more than the calls
     // (262,147 H2-air cells 412 -> 393 ms, 9,001 methane cells 429 -> 384 ms), and half the compile time
     o << "#define GDTK_FN static __device__ __noinline__\n";
-    o << kFastExpSource << "\n";
+    o << kFastExpSource << "\n" << kCeaPolySource << "\n";
     auto arr = [&](const char* name, std::function<double(int)> f) {
         o << "__constant__ double " << name << "[" << nsp << "] = {";
         for (int i = 0; i < nsp; ++i) o << (i ? ", " : "") << lit(f(i));

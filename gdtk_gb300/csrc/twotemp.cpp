@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstring>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -14,6 +15,7 @@
 
 #include "../../include/gdtk_chem.h"
 #include "api_internal.h"
+#include "codegen.h"
 #include "cea_thermo.h"
 #include "lua_table.h"
 #include "mechanism.h"
@@ -23,6 +25,8 @@ namespace gdtk {
 namespace {
 
 constexpr double R_universal = 8.31451;   // gas/physical_constants.d:13
+constexpr double Boltzmann = 1.380658e-23;   // gas/physical_constants.d:18
+constexpr double PI_D = 3.141592653589793;
 constexpr double Avogadro = 6.02214e23;   // gas/physical_constants.d:19
 constexpr double T_REF = 298.15;          // two_temperature_gas.d:26
 
@@ -47,7 +51,7 @@ void relaxation_time(const LuaValue& t, Eem2T& e, const GasModelHost& gm, int p,
         e.rt = model == "ParkHTC" ? RT_PARK_HTC : RT_PARK_HTC2;
         e.sigma = t.get("sigma").number();
         const double mq = gm.M[q] / Avogadro, mp = gm.M[p] / Avogadro;
-        e.mu = mq * mp / (mq + mp);
+        e.cs = std::sqrt(8.0 * Boltzmann / (PI_D * (mq * mp / (mq + mp))));
         const LuaValue& sub = t.get("submodel");
         if (sub.get("model").string() != "Millikan-White")
             throw std::runtime_error("Park's high-temperature correction is supported over Millikan-White only");
@@ -75,6 +79,8 @@ std::vector<Eem2T> load_energy_exchange(const std::string& path, const GasModelH
             e.p = species_index(gm, m.get("p").string());
             e.q = species_index(gm, m.get("q").string());
             relaxation_time(m.get("relaxation_time"), e, gm, e.p, e.q);
+            e.b = e.a * e.b + 18.42;
+            e.sigma *= e.cs;
         } else if (rate == "Marrone-Treanor") {   // energy_exchange_mechanism.d:195-253
             e.kind = EEM_MARRONE_TREANOR;
             e.p = species_index(gm, m.get("p").string());
@@ -120,6 +126,11 @@ struct Reactor2TObj {
     int n_i = 0, n_d = 0;
     Species2T* d_sp = nullptr;
     Eem2T* d_eem = nullptr;
+    double *d_thermo = nullptr, *d_eff = nullptr;
+    int* d_tab = nullptr;
+    Coupling2T* d_cpl = nullptr;
+    int neff = 0, n_tab = 0, ncpl = 0;
+    unsigned relaxing = 0;
     unsigned* d_counter = nullptr;   // work counter of the update's persistent launch
     int sm_count = 0;
     ~Reactor2TObj() {
@@ -128,6 +139,8 @@ struct Reactor2TObj {
         if (d_d) cudaFree(d_d);
         if (d_sp) cudaFree(d_sp);
         if (d_eem) cudaFree(d_eem);
+        for (void* p : {(void*)d_thermo, (void*)d_eff, (void*)d_tab, (void*)d_cpl})
+            if (p) cudaFree(p);
     }
 };
 
@@ -203,7 +216,66 @@ extern "C" int chem_reactor2t_new(const char* gas_file, const char* chem_file, c
             sp[i].h_f = cea_h(v, i, T_REF, std::log(T_REF), err);
             if (err) throw std::runtime_error("CEA curve of " + r->gm.names[i] + " cannot be evaluated at 298.15 K");
         }
+        // tables of the update kernel (twotemp.h)
+        std::vector<double> eff((size_t)std::max(pm.neff, 1) * r->nsp, 0.0);
+        for (int k = 0; k < pm.neff; ++k) {
+            const int* ei = v.eff_i(k);
+            for (int j = 0; j < ei[0]; ++j) eff[(size_t)k * r->nsp + ei[1 + j]] = v.eff_d(k)[ei[1 + j]];
+        }
+        std::vector<int> tab;
+        for (int ir = 0; ir < r->nr; ++ir) {
+            const int* x = v.rx(ir);
+            unsigned sp[2] = {0, 0}, co[2] = {(unsigned)x[RX_NREAC], (unsigned)x[RX_NPROD]};
+            for (int side = 0; side < 2; ++side)
+                for (unsigned k = 0; k < co[side] % 8; ++k) {
+                    const int idx = x[(side ? RX_PROD_IDX : RX_REAC_IDX) + k], c = x[(side ? RX_PROD_COEFF : RX_REAC_COEFF) + k];
+                    if (c < 0 || c > 127) throw std::runtime_error("stoichiometric coefficient above 127");
+                    sp[side] |= (unsigned)idx << (8 * k);
+                    co[side] |= (unsigned)c << (3 + 7 * k);
+                }
+            tab.insert(tab.end(), {(int)sp[0], (int)sp[1], (int)co[0], (int)co[1], x[RX_COLLIDER] ? x[RX_EFFSET] : -1});
+        }
+        auto net = [&](int ir, int isp) {
+            const int* x = v.rx(ir);
+            for (int k = 0; k < x[RX_NPART]; ++k)
+                if (x[RX_PART + k] == isp) return x[RX_PART_NU + k];
+            return 0;
+        };
+        std::vector<int> entries;
+        for (int i = 0; i < r->nsp; ++i) {
+            tab.push_back((int)entries.size() / 2);
+            for (int ir = 0; ir < r->nr; ++ir)
+                if (const double nu = net(ir, i); nu != 0.0) {
+                    uint64_t b;
+                    std::memcpy(&b, &nu, 8);
+                    entries.insert(entries.end(), {ir, (int)(unsigned)(b >> 32)});
+                }
+        }
+        tab.push_back((int)entries.size() / 2);
+        tab.insert(tab.end(), entries.begin(), entries.end());
+        std::vector<Coupling2T> cpl;
+        for (auto& e : eem) {
+            if (e.kind == EEM_LANDAU_TELLER) {
+                r->relaxing |= 1u << e.p;
+            } else {
+                e.slot = (int)cpl.size();
+                cpl.push_back({e.reaction, 0, (double)net(e.reaction, e.p)});
+            }
+        }
+        r->neff = pm.neff;
+        r->n_tab = (int)tab.size();
+        r->ncpl = (int)cpl.size();
+        const std::vector<double> thermo = fast_thermo_table(r->gm);
         r->sm_count = device_sm_count();
+        auto upload = [](auto& d, const auto& h) {
+            if (h.empty()) return;
+            ck(cudaMalloc(&d, h.size() * sizeof h[0]), "cudaMalloc");
+            ck(cudaMemcpy(d, h.data(), h.size() * sizeof h[0], cudaMemcpyHostToDevice), "cudaMemcpy");
+        };
+        upload(r->d_thermo, thermo);
+        upload(r->d_eff, eff);
+        upload(r->d_tab, tab);
+        upload(r->d_cpl, cpl);
         r->n_i = (int)pm.I.size();
         r->n_d = (int)pm.D.size();
         ck(cudaMalloc(&r->d_i, pm.I.size() * sizeof(int)), "cudaMalloc");
@@ -261,7 +333,9 @@ extern "C" int chem_reactor2t_update_cells(int h, int ncell, const double* rho, 
         a.ncell = ncell; a.rho = rho; a.T = T; a.Tve = T_ve; a.p = p; a.massf = massf; a.u = u; a.u_ve = u_ve;
         a.dt_chem = dt_chem; a.status = status; a.t_interval = t_interval; a.steps = steps;
         a.counter = r.d_counter;
-        ck(launch_two_temperature_update(a, r.sm_count, (cudaStream_t)stream), "two-temperature update launch");
+        a.thermo = r.d_thermo; a.eff = r.d_eff; a.tab = r.d_tab; a.cpl = r.d_cpl;
+        a.neff = r.neff; a.n_tab = r.n_tab; a.ncpl = r.ncpl; a.relaxing = r.relaxing;
+        ck(launch_two_temperature_update(a, r.nsp, r.nr, r.sm_count, (cudaStream_t)stream), "two-temperature update launch");
         return 0;
     });
 }

@@ -24,12 +24,20 @@ struct Eem2T {
     int rt;          // RT_* (Landau-Teller)
     int reaction;    // reaction index (Marrone-Treanor)
     int coupling;    // CPL_* (Marrone-Treanor)
-    double a, b;     // Millikan-White constants (relaxation_time.d:27-60)
-    double sigma;    // Park high-temperature cross section [m^2]
-    double mu;       // reduced mass of the p-q pair [kg]
+    int slot;        // index among the couplings (Marrone-Treanor)
+    double a, b;     // Millikan-White (relaxation_time.d:27-60): a, and a b + 18.42
+    double sigma;    // Park high-temperature cross section [m^2] times cs
+    double cs;       // sqrt(8 k / pi mu), mu the reduced mass of the p-q pair [kg]: the mean relative speed over T^(1/2)
     double D, Thetav;   // dissociation energy [J/mol] (T_D [K] for the modified form), vibrational temperature
     double U;           // Marrone-Treanor U [K] (exchange_chemistry_coupling.d:133-175)
     double aU, Ustar, nb;   // modified Marrone-Treanor (:181-227)
+};
+
+// A chemistry-vibration coupling: its reaction and the dissociating species' net coefficient there.
+struct Coupling2T {
+    int reaction;
+    int pad;
+    double nu;
 };
 
 // Per-species two-temperature constants (two_temperature_gas.d:45-80).
@@ -46,6 +54,14 @@ struct TwoTArgs {
     const Eem2T* eem;
     int neem;
     int electron;   // index of e-, or -1
+    const double* thermo;       // thermo table of cea_poly.cuh (fast_thermo_table)
+    const double* eff;          // [neff][nsp] third-body efficiencies, 0 where absent
+    const int* tab;             // per reaction: reactants, products (8 bits each), the number (3 bits) and coefficients
+                                // (7 bits each) of either, efficiency set or -1; first entry of each species; entries
+                                // (reaction, high word of the net coefficient)
+    const Coupling2T* cpl;
+    int neff, n_tab, ncpl;
+    unsigned relaxing;          // species with Landau-Teller mechanisms, as bits
     double tol;     // RKF errTol (atol = rtol)
     int max_subcycles, max_attempts;
     int ncell;
@@ -81,7 +97,7 @@ struct Thermo2TArgs {
     double* u_ve;
 };
 
-cudaError_t launch_two_temperature_update(const TwoTArgs& a, int sm_count, cudaStream_t s);
+cudaError_t launch_two_temperature_update(const TwoTArgs& a, int nsp, int nr, int sm_count, cudaStream_t s);
 cudaError_t launch_two_temperature_thermo_pT(const Thermo2TArgs& a, int sm_count, cudaStream_t s);
 
 }  // namespace gdtk
