@@ -44,8 +44,25 @@ bool tcgen05_gemm_eligible(const GemmArgs& g);
 bool tcgen05_gemm_enabled();
 int tcgen05_gemm_set(int enable);                   // -1 leaves it; returns the previous setting
 unsigned long long tcgen05_gemm_launches();         // launches so far in this process
-cudaError_t tcgen05_gemm_error(int* error);         // 1/2: a load/MMA wait gave up (read and cleared)
+cudaError_t tcgen05_gemm_error(int* error);         // not 0: a wait gave up (read and cleared)
 cudaError_t launch_gemm_bf16_tcgen05(const GemmArgs& g, cudaStream_t s);
+
+// The network's inference in one launch (mlp_tcgen05.cu): layer sizes dims[0..nlayers], multiples of 8 up to 256,
+// GELU between layers.  Input rows are Xh (BF16 [M][dims[0]]) or, with Xh null, bf16((X - xs) / xd) of raw rows X; the
+// output rows are FP32 [M][dims[nlayers]], times yd plus ys when those are set.  cudaErrorNotSupported as above.
+constexpr int FUSED_MAX_LAYERS = 17, FUSED_MAX_STAGES = 8;
+struct FusedMlp {
+    int M = 0, nlayers = 0;
+    const int* dims = nullptr;
+    const __nv_bfloat16* W[FUSED_MAX_LAYERS] = {};   // [dims[l + 1]][dims[l]]
+    const float* bias[FUSED_MAX_LAYERS] = {};
+    const __nv_bfloat16* Xh = nullptr;
+    const float *X = nullptr, *xs = nullptr, *xd = nullptr;
+    float* out = nullptr;
+    const float *ys = nullptr, *yd = nullptr;
+};
+cudaError_t launch_mlp_fused(const FusedMlp& f, cudaStream_t s);
+
 cudaError_t launch_column_sum(int M, int N, const float* x, float* partial, float* out, cudaStream_t s);
 cudaError_t launch_mse_grad(int M, int N, const float* pred, const float* y, const float* w, float* grad,
                             __nv_bfloat16* gradh, float* loss_sum, cudaStream_t s);

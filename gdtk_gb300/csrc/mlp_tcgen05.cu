@@ -1,8 +1,12 @@
-// mlp_tcgen05.cu -- the surrogate network's forward GEMM on the fifth-generation tensor cores:
+// mlp_tcgen05.cu -- the surrogate network on the fifth-generation tensor cores: a layer's forward GEMM (below), which
+// training takes because it keeps every layer's activations, and inference of the whole network in one kernel
+// (mlp_fused_kernel).
+//
+// The layer kernel:
 //   D[M][N] = A[M][K] W[N][K]^T + bias, then GELU (keeping the pre-activation) or nothing,
 // BF16 operands, FP32 accumulation in tensor memory (TMEM), K and N multiples of 16 up to 256.
 //
-// One persistent CTA of 128 threads per SM.  The CTA loads W once with TMA and keeps it in shared
+// One persistent CTA per SM.  The CTA loads W once with TMA and keeps it in shared
 // memory; for each 128-row tile of A it
 //   1. loads the tile with TMA (2-D boxes of 8 elements x rows, which land as the K-major,
 //      no-swizzle canonical layout: 8-row x 16-byte core matrices, rows 16 bytes apart, K-groups
@@ -120,6 +124,11 @@ __device__ __forceinline__ void tmem_ld16(unsigned taddr, unsigned (&r)[16]) {
 
 // Waits for this thread's TMEM loads; the empty statements after it make every later use of r depend on
 // the wait.
+__device__ __forceinline__ void tmem_ld_wait(unsigned (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[i])::"memory");
+}
 template <int Q>
 __device__ __forceinline__ void tmem_ld_wait(unsigned (&r)[Q][16]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
@@ -129,13 +138,52 @@ __device__ __forceinline__ void tmem_ld_wait(unsigned (&r)[Q][16]) {
         for (int i = 0; i < 16; ++i) asm volatile("" : "+r"(r[q][i])::"memory");
 }
 
-// GELU, tanh form, as the mma.sync kernel's epilogue: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2u)),
-// u = sqrt(2/pi) (x + 0.044715 x^3), with exp2f and __fdividef (each within 2 ulp); exp(-2u) -> inf gives
-// -0, exp(-2u) -> 0 gives x.
-__device__ __forceinline__ float gelu_tc(float x) {
-    const float m2c_log2e = -2.0f * 0.7978845608028654f * 1.4426950408889634f;
-    const float e = exp2f(m2c_log2e * (x + 0.044715f * x * x * x));
-    return __fdividef(x, 1.0f + e);
+// Two FP32 values in one 64-bit register, and the packed operations on them: one issue slot for two results.
+__device__ __forceinline__ unsigned long long pack2(float lo, float hi) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+    return r;
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    float2 r;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float ex2_ftz(float x) {
+    float r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_ftz(float x) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// GELU, tanh form, as the mma.sync kernel's epilogue, of two values: 0.5 x (1 + tanh(u)) = x / (1 + exp(-2u)),
+// u = sqrt(2/pi) (x + 0.044715 x^3), with the 2-ulp exponential and reciprocal.  exp(-2u) -> inf gives -0, exp(-2u) -> 0
+// gives x; flushing a subnormal exponential to zero or a reciprocal below 2^-126 changes neither.  The order of the
+// operations is that of x + 0.044715f * x * x * x in FP32, to the bit: a last-place change here turns BF16 roundings.
+__device__ __forceinline__ unsigned long long gelu2(unsigned long long x) {
+    const float c1 = -2.0f * 0.7978845608028654f * 1.4426950408889634f, c3 = 0.044715f;
+    const float2 d = unpack2(mul2(fma2(mul2(mul2(pack2(c3, c3), x), x), x, x), pack2(c1, c1)));
+    const float2 w = unpack2(add2(pack2(ex2_ftz(d.x), ex2_ftz(d.y)), pack2(1.f, 1.f)));
+    return mul2(x, pack2(rcp_ftz(w.x), rcp_ftz(w.y)));
 }
 
 __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
@@ -243,7 +291,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 __syncwarp();   // the TMEM loads are warp-collective
                 tmem_ld16(trow + (unsigned)(c0 + 16 * qb), r[0]);
                 if (qb + 1 < nq) tmem_ld16(trow + (unsigned)(c0 + 16 * qb + 16), r[1]);
-                tmem_ld_wait<2>(r);
+                tmem_ld_wait(r);
                 if (row >= g.M) continue;
 #pragma unroll
                 for (int q = 0; q < 2; ++q) {
@@ -252,11 +300,17 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                     const size_t o = (size_t)row * g.ldd + c;
                     float v[16];
 #pragma unroll
-                    for (int k = 0; k < 16; ++k) {
+                    for (int k = 0; k < 16; k += 2) {
                         v[k] = __uint_as_float(r[q][k]) + s_bias[c + k];
+                        v[k + 1] = __uint_as_float(r[q][k + 1]) + s_bias[c + k + 1];
                         if (g.act == ACT_GELU) {
-                            if (g.pre) g.pre[o + k] = v[k];
-                            v[k] = gelu_tc(v[k]);
+                            if (g.pre) {
+                                g.pre[o + k] = v[k];
+                                g.pre[o + k + 1] = v[k + 1];
+                            }
+                            const float2 h = unpack2(gelu2(pack2(v[k], v[k + 1])));
+                            v[k] = h.x;
+                            v[k + 1] = h.y;
                         }
                     }
                     if (g.D) {
@@ -293,6 +347,282 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                      : "memory");
 }
 
+// ------------------------------------------------------------------------------------------------------------
+// The whole inference network in one kernel: a row's activations stay in shared memory and tensor memory from the
+// first layer to the last, so that device memory sees the input and the output rows only.
+//
+// One persistent CTA per SM works on two 128-row tiles at a time.  Each of the two slots has an activation tile in
+// shared memory (BF16, the K-major no-swizzle layout), an FP32 accumulator of up to 256 TMEM columns and eight
+// epilogue warps (two per TMEM lane quarter, half of the columns each).  A slot's layer is: MMAs from its tile into
+// its accumulator; then its warps read the accumulator, add the bias, apply GELU and write the next layer's tile over
+// the one that the MMAs have finished with.  While one slot is in its epilogue the other's MMAs run.  The weights are
+// too large to stay (393 KB for three 256 x 256 layers) and come again for each slot's layer, 64 columns of K at a time,
+// through a ring of TMA stages of 128-byte rows (narrower rows load slower than the MMAs read).  Rows and columns past
+// a matrix's edge arrive as zeros, so sizes that are multiples of 8 are padded to 16.
+//
+// 262,147 rows of 16 -> 4 x 256 -> 16: 420 -> 182 us (five layer kernels, input and output passes before); 2,000 rows:
+// 27 us; 4 x 128: 105 us, 2 x 64: 47 us.  What bounds it is shared memory: a tile's 256 x 256 layer reads 64 KB of
+// activations and 128 KB of weights for the MMAs and writes 128 KB and 64 KB, about 3,100 cycles of its 4,900; its
+// exponentials and reciprocals take 3,100 more, which the other slot's MMAs hide in part.
+struct FusedArgs {
+    int M, nlayers;
+    int dims[FUSED_MAX_LAYERS + 1];          // nin_pad, width ..., nout_pad (multiples of 8)
+    int a_bytes, stage_bytes, stages;
+    unsigned tmem_cols;                      // per slot
+    const float* bias[FUSED_MAX_LAYERS];
+    const __nv_bfloat16* Xh;                 // input rows in BF16, or
+    const float *X, *xs, *xd;                // raw rows: bf16((X - xs) / xd)
+    float* out;                              // [M][nout_pad]: the output, or with ys: output * yd + ys
+    const float *ys, *yd;
+};
+struct FusedMaps {
+    CUtensorMap w[FUSED_MAX_LAYERS];
+};
+
+constexpr int FUSED_SLOT_WARPS = 8;
+constexpr int FUSED_THREADS = 32 * (2 + 2 * FUSED_SLOT_WARPS);
+constexpr int FUSED_KC = 64;                 // K columns per weight stage: one row of the 128-byte swizzle
+
+__host__ __device__ constexpr int pad16(int n) { return (n + 15) & ~15; }
+
+// K-major operand in the 128-byte swizzle: 8-row groups 1024 bytes apart
+__device__ __forceinline__ unsigned long long smem_desc_sw128(unsigned addr) {
+    return (unsigned long long)((addr & 0x3FFFFu) >> 4) | 1ull << 16 | (unsigned long long)(1024 >> 4) << 32 | 1ull << 46 |
+           2ull << 61;
+}
+
+// Eight columns from c of this thread's row, packed to BF16, into the row's 16 bytes of K-group c / 8.
+__device__ __forceinline__ void store_group(unsigned char* a, int row, int c, const unsigned long long* v) {
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 f = unpack2(v[k]);
+        h[k] = __floats2bfloat162_rn(f.x, f.y);
+    }
+    *reinterpret_cast<uint4*>(a + (c >> 3) * (TC_M * 16) + row * 16) = *reinterpret_cast<const uint4*>(h);
+}
+
+__device__ __forceinline__ void load8(const float* p, float (&v)[8]) {
+    const float4 a = __ldg(reinterpret_cast<const float4*>(p)), b = __ldg(reinterpret_cast<const float4*>(p) + 1);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+}
+
+// Eight output columns from c, times yd plus ys when those are set
+__device__ __forceinline__ void store_out(const FusedArgs& g, unsigned row, int c, int nout, const unsigned long long* v) {
+    if (c >= nout) return;
+    float f[8];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float2 x = unpack2(v[k]);
+        f[2 * k] = x.x;
+        f[2 * k + 1] = x.y;
+    }
+    if (g.ys) {
+        float ys[8], yd[8];
+        load8(g.ys + c, ys);
+        load8(g.yd + c, yd);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = f[k] * yd[k] + ys[k];
+    }
+    float4* o = reinterpret_cast<float4*>(g.out + (size_t)row * nout + c);
+    o[0] = make_float4(f[0], f[1], f[2], f[3]);
+    o[1] = make_float4(f[4], f[5], f[6], f[7]);
+}
+
+__global__ void __launch_bounds__(FUSED_THREADS, 1)
+    mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedArgs g) {
+    extern __shared__ __align__(1024) unsigned char smem[];
+    unsigned char* sW = smem;                                        // [stages][stage_bytes], on swizzle atoms
+    unsigned char* sA = sW + g.stages * g.stage_bytes;               // [2][a_bytes]
+    unsigned long long* bars = reinterpret_cast<unsigned long long*>(sA + 2 * g.a_bytes);
+    unsigned long long* w_full = bars;                               // [FUSED_MAX_STAGES]: a stage has landed
+    unsigned long long* w_empty = bars + FUSED_MAX_STAGES;           // [FUSED_MAX_STAGES]: its MMAs are done
+    unsigned long long* a_ready = bars + 2 * FUSED_MAX_STAGES;       // [2]: the slot's tile is written, its accumulator read
+    unsigned long long* acc_full = a_ready + 2;                      // [2]: the slot's layer is in its accumulator
+    unsigned long long* drained = a_ready + 4;                       // every MMA issued is done
+    unsigned* tmem_slot = reinterpret_cast<unsigned*>(a_ready + 5);
+    unsigned long long* bias_ready = a_ready + 6;                    // [2]: the slot's biases of the layer are written
+    float* s_bias = reinterpret_cast<float*>(a_ready + 8);           // [2][256], zeros past a layer's end
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+    if (threadIdx.x == 0) {
+        for (int k = 0; k < g.stages; ++k) {
+            mbar_init(&w_full[k], 1);
+            mbar_init(&w_empty[k], 1);
+        }
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(&a_ready[k], FUSED_SLOT_WARPS);
+            mbar_init(&acc_full[k], 1);
+            mbar_init(&bias_ready[k], FUSED_SLOT_WARPS);
+        }
+        mbar_init(drained, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(2 * g.tmem_cols)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    const unsigned tmem = *tmem_slot;
+    const int ntiles = (g.M - 1) / TC_M + 1;
+    int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    if (smem_u32(smem) & 1023u) {   // the swizzle is of shared addresses; the declaration asks for this alignment
+        if (threadIdx.x == 0) atomicExch(&g_tc_error, 6);
+        my_tiles = 0;
+    }
+    // tile j of this CTA is in slot j & 1; the layers of a pair of tiles alternate between the slots
+
+    if (warp == 0 && lane == 0) {   // MMAs
+        int stage = 0, failed = 0;
+        unsigned wpar = 0, issued = 0;
+        for (int j0 = 0; j0 < my_tiles && !failed; j0 += 2)
+            for (int l = 0; l < g.nlayers && !failed; ++l)
+                for (int s = 0; s < 2 && j0 + s < my_tiles && !failed; ++s) {
+                    const unsigned seq = (unsigned)(j0 >> 1) * g.nlayers + l;
+                    if (!mbar_wait(&a_ready[s], seq & 1)) { failed = 3; break; }
+                    tc_fence_after();
+                    const unsigned a = smem_u32(sA + s * g.a_bytes), acc = tmem + (unsigned)s * g.tmem_cols;
+                    const int K = pad16(g.dims[l]);
+                    // FP32 accumulator, BF16 A and B, both K-major, N >> 3, M >> 4
+                    const unsigned idesc = (1u << 4) | (1u << 7) | (1u << 10) |
+                                           ((unsigned)(pad16(g.dims[l + 1]) >> 3) << 17) | ((unsigned)(TC_M >> 4) << 24);
+                    for (int k0 = 0; k0 < K; k0 += FUSED_KC) {
+                        if (!mbar_wait(&w_full[stage], wpar)) { failed = 1; break; }
+                        tc_fence_after();
+                        const unsigned w = smem_u32(sW + stage * g.stage_bytes);
+                        for (int k = k0; k < min(K, k0 + FUSED_KC); k += 16)
+                            mma_bf16(acc, smem_desc(a + (k >> 3) * (TC_M * 16), TC_M * 16, 128),
+                                     smem_desc_sw128(w + 2 * (k - k0)), idesc, k > 0 ? 1u : 0u);
+                        mma_commit(&w_empty[stage]);
+                        issued = 1;
+                        if (++stage == g.stages) { stage = 0; wpar ^= 1; }
+                    }
+                    if (!failed) mma_commit(&acc_full[s]);
+                }
+        if (issued) {   // bounded: nothing of this CTA is in flight when it frees its memory
+            mma_commit(drained);
+            if (!mbar_wait(drained, 0) && !failed) failed = 2;
+        }
+        if (failed) atomicExch(&g_tc_error, failed);
+    } else if (warp == 1 && lane == 0) {   // weights
+        int stage = 0, failed = 0;
+        unsigned par = 1, loads = 0;   // a first wait on the phase before the first passes
+        for (int j0 = 0; j0 < my_tiles && !failed; j0 += 2)
+            for (int l = 0; l < g.nlayers && !failed; ++l)
+                for (int s = 0; s < 2 && j0 + s < my_tiles && !failed; ++s)
+                    for (int k0 = 0; k0 < pad16(g.dims[l]); k0 += FUSED_KC) {
+                        if (!mbar_wait(&w_empty[stage], par)) { failed = 5; break; }
+                        mbar_expect_tx(&w_full[stage], (unsigned)pad16(g.dims[l + 1]) * FUSED_KC * 2);
+                        tma_load_2d(sW + stage * g.stage_bytes, &maps.w[l], k0, 0, &w_full[stage]);
+                        ++loads;
+                        if (++stage == g.stages) { stage = 0; par ^= 1; }
+                    }
+        if (failed) {
+            atomicExch(&g_tc_error, failed);
+            for (unsigned q = loads > (unsigned)g.stages ? loads - g.stages : 0; q < loads; ++q)   // bounded: loads in flight
+                mbar_wait(&w_full[q % g.stages], (q / g.stages) & 1);
+        }
+    } else if (warp >= 2) {
+        const int s = (warp - 2) / FUSED_SLOT_WARPS, half = ((warp - 2) % FUSED_SLOT_WARPS) >> 2;
+        const int r = (warp & 3) * 32 + lane;   // the TMEM lanes that a warp may read are those of its number mod 4
+        const int tid = (threadIdx.x - 64) & (32 * FUSED_SLOT_WARPS - 1);
+        unsigned char* a = sA + s * g.a_bytes;
+        float* bias = s_bias + s * 256;
+        const unsigned trow = tmem + (unsigned)s * g.tmem_cols + ((unsigned)((warp & 3) * 32) << 16);
+        const int nin = g.dims[0], nout = g.dims[g.nlayers];
+        unsigned seq = 0;
+        bool ok = true;
+        for (int j = s; j < my_tiles && ok; j += 2) {
+            const unsigned row = (blockIdx.x + j * gridDim.x) * TC_M + r, M = g.M;
+            // the input tile: the two warps of a lane quarter take every other K-group
+            for (int c = 8 * half; c < pad16(nin); c += 16) {
+                uint4 h = make_uint4(0u, 0u, 0u, 0u);
+                if (row < M && c < nin) {
+                    if (g.Xh) {
+                        h = __ldg(reinterpret_cast<const uint4*>(g.Xh + (size_t)row * nin + c));
+                    } else {
+                        float x[8], m[8], d[8];
+                        load8(g.X + (size_t)row * nin + c, x);
+                        load8(g.xs + c, m);
+                        load8(g.xd + c, d);
+                        __nv_bfloat16 e[8];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) e[k] = __float2bfloat16((x[k] - m[k]) / d[k]);
+                        memcpy(&h, e, 16);
+                    }
+                }
+                *reinterpret_cast<uint4*>(a + (c >> 3) * (TC_M * 16) + r * 16) = h;
+            }
+            for (int l = 0; l < g.nlayers; ++l, ++seq) {
+                const float b0 = tid < g.dims[l + 1] ? __ldg(g.bias[l] + tid) : 0.f;   // one column's bias per thread
+                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the tile, to the MMAs
+                tc_fence_before();
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&a_ready[s]);
+                // the accumulator; and every warp of the slot is done with the layer before
+                ok = __all_sync(0xffffffffu, mbar_wait(&acc_full[s], seq & 1));
+                if (ok) {
+                    bias[tid] = b0;
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&bias_ready[s]);
+                    ok = __all_sync(0xffffffffu, mbar_wait(&bias_ready[s], seq & 1));
+                }
+                if (!ok) {
+                    if (lane == 0) atomicExch(&g_tc_error, 4);
+                    break;
+                }
+                tc_fence_after();
+                // 16-column chunks of this warp's half; the next chunk's accumulators load under this one's work
+                const int chunks = pad16(g.dims[l + 1]) / 16, c1 = 16 * ((half + 1) * chunks / 2);
+                int c = 16 * (half * chunks / 2);
+                if (c < c1) {
+                    unsigned t[2][16];
+                    __syncwarp();   // the TMEM loads are warp-collective
+                    tmem_ld16(trow + (unsigned)c, t[0]);
+                    for (; c < c1; c += 32) {
+#pragma unroll
+                        for (int q = 0; q < 2; ++q) {
+                            const int cc = c + 16 * q;
+                            if (cc >= c1) break;
+                            __syncwarp();
+                            tmem_ld_wait(t[q]);
+                            if (cc + 16 < c1) tmem_ld16(trow + (unsigned)cc + 16, t[q ^ 1]);
+                            const ulonglong2* b = reinterpret_cast<const ulonglong2*>(bias + cc);
+                            unsigned long long v[8];
+#pragma unroll
+                            for (int k = 0; k < 4; ++k) {
+                                const ulonglong2 b4 = b[k];
+                                v[2 * k] = add2(pack2(__uint_as_float(t[q][4 * k]), __uint_as_float(t[q][4 * k + 1])), b4.x);
+                                v[2 * k + 1] =
+                                    add2(pack2(__uint_as_float(t[q][4 * k + 2]), __uint_as_float(t[q][4 * k + 3])), b4.y);
+                            }
+                            if (l + 1 < g.nlayers) {
+#pragma unroll
+                                for (int k = 0; k < 8; ++k) v[k] = gelu2(v[k]);
+                                store_group(a, r, cc, v);
+                                store_group(a, r, cc + 8, v + 4);
+                            } else if (row < M) {
+                                store_out(g, row, cc, nout, v);
+                                store_out(g, row, cc + 8, nout, v + 4);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * g.tmem_cols)
+                     : "memory");
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
         void* p = nullptr;
@@ -305,16 +635,17 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     return fn;
 }
 
-// [rows][K] BF16 row-major with leading dimension ld, boxes of 8 elements x box_rows
-bool encode(CUtensorMap* map, const void* base, int K, int rows, int ld, int box_rows) {
+// [rows][K] BF16 row-major with leading dimension ld, boxes of box_k elements x box_rows
+bool encode(CUtensorMap* map, const void* base, int K, int rows, int ld, int box_rows, int box_k = 8,
+            CUtensorMapSwizzle swizzle = CU_TENSOR_MAP_SWIZZLE_NONE) {
     auto fn = encode_fn();
     if (!fn) return false;
     cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
     cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
-    cuuint32_t box[2] = {8u, (cuuint32_t)box_rows};
+    cuuint32_t box[2] = {(cuuint32_t)box_k, (cuuint32_t)box_rows};
     cuuint32_t estride[2] = {1u, 1u};
     return fn(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base), dim, stride, box, estride,
-              CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+              CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
@@ -322,6 +653,16 @@ std::atomic<int> g_enabled{-1};                // -1: from the environment on fi
 std::atomic<unsigned long long> g_launches{0};
 
 bool aligned16(const void* p) { return ((unsigned long long)p & 15u) == 0; }
+
+int sm_count() {
+    static const int sms = [] {
+        int dev = 0, n = 0;
+        cudaGetDevice(&dev);
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        return n < 1 ? 1 : n;
+    }();
+    return sms;
+}
 
 }  // namespace
 
@@ -377,18 +718,57 @@ cudaError_t launch_gemm_bf16_tcgen05(const GemmArgs& g, cudaStream_t s) {
     // inside the allocation
     size_t smem = (size_t)a.a_bytes + a.w_bytes + 64 + (size_t)g.N * 4;   // operands, barriers and state, bias
     if (smem < 64 * 1024) smem = 64 * 1024;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-        if (sms < 1) sms = 1;
-    }
+    const int sms = sm_count();
     cudaError_t e = cudaFuncSetAttribute(gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
     const int ntiles = (g.M + TC_M - 1) / TC_M;
     const int grid = ntiles < sms ? ntiles : sms;
     gemm_tc_kernel<<<grid, TC_THREADS, smem, s>>>(ma, mw, a);
+    e = cudaGetLastError();
+    if (e == cudaSuccess) g_launches.fetch_add(1);
+    return e;
+}
+
+// The network's inference in one kernel; cudaErrorNotSupported for sizes it does not take (a layer wider than one
+// accumulator's 256 columns, more layers than it has tensor maps for), which then go layer by layer.
+cudaError_t launch_mlp_fused(const FusedMlp& f, cudaStream_t s) {
+    if (!tcgen05_gemm_enabled() || f.nlayers < 1 || f.nlayers > FUSED_MAX_LAYERS || f.M < 1) return cudaErrorNotSupported;
+    if (!aligned16(f.Xh) || !aligned16(f.X) || !aligned16(f.xs) || !aligned16(f.xd) || !aligned16(f.out) ||
+        !aligned16(f.ys) || !aligned16(f.yd))
+        return cudaErrorNotSupported;
+    FusedMaps maps;
+    FusedArgs a{};
+    int kmax = 0, nmax = 0;
+    for (int l = 0; l <= f.nlayers; ++l) {
+        const int d = f.dims[l];
+        if (d < 8 || d > 256 || d % 8) return cudaErrorNotSupported;
+        a.dims[l] = d;
+        if (l < f.nlayers) kmax = d > kmax ? d : kmax;
+        if (l > 0) nmax = d > nmax ? d : nmax;
+    }
+    for (int l = 0; l < f.nlayers; ++l) {
+        const int K = f.dims[l], N = f.dims[l + 1];
+        if (!aligned16(f.W[l]) || !aligned16(f.bias[l]) ||
+            !encode(&maps.w[l], f.W[l], K, N, K, pad16(N), FUSED_KC, CU_TENSOR_MAP_SWIZZLE_128B))
+            return cudaErrorNotSupported;
+        a.bias[l] = f.bias[l];
+    }
+    for (int l = f.nlayers; l < FUSED_MAX_LAYERS; ++l) maps.w[l] = maps.w[0];
+    a.M = f.M; a.nlayers = f.nlayers;
+    a.a_bytes = TC_M * pad16(kmax) * 2;
+    a.stage_bytes = pad16(nmax) * FUSED_KC * 2;   // whole 1024-byte swizzle atoms: N is a multiple of 16
+    unsigned cols = 32;
+    while (cols < (unsigned)pad16(nmax)) cols <<= 1;
+    a.tmem_cols = cols;
+    const int bar_bytes = (2 * FUSED_MAX_STAGES + 8) * 8 + 2 * 256 * 4;   // barriers, biases
+    a.stages = (227 * 1024 - 2 * a.a_bytes - bar_bytes) / a.stage_bytes;   // 3 of 32 KB at width 256
+    if (a.stages > FUSED_MAX_STAGES) a.stages = FUSED_MAX_STAGES;
+    const int smem = a.stages * a.stage_bytes + 2 * a.a_bytes + bar_bytes;
+    a.Xh = f.Xh; a.X = f.X; a.xs = f.xs; a.xd = f.xd; a.out = f.out; a.ys = f.ys; a.yd = f.yd;
+    cudaError_t e = cudaFuncSetAttribute(mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    const int ntiles = (f.M - 1) / TC_M + 1, sms = sm_count();
+    mlp_fused_kernel<<<ntiles < sms ? ntiles : sms, FUSED_THREADS, smem, s>>>(maps, a);
     e = cudaGetLastError();
     if (e == cudaSuccess) g_launches.fetch_add(1);
     return e;

@@ -167,9 +167,27 @@ struct Mlp {
         i_a1.ensure((size_t)chunk * width);
     }
 
+    // The whole network in one launch (launch_mlp_fused); false for sizes that it does not take.
+    bool fused(FusedMlp& f, int B, float* out, cudaStream_t s) {
+        f.M = B;
+        f.nlayers = depth + 1;
+        f.dims = dims.data();
+        f.out = out;
+        for (int l = 0; l <= depth && l < FUSED_MAX_LAYERS; ++l) {
+            f.W[l] = W16(l);
+            f.bias[l] = bias(l);
+        }
+        const cudaError_t e = launch_mlp_fused(f, s);
+        if (e != cudaErrorNotSupported) ck(e, "surrogate network");
+        return e == cudaSuccess;
+    }
+
     // forward over B rows of bf16 inputs xh; training (into t_out) keeps every layer's
     // pre-activation and activation.  The fp32 output goes to out.
     void forward(int B, const __nv_bfloat16* xh, bool train, float* out, cudaStream_t s) {
+        FusedMlp f;
+        f.Xh = xh;
+        if (!train && fused(f, B, out, s)) return;
         if (train) ensure_train(B);
         else ensure_infer(B);
         const __nv_bfloat16* in = xh;
@@ -317,7 +335,10 @@ struct Surrogate {
     }
 
     void predict_raw(int n, const float* X, float* out, cudaStream_t s) {
-        // out = standardised prediction * y_scale + y_shift, chunk by chunk
+        // out = standardised prediction * y_scale + y_shift
+        FusedMlp f;
+        f.X = X; f.xs = d_xs.p; f.xd = d_xd.p; f.ys = d_ys.p; f.yd = d_yd.p;
+        if (net.fused(f, n, out, s)) return;
         const int chunk = std::min(n, 1 << 20);
         ensure_infer(chunk);
         for (int first = 0; first < n; first += chunk) {
