@@ -153,8 +153,7 @@ struct ReactorObj {
     bool large = false;                 // more than GDTK_MAX_SPECIES species or GDTK_MAX_REACTIONS reactions
     int warp_doubles = 0;
     DevBuf<int> wt_i;                   // warp-per-cell tables (WarpTables, chem_launch.h)
-    DevBuf<double> wt_d;
-    WarpTables wt{};
+    WarpTables wt[WARP_VARIANTS]{};
     ~ReactorObj() { if (counter) cudaFree(counter); }
 };
 
@@ -286,128 +285,146 @@ void run_fast(ReactorObj& r, FastArgs& a, int flags, cudaStream_t s) {
     r.last.blocks_per_sm = r.fast->blocks_per_sm;
 }
 
-// Tables of the warp-per-cell kernel (layout in chem_launch.h) from the packed mechanism: reaction terms
-// and third bodies, scaled tick-rate slots for coefficients above 1, the q / L gather tasks dealt whole to
-// the 32 lanes longest first, and the efficiency lists transposed.
+// Tables of the warp-per-cell kernel (layout in chem_launch.h) from the packed mechanism.
 void prepare_warp_path(ReactorObj& r, const PackedMech& pm) {
     r.large = pm.nsp > GDTK_MAX_SPECIES || pm.nr > GDTK_MAX_REACTIONS;
     MechView m;
     m.bind(pm.I.data(), pm.D.data());
     const int nsp = pm.nsp, nr = pm.nr, neff = pm.neff;
-    std::vector<int> tstart(nr + 1, 0), tmid(nr, 0), terms, rxeff(nr, -1), slot;
-    auto term = [&](int isp, int coeff) {
-        if (isp < 0 || isp >= nsp || coeff < 0 || coeff > 0xffffff) throw std::runtime_error("reaction term out of range");
-        terms.push_back(isp | coeff << 8);
-    };
-    std::map<std::pair<int, int>, int> slot_of;   // (reaction, |nu|) -> slot
-    struct Entry { int ir, nu; };
-    std::vector<std::vector<Entry>> per(nsp);   // species -> (reaction, nu), ascending reaction
+    if (2 * nr > 0x2000) throw std::runtime_error("too many tick-rate terms for the warp-per-cell gather");
+    // the reactions' factors, and their order: equal numbers of factors side by side
+    struct Rx { int ir; std::vector<int> f, b; };
+    std::vector<Rx> rx(nr);
     for (int ir = 0; ir < nr; ++ir) {
         const int* x = m.rx(ir);
-        for (int k = 0; k < x[RX_NREAC]; ++k) term(x[RX_REAC_IDX + k], x[RX_REAC_COEFF + k]);
-        tmid[ir] = (int)terms.size();
-        for (int k = 0; k < x[RX_NPROD]; ++k) term(x[RX_PROD_IDX + k], x[RX_PROD_COEFF + k]);
-        tstart[ir + 1] = (int)terms.size();
-        if (x[RX_COLLIDER]) rxeff[ir] = x[RX_EFFSET];
-        for (int k = 0; k < x[RX_NPART]; ++k) {
-            const int nu = x[RX_PART_NU + k];
-            if (nu == 0) continue;
-            const int a = nu < 0 ? -nu : nu;
-            if (a > 255) throw std::runtime_error("stoichiometric coefficient out of range");
-            if (a > 1 && !slot_of.count({ir, a})) {
-                slot_of[{ir, a}] = (int)slot.size();
-                slot.push_back(ir | a << 16);
+        rx[ir].ir = ir;
+        auto term = [&](std::vector<int>& v, int isp, int coeff) {
+            if (isp < 0 || isp >= nsp || coeff < 0 || coeff > 0xffffff) throw std::runtime_error("reaction term out of range");
+            if (coeff) v.push_back(isp | coeff << 8);
+        };
+        for (int k = 0; k < x[RX_NREAC]; ++k) term(rx[ir].f, x[RX_REAC_IDX + k], x[RX_REAC_COEFF + k]);
+        for (int k = 0; k < x[RX_NPROD]; ++k) term(rx[ir].b, x[RX_PROD_IDX + k], x[RX_PROD_COEFF + k]);
+    }
+    auto shape = [&](const Rx& x) { return std::make_tuple(m.rx(x.ir)[RX_COLLIDER] != 0, x.f.size(), x.b.size()); };
+    std::stable_sort(rx.begin(), rx.end(), [&](const Rx& a, const Rx& b) { return shape(a) < shape(b); });
+    std::vector<int> pos(nr), perm(nr), factors, rxm(nr, 0), lstart, lterms;
+    for (int k = 0; k < nr; ++k) {
+        pos[rx[k].ir] = k;
+        perm[k] = rx[k].ir;
+        const int* x = m.rx(rx[k].ir);
+        if (x[RX_COLLIDER]) rxm[k] = x[RX_EFFSET] + 1;
+        bool big = rx[k].f.size() > 4 || rx[k].b.size() > 4;
+        for (auto* v : {&rx[k].f, &rx[k].b})
+            for (int t : *v) big = big || t > 0xffff;
+        if (big) {
+            rxm[k] |= RX_LONG | (int)(lstart.size() / 3) << 16;
+            for (auto* v : {&rx[k].f, &rx[k].b}) {
+                lstart.push_back((int)lterms.size());
+                lterms.insert(lterms.end(), v->begin(), v->end());
             }
-            per[x[RX_PART + k]].push_back({ir, nu});
+            lstart.push_back((int)lterms.size());
+        }
+        for (auto* v : {&rx[k].f, &rx[k].b})
+            for (size_t j = 0; j < 4; j += 2) {
+                const unsigned lo = !big && j < v->size() ? (*v)[j] : 0, hi = !big && j + 1 < v->size() ? (*v)[j + 1] : 0;
+                factors.push_back((int)(lo | hi << 16));
+            }
+    }
+    // species -> the entries of its q and L, ascending reaction: q gets nu w_f (nu > 0) or -nu w_b, L gets nu w_b
+    // (nu > 0) or -nu w_f (reaction_mechanism.d:82-96), a coefficient as the powers of two that make it up
+    std::vector<std::vector<unsigned short>> per(2 * nsp);
+    for (int ir = 0; ir < nr; ++ir) {
+        const int* x = m.rx(ir);
+        for (int k = 0; k < x[RX_NPART]; ++k) {
+            const int nu = x[RX_PART_NU + k], a = nu < 0 ? -nu : nu;
+            if (a > 255) throw std::runtime_error("stoichiometric coefficient out of range");
+            for (int to_L = 0; to_L < 2; ++to_L)
+                for (int s = 0; s < 8; ++s)
+                    if (a >> s & 1)
+                        per[to_L * nsp + x[RX_PART + k]].push_back(
+                            (unsigned short)(((nu > 0) == (to_L != 0) ? nr + pos[ir] : pos[ir]) | s << 13));
         }
     }
-    const int nslot = (int)slot.size();
-    // element of w_f[nr], w_b[nr], |nu| w_f[nslot], |nu| w_b[nslot] that a (reaction, nu) term adds to q or L:
-    // q gets nu w_f (nu > 0) or -nu w_b, L gets nu w_b (nu > 0) or -nu w_f (reaction_mechanism.d:82-96)
-    auto index = [&](const Entry& e, bool to_L) {
-        const int a = e.nu < 0 ? -e.nu : e.nu;
-        const bool use_b = (e.nu > 0) == to_L;
-        if (a == 1) return use_b ? nr + e.ir : e.ir;
-        const int j = slot_of[{e.ir, a}];
-        return 2 * nr + (use_b ? nslot : 0) + j;
-    };
-    if (2 * nr + 2 * nslot > 0x2000) throw std::runtime_error("too many tick-rate terms for the warp-per-cell gather");
-    // tasks: the q and the L of each species; those longer than a lane's share of all entries are split into
-    // equal parts, whose later ones go to partial sums.  Longest first onto the least-loaded lane (ties: lowest)
-    struct Part { int target, isp; bool to_L; size_t lo, hi; };
+    struct Part { int target, from; size_t lo, hi; };
     std::vector<Part> parts;
     std::vector<int> comb;
     size_t total = 0;
-    for (auto& v : per) total += 2 * v.size();
-    const size_t share = std::max<size_t>(4, (total + 31) / 32);
+    for (auto& v : per) total += v.size();
+    const size_t share = std::max<size_t>(4, (total + 127) / 128);
     int npart = 0;
     for (int t = 0; t < 2 * nsp; ++t) {
-        const size_t len = per[t >> 1].size();
-        if (!len) continue;
-        size_t n = (len + share - 1) / share;
-        if (npart + (int)n - 1 > 128) n = 1;
-        if (n > 1) comb.push_back((t >> 1) | (t & 1) << 7 | npart << 8 | (int)(n - 1) << 16);
-        for (size_t k = 0; k < n; ++k)
-            parts.push_back({k == 0 ? t >> 1 : 128 + npart++, t >> 1, (t & 1) != 0, len * k / n, len * (k + 1) / n});
+        const size_t len = per[t].size(), n = (len + share - 1) / share;
+        if (n > 1) {
+            comb.push_back(t | npart << 16);
+            comb.push_back((int)n - 1);
+        }
+        for (size_t k = 0; k < n; ++k) parts.push_back({k == 0 ? t : 2 * nsp + npart++, t, len * k / n, len * (k + 1) / n});
     }
     std::stable_sort(parts.begin(), parts.end(), [](const Part& a, const Part& b) { return a.hi - a.lo > b.hi - b.lo; });
-    std::vector<std::vector<int>> lane_parts(32);
-    std::vector<size_t> load(32, 0);
-    for (size_t k = 0; k < parts.size(); ++k) {
-        const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
-        lane_parts[l].push_back((int)k);
-        load[l] += parts[k].hi - parts[k].lo;
-    }
-    std::vector<int> lane(33, 0), ent;
-    for (int l = 0; l < 32; ++l) {
-        for (int k : lane_parts[l]) {
-            const Part& t = parts[k];
-            for (size_t j = t.lo; j < t.hi; ++j)
-                ent.push_back(t.target | index(per[t.isp][j], t.to_L) << 8 | (t.to_L ? 1 : 0) << 21);
-        }
-        lane[l + 1] = (int)ent.size();
-    }
-    int maxlen = 0;
-    for (int s = 0; s < neff; ++s) maxlen = std::max(maxlen, m.eff_i(s)[0]);
-    std::vector<int> efflen(std::max(neff, 1), 0), effidx(std::max((size_t)maxlen * neff, (size_t)1), 0);
-    std::vector<double> effval(std::max((size_t)maxlen * neff, (size_t)1), 0.0);
+    std::vector<int> eff((size_t)2 * neff * nsp, 0), M((size_t)2 * nsp);
+    auto put_double = [](std::vector<int>& v, size_t k, double x) { std::memcpy(&v[2 * k], &x, 8); };
+    for (int i = 0; i < nsp; ++i) put_double(M, i, m.sp(i)[SP_M]);
     for (int s = 0; s < neff; ++s) {
         const int* ei = m.eff_i(s);
-        const double* ev = m.eff_d(s);
-        efflen[s] = ei[0];
-        for (int k = 0; k < ei[0]; ++k) {
-            effidx[(size_t)k * neff + s] = ei[1 + k];
-            effval[(size_t)k * neff + s] = ev[ei[1 + k]];
-        }
+        for (int k = 0; k < ei[0]; ++k) put_double(eff, (size_t)s * nsp + ei[1 + k], m.eff_d(s)[ei[1 + k]]);
     }
+    const bool eff_staged = eff.size() * 4 <= 16384;   // beyond that they would take a cell's place
     std::vector<int> all;
+    size_t base = 0;   // of the variant's tables
     auto put = [&](const std::vector<int>& v) {
-        const int off = (int)all.size();
+        while (all.size() % 4) all.push_back(0);
+        const int off = (int)(all.size() - base);
         all.insert(all.end(), v.begin(), v.end());
         return off;
     };
-    WarpTables& t = r.wt;
-    t.nslot = nslot;
-    t.off_tstart = put(tstart);
-    t.off_tmid = put(tmid);
-    t.off_terms = put(terms);
-    t.off_rxeff = put(rxeff);
-    t.off_slot = put(slot);
-    t.off_lane = put(lane);
-    t.off_ent = put(ent);
-    t.off_comb = put(comb);
-    t.ncomb = (int)comb.size();
-    t.npart = npart;
-    t.n_smem_ints = (int)all.size();
-    t.off_efflen = put(efflen);
-    t.off_effidx = put(effidx);
-    r.warp_doubles = chem_warp_doubles(nsp, nr, neff, pm.method, nslot, npart);
+    size_t bases[WARP_VARIANTS];
+    for (int v = 0; v < WARP_VARIANTS; ++v) {
+        const int lanes = 32 << v;
+        std::vector<std::vector<int>> lane_parts(lanes);
+        std::vector<size_t> load(lanes, 0);
+        for (size_t k = 0; k < parts.size(); ++k) {   // longest first onto the least-loaded lane (ties: lowest)
+            const int l = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+            lane_parts[l].push_back((int)k);
+            load[l] += parts[k].hi - parts[k].lo;
+        }
+        const size_t longest = *std::max_element(load.begin(), load.end());
+        std::vector<int> lane(1, 0), task;
+        std::vector<unsigned short> e16((longest * lanes + 1) / 2 * 2, 0);
+        for (int l = 0; l < lanes; ++l) {
+            size_t at = 0;
+            for (int k : lane_parts[l]) {
+                const Part& t = parts[k];
+                task.push_back(t.target | (int)(t.hi - t.lo) << 16);
+                for (size_t j = t.lo; j < t.hi; ++j) e16[at++ * lanes + l] = per[t.from][j];
+            }
+            lane.push_back((int)task.size());
+        }
+        std::vector<int> ent(e16.size() / 2);
+        if (!ent.empty()) std::memcpy(ent.data(), e16.data(), e16.size() * 2);
+        put({});
+        base = bases[v] = all.size();
+        WarpTables& t = r.wt[v];
+        put(factors);
+        t.off_rxm = put(rxm);
+        t.off_M = put(M);
+        t.off_lane = put(lane);
+        t.off_task = put(task);
+        t.off_ent = put(ent);
+        t.off_comb = put(comb);
+        t.ncomb = (int)comb.size() / 2;
+        t.npart = npart;
+        if (eff_staged) t.off_eff = put(eff);
+        put({});
+        t.n_smem_ints = (int)(all.size() - base);
+        if (!eff_staged) t.off_eff = put(eff);
+        t.off_perm = put(perm);
+        t.off_lstart = put(lstart);
+        t.off_lterms = put(lterms);
+    }
+    r.warp_doubles = chem_warp_doubles(nsp, nr, neff, pm.method, npart);
     r.wt_i.ensure(all.size());
-    r.wt_d.ensure(effval.size());
     check(cudaMemcpy(r.wt_i.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice), "cudaMemcpy");
-    check(cudaMemcpy(r.wt_d.p, effval.data(), effval.size() * sizeof(double), cudaMemcpyHostToDevice), "cudaMemcpy");
-    t.gi = r.wt_i.p;
-    t.eff_val = r.wt_d.p;
+    for (int v = 0; v < WARP_VARIANTS; ++v) r.wt[v].gi = r.wt_i.p + bases[v];
 }
 
 int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, double* T, double* p, double* massf,
@@ -421,7 +438,7 @@ int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, 
     if (!r.counter) check(cudaMalloc(&r.counter, sizeof(unsigned)), "cudaMalloc");
     check(cudaMemsetAsync(r.counter, 0, sizeof(unsigned), s), "cudaMemsetAsync");
     if ((flags & GDTK_CHEM_WARP_PER_CELL) || r.large) {
-        if (!r.wt.gi) throw std::runtime_error("warp-per-cell tables were not uploaded");
+        if (!r.wt[0].gi) throw std::runtime_error("warp-per-cell tables were not uploaded");
         ChemUpdateArgs a{};
         a.mech_i = r.dev.I;
         a.mech_d = r.dev.D;

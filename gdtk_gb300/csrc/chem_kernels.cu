@@ -741,67 +741,103 @@ __global__ void order_scatter(const float* key, int n, int* hist, int* order) {
 
 #if GDTK_WARP_TU
 // ---------------------------------------------------------------- one warp per cell (large mechanisms)
-// The reference-order update (chem_update_kernel above) with one warp integrating one cell: species
-// and reactions are spread over the lanes, and the cell's vectors live in the warp's share of shared
-// memory.  The right-hand side reads compact tables (WarpTables): each reaction's concentration terms
-// from shared memory, the third-body efficiency lists transposed in global memory (one list per lane,
-// consecutive words across lanes), and a species -> (reaction, coefficient) gather whose species are
-// dealt to the lanes longest first, so that the lanes' loops are about equally long.  Rate constants
-// and thermo read the packed mechanism from global memory (they need not fit in shared memory).
-// Sums the reference takes over species in order (energies, gas constant, mass-fraction total,
-// RKF error norm) are taken by lane 0 in that order from per-species terms the lanes computed; q and L
-// gather each species' terms in reaction order, a long species' in parts, and third-body sums are spread
-// over lanes.  This translation unit is compiled with FMA contraction and its alpha-QSS step takes the two-division
+// The reference-order update (chem_update_kernel above) with one, two or four warps (NW) integrating one cell: species
+// and reactions are spread over the lanes, and the cell's vectors live in its share of shared memory.  The
+// right-hand side reads compact tables (WarpTables) from shared memory: the reactions sorted by shape, so that the
+// lanes of a warp take the same turns, and a species -> (reaction, coefficient) gather dealt to the lanes in parts of
+// at most a 128th of its entries.  Rate constants and thermo read the packed mechanism from global memory (they need
+// not fit in shared memory).  Sums the reference takes over species in order (energies, gas constant, the final
+// mass-fraction total, RKF error norm) are taken by lane 0 in that order from per-species terms the lanes computed.
+// This translation unit is compiled with FMA contraction and its alpha-QSS step takes the two-division
 // form (w_aqss_step), so values agree with the reference-order kernel to rounding, not bitwise.
-// Minima and maxima (step estimate, sigma) are order-free.
+// Minima and maxima (step estimate, sigma) are order-free; no sum of a result depends on NW.
+//
+// A right-hand side of the acetylene mechanism (75 species, 474 reactions) is a chain of latencies, shared memory's and
+// the FP64 pipe's: 31 us for a warp, with one cell on an SM or with the eight that shared memory holds.  Warps that
+// share a cell cut the chain and raise the warps in flight.  Four warps to a cell: 304 cells 63.1 -> 18.7 ms; two:
+// 6,007 cells 155 -> 91 ms (with the sums of q and L on the integer pipe and the reactions sorted, in both).
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 struct WarpLayout {
-    int y0, yout, q, L, mf, g, tmp, kf, kb, wf, wb, wsf, wsb, part, meff, ext, total;
-    __device__ __host__ void make(int nsp, int nr, int neff, int method, int nslot, int npart) {
-        y0 = 0; yout = nsp; q = 2 * nsp; L = 3 * nsp; mf = 4 * nsp; g = 5 * nsp; tmp = 6 * nsp;
-        kf = 8 * nsp; kb = kf + nr; wf = kb + nr; wb = wf + nr; wsf = wb + nr; wsb = wsf + nslot;
-        part = wsb + nslot;
-        meff = part + npart;
+    int y0, yout, q, L, part, mf, g, tmp, kf, kb, wf, wb, meff, ext, red, total;
+    __device__ __host__ void make(int nsp, int nr, int neff, int method, int npart) {
+        y0 = 0; yout = nsp; q = 2 * nsp; L = 3 * nsp; part = 4 * nsp; mf = part + npart; g = mf + nsp; tmp = g + nsp;
+        kf = tmp + 2 * nsp; kb = kf + nr; wf = kb + nr; wb = wf + nr;
+        meff = wb + nr;
         ext = meff + (neff > 0 ? neff : 1);
-        total = ext + (method == METHOD_RKF ? 7 * nsp : 4 * nsp);
+        red = ext + (method == METHOD_RKF ? 7 * nsp : 4 * nsp);
+        total = red + 6;
     }
 };
 
+template <int NW>
 struct WarpCtx {
+    static constexpr int NL = 32 * NW;   // lanes of a cell
     MechView m;
-    const int* tstart;      // shared: reaction ir's terms tstart[ir] .. tstart[ir + 1], products from tmid[ir]
-    const int* tmid;
-    const int* terms;       // shared: species | coeff << 8
-    const int* rxeff;       // shared: third-body efficiency list of each reaction, or -1
-    const int* slot;        // shared: reaction | |nu| << 16 of each scaled tick-rate slot
-    int nslot;
-    double* wsf;            // the warp's |nu| w_f and |nu| w_b of each slot
-    double* wsb;
-    double* part;           // the warp's partial q and L of split tasks
-    int ent_lo, ent_hi;     // this lane's gather entries
-    const int* ent;         // shared: target | index << 8 | L << 21
-    const int* comb;        // shared: species | L << 7 | first part << 8 | number of parts << 16, per split task
+    const uint4* rx;        // shared: up to four reactant and four product factors of the reaction at each position
+    const int* rxm;         // shared: its efficiency list + 1, or with RX_LONG its place in the long lists
+    const int* lstart;      // global: a long reaction's reaction terms lstart[3 j] .., products from lstart[3 j + 1], end
+    const int* lterms;      // global: species | coeff << 8
+    const int* perm;        // global: the reaction at each position
+    const unsigned short* ent;   // shared: [entry][lane], index | shift << 13
+    int task_lo, task_hi;   // this lane's gather tasks
+    const int* task;        // shared: target | number of entries << 16
+    const int* comb;        // shared: target | first part << 16, number of parts, per split task
     int ncomb;
-    const int* efflen;      // global: length of each efficiency list
-    const int* effidx;      // global, [k][neff]: species of entry k of each list
-    const double* effval;   // global, [k][neff]: its efficiency
-    int lane;
+    const double* eff;      // shared or global: [neff][nsp] efficiencies
+    const double* M;        // shared: molar masses
+    double* red;            // the cell's scratch of reductions over its warps
+    int lane, bar;
+
+    // all lanes of the cell
+    __device__ __forceinline__ void sync() const {
+        if (NW == 1) __syncwarp();
+        else asm volatile("barrier.cta.sync %0, %1;" ::"r"(bar), "n"(NL) : "memory");
+    }
+    __device__ __forceinline__ bool any(bool p) const {
+        if (NW == 1) return __any_sync(FULL_MASK, p);
+        unsigned r;
+        asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\tbarrier.cta.red.or.pred q, %2, %3, p;\n\t"
+                     "selp.u32 %0, 1, 0, q;\n\t}"
+                     : "=r"(r) : "r"((unsigned)p), "r"(bar), "n"(NL) : "memory");
+        return r != 0;
+    }
+    __device__ __forceinline__ double bcast(double v) const {   // lane 0's value
+        if (NW == 1) return __shfl_sync(FULL_MASK, v, 0);
+        if (lane == 0) red[0] = v;
+        sync();
+        const double r = red[0];
+        sync();
+        return r;
+    }
+    // f over the cell's lanes, from each lane's value
+    template <class F>
+    __device__ __forceinline__ double reduce(double v, F f) const {
+        for (int o = 16; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(FULL_MASK, v, o));
+        if (NW == 1) return v;
+        if (!(lane & 31)) red[1 + (lane >> 5)] = v;
+        sync();
+        v = red[1];
+        for (int k = 1; k < NW; ++k) v = f(v, red[1 + k]);
+        sync();
+        return v;
+    }
 };
 
-__device__ __forceinline__ double bcast(double v) { return __shfl_sync(FULL_MASK, v, 0); }
-
 // lane 0 sums v[0..n) in order; every lane gets the result
-__device__ __forceinline__ double serial_sum(const WarpCtx& w, const double* v, int n) {
+template <int NW>
+__device__ __forceinline__ double serial_sum(const WarpCtx<NW>& w, const double* v, int n) {
     double s = 0.0;
     if (w.lane == 0)
         for (int i = 0; i < n; ++i) s += v[i];
-    return bcast(s);
+    return w.bcast(s);
 }
 
-__device__ __forceinline__ int warp_or(int e) { return __any_sync(FULL_MASK, e != 0) ? (e ? e : 1) : 0; }
+template <int NW>
+__device__ __forceinline__ int warp_or(const WarpCtx<NW>& w, int e) { return w.any(e != 0) ? (e ? e : 1) : 0; }
 
-__device__ void w_rate_constants(const WarpCtx& w, double Tq, double* kf, double* kb, double* g, const double* mf,
+template <int NW>
+__device__ void w_rate_constants(const WarpCtx<NW>& w, double Tq, double* kf, double* kb, double* g, const double* mf,
                                  double rho, int& err) {
     const MechView& m = w.m;
     double T = Tq;
@@ -809,14 +845,15 @@ __device__ void w_rate_constants(const WarpCtx& w, double Tq, double* kf, double
     if (T > m.T_upper()) T = m.T_upper();
     const double logT = log(T);
     int e = 0;
-    for (int i = w.lane; i < m.nsp; i += 32) {
+    for (int i = w.lane; i < m.nsp; i += 32 * NW) {
         double h = cea_h(m, i, T, logT, e);
         double sv = cea_s(m, i, T, logT, e);
         g[i] = h - T * sv;
     }
-    __syncwarp();
+    w.sync();
     Vec mfv{const_cast<double*>(mf), 1};
-    for (int ir = w.lane; ir < m.nr; ir += 32) {
+    for (int j = w.lane; j < m.nr; j += 32 * NW) {
+        const int ir = w.perm[j];
         const int* r = m.rx(ir);
         const double* d = m.rxd(ir);
         double Kc = 1.0;
@@ -834,95 +871,122 @@ __device__ void w_rate_constants(const WarpCtx& w, double Tq, double* kf, double
         if (r[RX_FRC] != RATE_FROM_EQ) {
             double f = (r[RX_FRC] == RATE_ARRHENIUS || r[RX_FRC] == RATE_ARRHENIUS2)
                            ? simple_rate(r[RX_FRC], d, T) : pressure_dependent_kf(m, r, d, T, mfv, rho);
-            kf[ir] = f;
-            kb[ir] = (r[RX_BRC] == RATE_FROM_EQ) ? f / Kc : simple_rate(r[RX_BRC], d + 3, T);
+            kf[j] = f;
+            kb[j] = (r[RX_BRC] == RATE_FROM_EQ) ? f / Kc : simple_rate(r[RX_BRC], d + 3, T);
         } else {
             double b = simple_rate(r[RX_BRC], d + 3, T);
-            kb[ir] = b;
-            kf[ir] = b * Kc;
+            kb[j] = b;
+            kf[j] = b * Kc;
         }
     }
-    __syncwarp();
-    const int any = warp_or(e);
+    w.sync();
+    const int any = warp_or(w, e);
     if (any) err = CELL_CEA_RANGE;
 }
 
-// tick rates, then q and L per species in reaction order (reaction_mechanism.d:82-96)
-__device__ void w_split_rates(const WarpCtx& w, const double* c, double* q, double* L, const double* kf,
-                              const double* kb, double* wf, double* wb, double* meff) {
-    const MechView& m = w.m;
-    const int neff = m.neff;
-    // third bodies (reaction.d:450-456): the lists spread over all lanes, 2^n lanes to a list
-    int per = 1;
-    while (2 * per * neff <= 32) per *= 2;
-    for (int s0 = 0; s0 < neff; s0 += 32 / per) {
-        const int s = s0 + w.lane / per;
-        double term = 0.0;
-        if (s < neff) {
-            const int len = w.efflen[s];
-            for (int k = w.lane & (per - 1); k < len; k += per) term = fma(w.effval[k * neff + s], c[w.effidx[k * neff + s]], term);
+// The sum of a task's terms: W 2^shift of each entry.  The alpha-QSS sums are taken on the integer pipe, where a term
+// costs about 22 cycles beside the FP64 pipe that an addition would hold for 76 (chem_group.cuh's grp_gather): the
+// terms, all >= 0, are aligned to the largest with 5 bits below its last, and the sum is rounded once.
+template <int METHOD, int NL>
+__device__ __forceinline__ double w_gather(const unsigned short* ent, int n, const double* W) {
+    if (METHOD != METHOD_RKF) {
+        const unsigned* H = reinterpret_cast<const unsigned*>(W) + 1;
+        unsigned mx = 0;
+#pragma unroll 4
+        for (int k = 0; k < n; ++k) {
+            const unsigned x = ent[k * NL];
+            mx = max(mx, H[2 * (x & 0x1fff)] + ((x >> 13) << 20));
         }
-        for (int o = 1; o < per; o <<= 1) term += __shfl_xor_sync(FULL_MASK, term, o);
-        if (s < neff && !(w.lane & (per - 1))) meff[s] = term;
+        if (mx == 0) return 0.0;   // absent species' rates: all terms below 2^-1054
+        if (mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {   // a normal largest term, far from the range's ends
+            const int E6 = (int)(mx >> 20) + 6;
+            unsigned long long acc = 0;
+#pragma unroll 4
+            for (int k = 0; k < n; ++k) {
+                const unsigned x = ent[k * NL];
+                const unsigned long long v = (unsigned long long)__double_as_longlong(W[x & 0x1fff]);
+                const int ve = (int)(v >> 52), d = E6 - ve - (int)(x >> 13);
+                if (ve != 0 && d < 64) acc += ((v << 11) | 0x8000000000000000ull) >> d;
+            }
+            const int c = __clzll((long long)acc);   // 1..6
+            acc <<= c;
+            return __longlong_as_double(
+                (long long)((acc >> 11) + ((acc >> 10) & 1) + ((unsigned long long)(unsigned)(E6 - c - 1) << 52)));
+        }
     }
-    for (int i = w.lane; i < m.nsp; i += 32) { q[i] = 0.0; L[i] = 0.0; }
-    __syncwarp();
-    for (int ir = w.lane; ir < m.nr; ir += 32) {
-        double f = kf[ir], b = kb[ir];
-        const int e = w.rxeff[ir];
-        if (e >= 0) { const double t = meff[e]; f = f * t; b = b * t; }
-        const int k0 = w.tstart[ir], km = w.tmid[ir], k1 = w.tstart[ir + 1];
-        for (int k = k0; k < km; ++k) f *= ipow(c[w.terms[k] & 0xff], w.terms[k] >> 8);
-        for (int k = km; k < k1; ++k) b *= ipow(c[w.terms[k] & 0xff], w.terms[k] >> 8);
-        wf[ir] = f;
-        wb[ir] = b;
-    }
-    __syncwarp();
-    for (int j = w.lane; j < w.nslot; j += 32) {   // (double)nu * w, as the reference forms it
-        const int sl = w.slot[j], ir = sl & 0xffff;
-        const double nu = (double)(sl >> 16);
-        w.wsf[j] = nu * wf[ir];
-        w.wsb[j] = nu * wb[ir];
-    }
-    __syncwarp();
-    // q, L: each of this lane's tasks adds its terms in reaction order from 0 (reaction_mechanism.d:82-96);
-    // an entry's index runs over w_f, w_b and the slots' |nu| w_f, |nu| w_b, which lie end to end.  A task that
-    // is longer than a lane's fair share (a long species of the acetylene model, H, has 187 terms) is split; its later
-    // parts go to w.part and are added below.
-    int cur = -1;
     double sum = 0.0;
-    auto flush = [&]() {
-        if (cur & 0x80) w.part[cur & 0x7f] = sum;
-        else ((cur >> 21) ? L : q)[cur & 0x7f] = sum;
-    };
-    for (int k = w.ent_lo; k < w.ent_hi; ++k) {
-        const int e = w.ent[k];
-        const int key = e & 0x2000ff;   // target and the q / L bit
-        const double v = wf[(e >> 8) & 0x1fff];
-        if (key != cur) {
-            if (cur >= 0) flush();
-            cur = key;
-            sum = v;
-        } else {
-            sum += v;
-        }
+    for (int k = 0; k < n; ++k) {
+        const unsigned x = ent[k * NL];
+        sum = fma((double)(1u << (x >> 13)), W[x & 0x1fff], sum);
     }
-    if (cur >= 0) flush();
-    __syncwarp();
-    for (int k = w.lane; k < w.ncomb; k += 32) {
-        const int e = w.comb[k], first = (e >> 8) & 0xff, n = e >> 16;
-        double* dst = ((e & 0x80) ? L : q) + (e & 0x7f);
-        double v = *dst;
-        for (int j = 0; j < n; ++j) v += w.part[first + j];
-        *dst = v;
-    }
-    __syncwarp();
+    return sum;
 }
 
-__device__ double w_estimate(const WarpCtx& w, const double* c, const double* q, const double* L) {
+// tick rates, then q and L per species in reaction order (reaction_mechanism.d:82-96)
+template <int METHOD, int NW>
+__device__ void w_split_rates(const WarpCtx<NW>& w, const double* c, double* q, double* L, const double* kf,
+                              const double* kb, double* wf, double* wb, double* meff) {
+    constexpr int NL = 32 * NW;
+    const MechView& m = w.m;
+    // third bodies (reaction.d:450-456): eight lanes to a list
+    for (int s0 = 0; s0 < m.neff; s0 += NL / 8) {
+        const int s = s0 + w.lane / 8;
+        double term = 0.0;
+        if (s < m.neff) {
+            const double* ef = w.eff + s * m.nsp;
+            for (int i = w.lane & 7; i < m.nsp; i += 8) term = fma(ef[i], c[i], term);
+        }
+        for (int o = 1; o < 8; o <<= 1) term += __shfl_xor_sync(FULL_MASK, term, o);
+        if (s < m.neff && !(w.lane & 7)) meff[s] = term;
+    }
+    for (int i = w.lane; i < 2 * m.nsp; i += NL) q[i] = 0.0;   // and L, which follows
+    w.sync();
+    for (int k = w.lane; k < m.nr; k += NL) {
+        double f = kf[k], b = kb[k];
+        const int e = w.rxm[k];
+        if (e & 0xffff) { const double t = meff[(e & 0xffff) - 1]; f = f * t; b = b * t; }
+        if (!(e & RX_LONG)) {
+            const uint4 x = w.rx[k];
+            unsigned long long F = (unsigned long long)x.y << 32 | x.x, B = (unsigned long long)x.w << 32 | x.z;
+            while (F | B) {
+                const unsigned tf = (unsigned)F & 0xffff, tb = (unsigned)B & 0xffff;
+                if (tf) f *= ipow(c[tf & 0xff], tf >> 8);
+                if (tb) b *= ipow(c[tb & 0xff], tb >> 8);
+                F >>= 16;
+                B >>= 16;
+            }
+        } else {
+            const int* ls = w.lstart + 3 * ((e >> 16) & 0x3fff);
+            for (int j = ls[0]; j < ls[1]; ++j) f *= ipow(c[w.lterms[j] & 0xff], w.lterms[j] >> 8);
+            for (int j = ls[1]; j < ls[2]; ++j) b *= ipow(c[w.lterms[j] & 0xff], w.lterms[j] >> 8);
+        }
+        wf[k] = f;
+        wb[k] = b;
+    }
+    w.sync();
+    // q, L: each of this lane's tasks adds its terms in reaction order (reaction_mechanism.d:82-96).  A long
+    // species' sum (H of the acetylene model has 187 terms) is split; its later parts are added below.
+    const unsigned short* ent = w.ent + w.lane;
+    for (int t = w.task_lo; t < w.task_hi; ++t) {
+        const int x = w.task[t], n = x >> 16;
+        q[x & 0xffff] = w_gather<METHOD, NL>(ent, n, wf);
+        ent += n * NL;
+    }
+    w.sync();
+    for (int k = w.lane; k < w.ncomb; k += NL) {
+        const int x = w.comb[2 * k], first = x >> 16, n = w.comb[2 * k + 1];
+        double v = q[x & 0xffff];
+        for (int j = 0; j < n; ++j) v += q[2 * m.nsp + first + j];
+        q[x & 0xffff] = v;
+    }
+    if (w.ncomb) w.sync();
+}
+
+template <int NW>
+__device__ double w_estimate(const WarpCtx<NW>& w, const double* c, const double* q, const double* L) {
     const double MUCH_LARGER_FACTOR = 10000.0, ZERO_TOL = 1.0e-30, EPS1 = 1.0e-3;
     double min_dt = 1.0e6;
-    for (int i = w.lane; i < w.m.nsp; i += 32) {
+    for (int i = w.lane; i < w.m.nsp; i += 32 * NW) {
         double ci = c[i], qi = q[i], Li = L[i], dt;
         if (ci > 0.0 && (fabs(qi - Li) > ZERO_TOL)) {
             if (qi > MUCH_LARGER_FACTOR * Li) dt = ci / (Li + ZERO_EPS);
@@ -930,7 +994,7 @@ __device__ double w_estimate(const WarpCtx& w, const double* c, const double* q,
             min_dt = fmin(min_dt, dt);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) min_dt = fmin(min_dt, __shfl_xor_sync(FULL_MASK, min_dt, o));
+    min_dt = w.reduce(min_dt, [](double a, double b) { return fmin(a, b); });
     double dt_chem = EPS1 * min_dt;
     dt_chem = fmin(dt_chem, 1.0e-10);
     dt_chem = fmax(dt_chem, 1.0e-15);
@@ -938,7 +1002,8 @@ __device__ double w_estimate(const WarpCtx& w, const double* c, const double* q,
 }
 
 // therm_perf_gas_mix.d:406-468 with the per-species terms in tmp[0..nsp) and tmp[nsp..2nsp)
-__device__ double w_T_from_u(const WarpCtx& w, const double* mf, double u_tgt, double T_guess, int& err, int& iters,
+template <int NW>
+__device__ double w_T_from_u(const WarpCtx<NW>& w, const double* mf, double u_tgt, double T_guess, int& err, int& iters,
                              double* tmp) {
     const MechView& m = w.m;
     const int n = m.nsp;
@@ -946,20 +1011,20 @@ __device__ double w_T_from_u(const WarpCtx& w, const double* mf, double u_tgt, d
     auto energy = [&](double T) {
         const double logT = log(T);
         int e = 0;
-        for (int i = w.lane; i < n; i += 32) tmp[i] = mf[i] * (cea_h(m, i, T, logT, e) - m.sp(i)[SP_R] * T);
-        __syncwarp();
-        if (warp_or(e)) err = CELL_CEA_RANGE;
+        for (int i = w.lane; i < n; i += 32 * NW) tmp[i] = mf[i] * (cea_h(m, i, T, logT, e) - m.sp(i)[SP_R] * T);
+        w.sync();
+        if (warp_or(w, e)) err = CELL_CEA_RANGE;
         const double s = serial_sum(w, tmp, n);
-        __syncwarp();
+        w.sync();
         return s;
     };
     auto cv = [&](double T) {
         int e = 0;
-        for (int i = w.lane; i < n; i += 32) tmp[n + i] = mf[i] * (cea_Cp(m, i, T, e) - m.sp(i)[SP_R]);
-        __syncwarp();
-        if (warp_or(e)) err = CELL_CEA_RANGE;
+        for (int i = w.lane; i < n; i += 32 * NW) tmp[n + i] = mf[i] * (cea_Cp(m, i, T, e) - m.sp(i)[SP_R]);
+        w.sync();
+        if (warp_or(w, e)) err = CELL_CEA_RANGE;
         const double s = serial_sum(w, tmp + n, n);
-        __syncwarp();
+        w.sync();
         return s;
     };
     double T = T_guess;
@@ -977,22 +1042,25 @@ __device__ double w_T_from_u(const WarpCtx& w, const double* mf, double u_tgt, d
     return T;
 }
 
-__device__ double w_gas_constant(const WarpCtx& w, const double* mf, double* tmp) {
-    for (int i = w.lane; i < w.m.nsp; i += 32) tmp[i] = mf[i] * w.m.sp(i)[SP_R];
-    __syncwarp();
+template <int NW>
+__device__ double w_gas_constant(const WarpCtx<NW>& w, const double* mf, double* tmp) {
+    for (int i = w.lane; i < w.m.nsp; i += 32 * NW) tmp[i] = mf[i] * w.m.sp(i)[SP_R];
+    w.sync();
     const double r = serial_sum(w, tmp, w.m.nsp);
-    __syncwarp();
+    w.sync();
     return r;
 }
 
 // lane 0: Phobos' pairwise sum of v[0..n), broadcast
-__device__ double w_sum_pairwise(const WarpCtx& w, double* v, int n) {
+template <int NW>
+__device__ double w_sum_pairwise(const WarpCtx<NW>& w, double* v, int n) {
     double s = 0.0;
     if (w.lane == 0) s = sum_pairwise(Vec{v, 1}, n);
-    return bcast(s);
+    return w.bcast(s);
 }
 
-__device__ bool w_rkf_step(const WarpCtx& w, const double* y0, double h, double* yOut, double& hSuggest, double* q,
+template <int NW>
+__device__ bool w_rkf_step(const WarpCtx<NW>& w, const double* y0, double h, double* yOut, double& hSuggest, double* q,
                            double* L, const double* kf, const double* kb, double* wf, double* wb, double* meff,
                            double* ext, double* tmp, int& nrhs) {
     const double a21 = 1. / 5., a31 = 3. / 40., a32 = 9. / 40., a41 = 3. / 10., a42 = -9. / 10., a43 = 6. / 5.,
@@ -1004,39 +1072,39 @@ __device__ bool w_rkf_step(const WarpCtx& w, const double* y0, double h, double*
     double *k1 = ext, *k2 = ext + n, *k3 = ext + 2 * n, *k4 = ext + 3 * n, *k5 = ext + 4 * n, *k6 = ext + 5 * n,
            *yT = ext + 6 * n;
     auto rates = [&](const double* c, double* out) {
-        w_split_rates(w, c, q, L, kf, kb, wf, wb, meff);
+        w_split_rates<METHOD_RKF>(w, c, q, L, kf, kb, wf, wb, meff);
         ++nrhs;
-        for (int i = w.lane; i < n; i += 32) out[i] = q[i] - L[i];
-        __syncwarp();
+        for (int i = w.lane; i < n; i += 32 * NW) out[i] = q[i] - L[i];
+        w.sync();
     };
     rates(y0, k1);
-    for (int i = w.lane; i < n; i += 32) yT[i] = y0[i] + h * (a21 * k1[i]);
-    __syncwarp();
+    for (int i = w.lane; i < n; i += 32 * NW) yT[i] = y0[i] + h * (a21 * k1[i]);
+    w.sync();
     rates(yT, k2);
-    for (int i = w.lane; i < n; i += 32) yT[i] = y0[i] + h * (a31 * k1[i] + a32 * k2[i]);
-    __syncwarp();
+    for (int i = w.lane; i < n; i += 32 * NW) yT[i] = y0[i] + h * (a31 * k1[i] + a32 * k2[i]);
+    w.sync();
     rates(yT, k3);
-    for (int i = w.lane; i < n; i += 32) yT[i] = y0[i] + h * (a41 * k1[i] + a42 * k2[i] + a43 * k3[i]);
-    __syncwarp();
+    for (int i = w.lane; i < n; i += 32 * NW) yT[i] = y0[i] + h * (a41 * k1[i] + a42 * k2[i] + a43 * k3[i]);
+    w.sync();
     rates(yT, k4);
-    for (int i = w.lane; i < n; i += 32) yT[i] = y0[i] + h * (a51 * k1[i] + a52 * k2[i] + a53 * k3[i] + a54 * k4[i]);
-    __syncwarp();
+    for (int i = w.lane; i < n; i += 32 * NW) yT[i] = y0[i] + h * (a51 * k1[i] + a52 * k2[i] + a53 * k3[i] + a54 * k4[i]);
+    w.sync();
     rates(yT, k5);
-    for (int i = w.lane; i < n; i += 32)
+    for (int i = w.lane; i < n; i += 32 * NW)
         yT[i] = y0[i] + h * (a61 * k1[i] + a62 * k2[i] + a63 * k3[i] + a64 * k4[i] + a65 * k5[i]);
-    __syncwarp();
+    w.sync();
     rates(yT, k6);
     const double atol = w.m.err_tol(), rtol = w.m.err_tol();
-    for (int i = w.lane; i < n; i += 32) {
+    for (int i = w.lane; i < n; i += 32 * NW) {
         double yo = y0[i] + h * (b51 * k1[i] + b53 * k3[i] + b54 * k4[i] + b56 * k6[i]);
         yOut[i] = yo;
         double ye = yo - (y0[i] + h * (b41 * k1[i] + b43 * k3[i] + b44 * k4[i] + b45 * k5[i] + b46 * k6[i]));
         double sk = atol + rtol * fmax(fabs(y0[i]), fabs(yo));
         tmp[i] = (ye / sk) * (ye / sk);
     }
-    __syncwarp();
+    w.sync();
     double err = serial_sum(w, tmp, n);
-    __syncwarp();
+    w.sync();
     err = sqrt(err / n);
     const double maxscale = 10.0, minscale = 0.2, safe = 0.9, alpha = 0.2;
     double scale;
@@ -1085,16 +1153,17 @@ __device__ __forceinline__ void w_alpha_nd(double s, double& N, double& D) {
 // divisions instead of four, by the refined hardware reciprocal (fast_exp.h); sigma as the largest ratio
 // found by cross products, one division per lane.  Mathematically the reference's step, in rounding only
 // different.
-__device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double* yOut, double& hSuggest, double* q,
+template <int NW>
+__device__ bool w_aqss_step(const WarpCtx<NW>& w, const double* y0, double h, double* yOut, double& hSuggest, double* q,
                             double* L, const double* kf, const double* kb, double* wf, double* wb, double* meff,
                             double* ext, int& nrhs) {
     const MechView& m = w.m;
     const int n = m.nsp;
     const double eps1 = m.eps1(), eps2 = m.eps2(), delta = m.delta();
     double *q0 = ext, *p0 = ext + n, *yp0 = ext + 2 * n, *yp = ext + 3 * n;   // p0 holds p0 / 2
-    w_split_rates(w, y0, q, L, kf, kb, wf, wb, meff);
+    w_split_rates<METHOD_ALPHA_QSS>(w, y0, q, L, kf, kb, wf, wb, meff);
     ++nrhs;
-    for (int i = w.lane; i < n; i += 32) {
+    for (int i = w.lane; i < n; i += 32 * NW) {
         const double y = y0[i];
         const double qi = q[i];
         const double pi = w_qss_p(L[i], y);
@@ -1103,13 +1172,13 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
         const double v = y + gdtk_div(h * (D * fma(-pi, y, qi)), fma(N, h * pi, D));
         q0[i] = qi; p0[i] = 0.5 * pi; yp[i] = v; yp0[i] = v;
     }
-    __syncwarp();
+    w.sync();
     bool converged = false;
     for (int corr = 0; corr < m.max_iters(); ++corr) {
-        w_split_rates(w, yp, q, L, kf, kb, wf, wb, meff);
+        w_split_rates<METHOD_ALPHA_QSS>(w, yp, q, L, kf, kb, wf, wb, meff);
         ++nrhs;
         bool conv = true;
-        for (int i = w.lane; i < n; i += 32) {
+        for (int i = w.lane; i < n; i += 32 * NW) {
             const double y = y0[i];
             const double pp = w_qss_p(L[i], yp[i]);
             double N, D;
@@ -1122,12 +1191,12 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
                 if (!w_below(test, tol) && !w_nan(test)) conv = false;
             }
         }
-        __syncwarp();
-        converged = __all_sync(FULL_MASK, conv);
+        converged = !w.any(!conv);   // and all of yp is written
+        if (NW == 1) __syncwarp();
         if (converged) break;
     }
     double snum = 0.0, sden = 1.0;   // this lane's largest |yc - yp0| / (eps2 (yc + delta))
-    for (int i = w.lane; i < n; i += 32) {
+    for (int i = w.lane; i < n; i += 32 * NW) {
         const double yc = yp[i];
         if (!w_present(yc)) continue;
         const double num = fabs(yc - yp0[i]), den = fma(eps2, yc, eps2 * delta);
@@ -1135,56 +1204,57 @@ __device__ bool w_aqss_step(const WarpCtx& w, const double* y0, double h, double
         if (w_below(b, a) && !w_nan(a)) { snum = num; sden = den; }
     }
     double sigma = gdtk_div(snum, sden);
-    for (int o = 16; o > 0; o >>= 1) {
-        const double other = __shfl_xor_sync(FULL_MASK, sigma, o);
-        if (other > sigma) sigma = other;
+    sigma = w.reduce(sigma, [](double a, double b) { return b > a ? b : a; });
+    double h_new = 0.0;
+    if (w.lane < 32) {   // one warp, for the FP64 pipe's sake
+        if (sigma <= 0.0) h_new = 10.0 * h;
+        else {
+            double x = sigma;
+            x = x - 0.5 * gdtk_div(x * x - sigma, x);
+            x = x - 0.5 * gdtk_div(x * x - sigma, x);
+            x = x - 0.5 * gdtk_div(x * x - sigma, x);
+            h_new = h * (gdtk_rcp(x) + 0.005);
+        }
     }
-    double h_new;
-    if (sigma <= 0.0) h_new = 10.0 * h;
-    else {
-        double x = sigma;
-        x = x - 0.5 * gdtk_div(x * x - sigma, x);
-        x = x - 0.5 * gdtk_div(x * x - sigma, x);
-        x = x - 0.5 * gdtk_div(x * x - sigma, x);
-        h_new = h * (gdtk_rcp(x) + 0.005);
-    }
-    hSuggest = h_new;
+    hSuggest = NW == 1 ? h_new : w.bcast(h_new);
     if (converged)
-        for (int i = w.lane; i < n; i += 32) yOut[i] = yp[i];
-    __syncwarp();
+        for (int i = w.lane; i < n; i += 32 * NW) yOut[i] = yp[i];
+    w.sync();
     return converged;
 }
 
-template <int METHOD>
+// Tables first, then each cell's vectors.  A block holds cells = blockDim.x / (32 NW) of them; the warps of a cell meet at
+// named barrier 1 + cell, and everything that decides its control flow is the same in all of them.
+template <int METHOD, int NW>
 __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTables tb, int warp_doubles) {
-    extern __shared__ double smem_w[];
+    extern __shared__ __align__(16) double smem_w[];
     int* ti = reinterpret_cast<int*>(smem_w);
     for (int k = threadIdx.x; k < tb.n_smem_ints; k += blockDim.x) ti[k] = tb.gi[k];
     __syncthreads();
-    WarpCtx w;
+    const int cell = threadIdx.x / (32 * NW);
+    WarpCtx<NW> w;
     w.m.bind(a.mech_i, a.mech_d);
-    w.lane = threadIdx.x & 31;
-    w.tstart = ti + tb.off_tstart;
-    w.tmid = ti + tb.off_tmid;
-    w.terms = ti + tb.off_terms;
-    w.rxeff = ti + tb.off_rxeff;
-    w.slot = ti + tb.off_slot;
-    w.nslot = tb.nslot;
-    w.ent = ti + tb.off_ent;
-    w.ent_lo = ti[tb.off_lane + w.lane];
-    w.ent_hi = ti[tb.off_lane + w.lane + 1];
-    w.efflen = tb.gi + tb.off_efflen;
-    w.effidx = tb.gi + tb.off_effidx;
-    w.effval = tb.eff_val;
-    const MechView& m = w.m;
-    WarpLayout lay;
-    lay.make(m.nsp, m.nr, m.neff, METHOD, tb.nslot, tb.npart);
-    double* S = smem_w + (tb.n_smem_ints + 1) / 2 + (size_t)(threadIdx.x >> 5) * warp_doubles;
-    w.wsf = S + lay.wsf;
-    w.wsb = S + lay.wsb;
-    w.part = S + lay.part;
+    w.lane = threadIdx.x % (32 * NW);
+    w.bar = 1 + cell;
+    w.rx = reinterpret_cast<const uint4*>(ti);
+    w.rxm = ti + tb.off_rxm;
+    w.lstart = tb.gi + tb.off_lstart;
+    w.lterms = tb.gi + tb.off_lterms;
+    w.perm = tb.gi + tb.off_perm;
+    w.ent = reinterpret_cast<const unsigned short*>(ti + tb.off_ent);
+    w.task = ti + tb.off_task;
+    w.task_lo = ti[tb.off_lane + w.lane];
+    w.task_hi = ti[tb.off_lane + w.lane + 1];
     w.comb = ti + tb.off_comb;
     w.ncomb = tb.ncomb;
+    w.M = reinterpret_cast<const double*>(ti + tb.off_M);
+    w.eff = tb.off_eff < tb.n_smem_ints ? reinterpret_cast<const double*>(ti + tb.off_eff)
+                                        : reinterpret_cast<const double*>(tb.gi + tb.off_eff);
+    const MechView& m = w.m;
+    WarpLayout lay;
+    lay.make(m.nsp, m.nr, m.neff, METHOD, tb.npart);
+    double* S = smem_w + tb.n_smem_ints / 2 + (size_t)cell * warp_doubles;
+    w.red = S + lay.red;
     double *y0 = S + lay.y0, *yout = S + lay.yout, *q = S + lay.q, *L = S + lay.L, *mf = S + lay.mf, *g = S + lay.g,
            *tmp = S + lay.tmp, *kf = S + lay.kf, *kb = S + lay.kb, *wf = S + lay.wf, *wb = S + lay.wb,
            *meff = S + lay.meff, *ext = S + lay.ext;
@@ -1194,7 +1264,7 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
     while (true) {
         unsigned c = 0;
         if (w.lane == 0) c = atomicAdd(a.counter, 1u);
-        c = __shfl_sync(FULL_MASK, c, 0);
+        c = (unsigned)w.bcast((double)c);
         if (c >= ncell) break;
         const double rho = a.rho[c], u = a.u[c], T0 = a.T[c], p0 = a.p[c];
         double dtS0 = a.dt_chem[c];
@@ -1206,6 +1276,7 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
             if (w.lane == 0 && a.status) a.status[c] = CELL_BAD_INPUT;
             continue;
         }
+        const double rrho = 1.0 / rho;
         bool retried = false;
         int n_steps = 0, n_rhs = 0, n_kc = 0, n_newton = 0, n_rej = 0, n_est = 0;
         int final_status = 0;
@@ -1215,17 +1286,17 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
             restart = false;
             int err = 0;
             T = T0; p = p0; dtS = dtS0; t = 0.0;
-            for (int i = w.lane; i < nsp; i += 32) {
+            for (int i = w.lane; i < nsp; i += 32 * NW) {
                 double v = a.massf[(size_t)i * ncell + c] * rho / m.sp(i)[SP_M];
                 y0[i] = (v < MIN_MOLES) ? 0.0 : v;
                 mf[i] = a.massf[(size_t)i * ncell + c];
             }
-            __syncwarp();
+            w.sync();
             w_rate_constants(w, T, kf, kb, g, mf, rho, err);
             ++n_kc;
             if (dtS > tI) h = tI;
             else if (dtS <= 0.0) {
-                w_split_rates(w, y0, q, L, kf, kb, wf, wb, meff);
+                w_split_rates<METHOD>(w, y0, q, L, kf, kb, wf, wb, meff);
                 ++n_rhs;
                 ++n_est;
                 h = w_estimate(w, y0, q, L);
@@ -1247,27 +1318,26 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
                                   ? w_rkf_step(w, y0, h, yout, dtS, q, L, kf, kb, wf, wb, meff, ext, tmp, n_rhs)
                                   : w_aqss_step(w, y0, h, yout, dtS, q, L, kf, kb, wf, wb, meff, ext, n_rhs);
                     if (ok) {   // mass-fraction test on conc2massf(concOut)
-                        for (int i = w.lane; i < nsp; i += 32) {
-                            double mfv = yout[i] * m.sp(i)[SP_M] / rho;
-                            tmp[i] = (mfv < MIN_MASS_FRACTION) ? 0.0 : mfv;
+                        double tot = 0.0;   // a test only: the sum's order is free
+                        for (int i = w.lane; i < nsp; i += 32 * NW) {
+                            const double mfv = yout[i] * (w.M[i] * rrho);
+                            tot += (mfv < MIN_MASS_FRACTION) ? 0.0 : mfv;
                         }
-                        __syncwarp();
-                        double tot = w_sum_pairwise(w, tmp, nsp);
-                        __syncwarp();
+                        tot = w.reduce(tot, [](double a, double b) { return a + b; });
                         if (fabs(tot - 1.0) > ALLOWABLE_MASSF_ERROR) ok = false;
                     }
                     if (ok) {
                         t += h;
-                        for (int i = w.lane; i < nsp; i += 32) y0[i] = yout[i];
-                        __syncwarp();
+                        for (int i = w.lane; i < nsp; i += 32 * NW) y0[i] = yout[i];
+                        w.sync();
                         double hMax = h * (1.0 + DT_INCREASE_PERCENT / 100.0);
                         if (dtS > h) h = fmin(dtS, hMax);
                         if (m.tight()) {   // chemistry_update.d:265-269
-                            for (int i = w.lane; i < nsp; i += 32) {
+                            for (int i = w.lane; i < nsp; i += 32 * NW) {
                                 double mfv = y0[i] * m.sp(i)[SP_M] / rho;
                                 mf[i] = (mfv < MIN_MASS_FRACTION) ? 0.0 : mfv;
                             }
-                            __syncwarp();
+                            w.sync();
                             T = w_T_from_u(w, mf, u, T, err, n_newton, tmp);
                             p = rho * w_gas_constant(w, mf, tmp) * T;
                             need_kc = true;
@@ -1303,15 +1373,15 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
         if (final_status) {
             if (w.lane == 0 && a.status) a.status[c] = final_status;
         } else {   // chemistry_update.d:290-325, then fluidfvcell.d:956
-            for (int i = w.lane; i < nsp; i += 32) {
+            for (int i = w.lane; i < nsp; i += 32 * NW) {
                 double mfv = y0[i] * m.sp(i)[SP_M] / rho;
                 q[i] = (mfv < MIN_MASS_FRACTION) ? 0.0 : mfv;
             }
-            __syncwarp();
+            w.sync();
             double tot = w_sum_pairwise(w, q, nsp);
-            __syncwarp();
-            for (int i = w.lane; i < nsp; i += 32) q[i] = q[i] / tot;
-            __syncwarp();
+            w.sync();
+            for (int i = w.lane; i < nsp; i += 32 * NW) q[i] = q[i] / tot;
+            w.sync();
             int st = 0;
             if (a.flags & CHEM_FLAG_UPDATE_THERMO) {
                 T = w_T_from_u(w, q, u, T, st, n_newton, tmp);
@@ -1320,7 +1390,7 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
             if (st) {
                 if (w.lane == 0 && a.status) a.status[c] = st;
             } else {
-                for (int i = w.lane; i < nsp; i += 32) a.massf[(size_t)i * ncell + c] = q[i];
+                for (int i = w.lane; i < nsp; i += 32 * NW) a.massf[(size_t)i * ncell + c] = q[i];
                 if (w.lane == 0) {
                     a.T[c] = T;
                     a.p[c] = p;
@@ -1347,7 +1417,7 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
                 atomicAdd(a.totals + 5, (unsigned long long)n_est);
             }
         }
-        __syncwarp();
+        w.sync();
     }
 }
 #endif   // GDTK_WARP_TU
@@ -1372,44 +1442,56 @@ cudaError_t launch_bucket_order(const float* key, int n, int* order, int* hist, 
 // ---------------------------------------------------------------- host-side launchers
 
 #if GDTK_WARP_TU
-int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot, int npart) {
+int chem_warp_doubles(int nsp, int nr, int neff, int method, int npart) {
     WarpLayout l;
-    l.make(nsp, nr, neff, method, nslot, npart);
-    return l.total;
+    l.make(nsp, nr, neff, method, npart);
+    return (l.total + 1) & ~1;
 }
 
-cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables& t, int warp_doubles,
+namespace {
+using WarpKernel = void (*)(ChemUpdateArgs, WarpTables, int);
+template <int METHOD>
+WarpKernel warp_kernel(int v) {
+    return v == 0 ? chem_warp_kernel<METHOD, 1> : v == 1 ? chem_warp_kernel<METHOD, 2> : chem_warp_kernel<METHOD, 4>;
+}
+}  // namespace
+
+cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info) {
     if (a.ncell <= 0) return cudaSuccess;
-    const size_t limit = 227 * 1024;
-    const size_t tables = (size_t)((t.n_smem_ints + 1) / 2) * 8, per_warp = (size_t)warp_doubles * 8;
-    if (tables + per_warp > limit) return cudaErrorInvalidConfiguration;
-    const void* fn = (method == METHOD_RKF) ? (const void*)chem_warp_kernel<METHOD_RKF>
-                                            : (const void*)chem_warp_kernel<METHOD_ALPHA_QSS>;
-    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
-    if (e != cudaSuccess) return e;
-    // the block size (warps each holding one cell's vectors beside the block's copy of the tables) that
-    // keeps the most warps resident per SM; ties go to the larger block
-    int warps = 0, per_sm = 0;
-    for (int w : {16, 12, 8, 6, 4, 2, 1}) {
-        if (tables + per_warp * w > limit) continue;
-        int nb = 0;
-        e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, fn, 32 * w, tables + per_warp * w);
-        if (e != cudaSuccess) return e;
-        if (nb * w > per_sm * warps) { warps = w; per_sm = nb; }
+    const size_t limit = 227 * 1024, per_cell = (size_t)warp_doubles * 8;
+    const int share = (a.ncell + sm_count - 1) / sm_count;   // cells for an SM
+    // Warps per cell: as many as leave an SM the cells that it can have at all, its share or what shared memory
+    // holds, in 16 warps (128 registers a thread).  Acetylene cells over 1e-6 s: 304 with four warps 18.7 ms (63 with one),
+    // 1,000 with two 33.5 (63), 6,007 with two 91 (155).
+    int v = -1, cells = 0, per_sm = 0;
+    WarpKernel fn = nullptr;
+    size_t smem = 0;
+    for (int k = 2; k >= 0; --k) {
+        const int nw = 1 << k;
+        const size_t tables = (size_t)tabs[k].n_smem_ints * 4;
+        if (tables + per_cell > limit) continue;
+        int most = (int)((limit - tables) / per_cell), fit = 16 / nw < most ? 16 / nw : most;
+        if (k > 0 && fit < most && fit < share && fit < 16) continue;
+        v = k;
+        cells = fit < share ? fit : share;
+        break;
     }
-    if (warps < 1 || per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int block = 32 * warps;
-    const size_t smem = tables + per_warp * warps;
-    long long want = ((long long)a.ncell + warps - 1) / warps;
+    if (v < 0) return cudaErrorInvalidConfiguration;
+    fn = (method == METHOD_RKF) ? warp_kernel<METHOD_RKF>(v) : warp_kernel<METHOD_ALPHA_QSS>(v);
+    const int nw = 1 << v;
+    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+    if (e != cudaSuccess) return e;
+    smem = (size_t)tabs[v].n_smem_ints * 4 + per_cell * cells;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, 32 * nw * cells, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) return cudaErrorInvalidConfiguration;
+    const int block = 32 * nw * cells;
+    long long want = ((long long)a.ncell + cells - 1) / cells;
     long long grid = (long long)sm_count * per_sm;
     if (want < grid) grid = want;
-    if (grid < 1) grid = 1;
     if (info) { info->grid = (int)grid; info->block = block; info->smem = (int)smem; info->blocks_per_sm = per_sm; }
-    if (method == METHOD_RKF)
-        chem_warp_kernel<METHOD_RKF><<<(unsigned)grid, block, smem, stream>>>(a, t, warp_doubles);
-    else
-        chem_warp_kernel<METHOD_ALPHA_QSS><<<(unsigned)grid, block, smem, stream>>>(a, t, warp_doubles);
+    fn<<<(unsigned)grid, block, smem, stream>>>(a, tabs[v], warp_doubles);
     return cudaGetLastError();
 }
 

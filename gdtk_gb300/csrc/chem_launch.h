@@ -55,34 +55,38 @@ int chem_scratch_doubles(int nsp, int nr, int neff, int method);
 cudaError_t launch_chem_update(const ChemUpdateArgs& a, int method, int scratch_doubles, int sm_count,
                                cudaStream_t stream, LaunchInfo* info);
 cudaError_t launch_gas_service(const GasServiceArgs& a, int sm_count, cudaStream_t stream);
-// One warp per cell (mechanisms too large for the thread-per-cell kernels): the reference-order update with
-// species and reactions over the lanes.  Its tables (built by the host from the packed mechanism):
+// One, two or four warps per cell (mechanisms too large for the thread-per-cell kernels): the reference-order update
+// with species and reactions over the lanes.  Its tables (built by the host from the packed mechanism, one set for each
+// number of warps):
 //   ints [0, n_smem_ints), staged in shared memory by every block:
-//     [off_tstart + ir]  first concentration term of reaction ir (nr + 1 entries)
-//     [off_tmid + ir]    first product term of reaction ir
-//     [off_terms + k]    term k: species | coeff << 8; reactants, then products, each in the reaction's order
-//     [off_rxeff + ir]   efficiency list of reaction ir's third body, or -1
-//     [off_slot + j]     scaled tick-rate slot j: reaction | |nu| << 16, for each (reaction, |nu| >= 2) pair
-//     [off_lane + l]     first gather entry of lane l (33 entries)
-//     [off_ent + k]      gather entry: target | index << 8 | (1 for L) << 21, adding element `index` of
-//                        the warp's w_f[nr], w_b[nr], |nu| w_f[nslot], |nu| w_b[nslot] (end to end) to q or
-//                        L of the species `target`, or to partial sum target - 128.  The tasks (one species' q,
-//                        or its L; those longer than a lane's share in parts) are dealt to the lanes,
-//                        longest first; a task's entries are in ascending reaction order
-//     [off_comb + k]     split task k: species | (1 for L) << 7 | first partial sum << 8 | their number << 16
-//   ints [off_efflen, ...) and doubles, read from global memory:
-//     [off_efflen + s]            length of efficiency list s
-//     [off_effidx + k*neff + s]   species of the k-th entry of list s (transposed: lanes read one list each)
-//     eff_val[k*neff + s]         its efficiency
+//     [4 k]              reaction at position k: up to four reactant and four product factors, 16 bits each, species |
+//                        coeff << 8; the reactions are sorted by their numbers of factors and third bodies
+//     [off_rxm + k]      efficiency list of its third body + 1, or 0; with RX_LONG (more factors, or larger coefficients)
+//                        its number among the long reactions << 16 as well
+//     [off_M + 2 i]      molar mass of species i (a double)
+//     [off_lane + l]     first gather task of lane l (one entry more than lanes)
+//     [off_task + t]     task t: target | number of entries << 16.  Targets: q of each species, L of each, partial sums.
+//                        A species' q or L of more than a 128th of all entries is split into parts, the later ones
+//                        partial sums; the tasks are dealt to the lanes, longest first
+//     [off_ent]          16-bit entries [k][lane], a lane's tasks one after the other: index | shift << 13, adding element
+//                        `index` of w_f[nr], w_b[nr] (end to end) times 2^shift.  Ascending reaction order
+//     [off_comb + 2 k]   split task k: target | first partial sum << 16, and their number
+//     [off_eff + 2 (s nsp + i)]   efficiency of species i in list s (doubles); read from global memory if they lie past
+//                        n_smem_ints
+//   ints read from global memory:
+//     [off_perm + k]     the reaction at position k
+//     [off_lstart + 3 j] long reaction j: its first term, its first product term, its end
+//     [off_lterms + k]   term: species | coeff << 8
 struct WarpTables {
     const int* gi;
-    const double* eff_val;
-    int n_smem_ints, nslot, npart, ncomb;
-    int off_tstart, off_tmid, off_terms, off_rxeff, off_slot, off_lane, off_ent, off_comb, off_efflen, off_effidx;
+    int n_smem_ints, npart, ncomb;
+    int off_rxm, off_M, off_lane, off_task, off_ent, off_comb, off_eff, off_perm, off_lstart, off_lterms;
 };
-// Shared-memory doubles of one warp's vectors.
-int chem_warp_doubles(int nsp, int nr, int neff, int method, int nslot, int npart);
-cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables& t, int warp_doubles,
+constexpr int RX_LONG = 1 << 30;
+constexpr int WARP_VARIANTS = 3;   // 1, 2, 4 warps per cell
+// Shared-memory doubles of one cell's vectors.
+int chem_warp_doubles(int nsp, int nr, int neff, int method, int npart);
+cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info);
 // Cost buckets of the longest-first ordering: launch_bucket_order's hist scratch holds this many ints.
 constexpr int ORDER_BUCKETS = 256;
