@@ -755,7 +755,8 @@ __global__ void order_scatter(const float* key, int n, int* hist, int* order) {
 // A right-hand side of the acetylene mechanism (75 species, 474 reactions) is a chain of latencies, shared memory's and
 // the FP64 pipe's: 31 us for a warp, with one cell on an SM or with the eight that shared memory holds.  Warps that
 // share a cell cut the chain and raise the warps in flight.  Four warps to a cell: 304 cells 63.1 -> 18.7 ms; two:
-// 6,007 cells 155 -> 91 ms (with the sums of q and L on the integer pipe and the reactions sorted, in both).
+// 6,007 cells 155 -> 91 ms (with the sums of q and L on the integer pipe and the reactions sorted, in both), and longest
+// cells first 75.
 constexpr unsigned FULL_MASK = 0xffffffffu;
 
 struct WarpLayout {
@@ -1225,8 +1226,10 @@ __device__ bool w_aqss_step(const WarpCtx<NW>& w, const double* y0, double h, do
 
 // Tables first, then each cell's vectors.  A block holds cells = blockDim.x / (32 NW) of them; the warps of a cell meet at
 // named barrier 1 + cell, and everything that decides its control flow is the same in all of them.
-template <int METHOD, int NW>
-__global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTables tb, int warp_doubles) {
+// With COST it only writes the cells' cost keys: the growth of the step from its start to the interval, and for alpha-QSS
+// a power of the fastest loss rate times the interval (the key of gdtk_chem_cost, chem_fast.cuh).
+template <int METHOD, int NW, bool COST>
+__global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTables tb, int warp_doubles, float* key) {
     extern __shared__ __align__(16) double smem_w[];
     int* ti = reinterpret_cast<int*>(smem_w);
     for (int k = threadIdx.x; k < tb.n_smem_ints; k += blockDim.x) ti[k] = tb.gi[k];
@@ -1266,8 +1269,36 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
         if (w.lane == 0) c = atomicAdd(a.counter, 1u);
         c = (unsigned)w.bcast((double)c);
         if (c >= ncell) break;
+        if (!COST && a.order) c = (unsigned)a.order[c];
         const double rho = a.rho[c], u = a.u[c], T0 = a.T[c], p0 = a.p[c];
         double dtS0 = a.dt_chem[c];
+        if (COST) {
+            float k = 0.0f;
+            if (T0 > a.T_frozen && rho > 0.0) {
+                int err = 0;
+                for (int i = w.lane; i < nsp; i += 32 * NW) {
+                    mf[i] = a.massf[(size_t)i * ncell + c];
+                    const double v = mf[i] * rho / w.M[i];
+                    y0[i] = (v < MIN_MOLES) ? 0.0 : v;
+                }
+                w.sync();
+                double h = fmin(dtS0, tI), x = 0.0;
+                if (METHOD != METHOD_RKF || !(dtS0 > 0.0)) {
+                    w_rate_constants(w, T0, kf, kb, g, mf, rho, err);
+                    w_split_rates<METHOD>(w, y0, q, L, kf, kb, wf, wb, meff);
+                    if (!(dtS0 > 0.0)) h = w_estimate(w, y0, q, L);
+                    if (METHOD != METHOD_RKF) {
+                        for (int i = w.lane; i < nsp; i += 32 * NW)
+                            if (y0[i] > 0.0) x = fmax(x, L[i] / y0[i]);
+                        x = w.reduce(x, [](double a, double b) { return fmax(a, b); });
+                    }
+                }
+                k = log1pf((float)(0.1 * tI / h)) * 10.4920587f + 40.0f * __powf((float)fmin(x * tI, 1.0e9), 0.4f);   // / ln 1.1
+            }
+            if (w.lane == 0) key[c] = k;
+            w.sync();
+            continue;
+        }
         if (T0 <= a.T_frozen) {
             if (w.lane == 0 && a.status) a.status[c] = CELL_FROZEN;
             continue;
@@ -1449,50 +1480,80 @@ int chem_warp_doubles(int nsp, int nr, int neff, int method, int npart) {
 }
 
 namespace {
-using WarpKernel = void (*)(ChemUpdateArgs, WarpTables, int);
+using WarpKernel = void (*)(ChemUpdateArgs, WarpTables, int, float*);
 template <int METHOD>
 WarpKernel warp_kernel(int v) {
-    return v == 0 ? chem_warp_kernel<METHOD, 1> : v == 1 ? chem_warp_kernel<METHOD, 2> : chem_warp_kernel<METHOD, 4>;
+    return v == 0 ? chem_warp_kernel<METHOD, 1, false>
+                  : v == 1 ? chem_warp_kernel<METHOD, 2, false> : chem_warp_kernel<METHOD, 4, false>;
+}
+
+struct WarpShape {
+    int v, cells, per_sm;   // variant (2^v warps per cell), cells per block, blocks per SM
+    WarpKernel fn;
+    size_t smem;
+};
+
+// Warps per cell, in 16 warps (128 registers a thread): four while the batch is the longest cells' latency, up to five
+// turns of the cells that an SM then holds; beyond that as many as leave an SM the cells that shared memory holds.
+// Acetylene cells over 1e-6 s with one / two / four warps, in ms: 400 44.5 / 29.1 / 18.3, 1,000 49.4 / 32.7 / 23.2, 2,500
+// 56.2 / 42.7 / 37.8, 6,007 90.2 / 75.1 / 83.9; 20,000 over 1e-7 s 140 / 122 / 136.  The cost keys take one warp.
+cudaError_t warp_shape(int ncell, int method, bool cost, const WarpTables* tabs, int warp_doubles, int sm_count,
+                       WarpShape& w) {
+    const size_t limit = 227 * 1024, per_cell = (size_t)warp_doubles * 8;
+    const int share = (ncell + sm_count - 1) / sm_count;   // cells for an SM
+    w.v = -1;
+    for (int k = cost ? 0 : 2; k >= 0; --k) {
+        const int nw = 1 << k;
+        const size_t tables = (size_t)tabs[k].n_smem_ints * 4;
+        if (tables + per_cell > limit) continue;
+        const int most = (int)((limit - tables) / per_cell), fit = 16 / nw < most ? 16 / nw : most;
+        if (k > 0 && fit < most && 5 * fit < share) continue;
+        w.v = k;
+        w.cells = fit < share ? fit : share;
+        break;
+    }
+    if (w.v < 0) return cudaErrorInvalidConfiguration;
+    w.fn = cost ? (method == METHOD_RKF ? chem_warp_kernel<METHOD_RKF, 1, true> : chem_warp_kernel<METHOD_ALPHA_QSS, 1, true>)
+                : (method == METHOD_RKF ? warp_kernel<METHOD_RKF>(w.v) : warp_kernel<METHOD_ALPHA_QSS>(w.v));
+    cudaError_t e = cudaFuncSetAttribute((const void*)w.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
+    if (e != cudaSuccess) return e;
+    w.smem = (size_t)tabs[w.v].n_smem_ints * 4 + per_cell * w.cells;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w.per_sm, (const void*)w.fn, (32 << w.v) * w.cells, w.smem);
+    if (e != cudaSuccess) return e;
+    return w.per_sm < 1 ? cudaErrorInvalidConfiguration : cudaSuccess;
+}
+
+cudaError_t launch_warp(const ChemUpdateArgs& a, const WarpShape& w, const WarpTables* tabs, int warp_doubles, int sm_count,
+                        float* key, cudaStream_t stream, LaunchInfo* info) {
+    const int block = (32 << w.v) * w.cells;
+    const long long want = ((long long)a.ncell + w.cells - 1) / w.cells;
+    long long grid = (long long)sm_count * w.per_sm;
+    if (want < grid) grid = want;
+    if (info) { info->grid = (int)grid; info->block = block; info->smem = (int)w.smem; info->blocks_per_sm = w.per_sm; }
+    w.fn<<<(unsigned)grid, block, w.smem, stream>>>(a, tabs[w.v], warp_doubles, key);
+    return cudaGetLastError();
 }
 }  // namespace
+
+int chem_warp_resident(int ncell, int method, const WarpTables* tabs, int warp_doubles, int sm_count) {
+    WarpShape w;
+    if (ncell <= 0 || warp_shape(ncell, method, false, tabs, warp_doubles, sm_count, w) != cudaSuccess) return 0;
+    return sm_count * w.per_sm * w.cells;
+}
+
+cudaError_t launch_chem_warp_cost(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
+                                  int sm_count, float* key, cudaStream_t stream) {
+    WarpShape w;
+    const cudaError_t e = warp_shape(a.ncell, method, true, tabs, warp_doubles, sm_count, w);
+    return e == cudaSuccess ? launch_warp(a, w, tabs, warp_doubles, sm_count, key, stream, nullptr) : e;
+}
 
 cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info) {
     if (a.ncell <= 0) return cudaSuccess;
-    const size_t limit = 227 * 1024, per_cell = (size_t)warp_doubles * 8;
-    const int share = (a.ncell + sm_count - 1) / sm_count;   // cells for an SM
-    // Warps per cell: as many as leave an SM the cells that it can have at all, its share or what shared memory
-    // holds, in 16 warps (128 registers a thread).  Acetylene cells over 1e-6 s: 304 with four warps 18.7 ms (63 with one),
-    // 1,000 with two 33.5 (63), 6,007 with two 91 (155).
-    int v = -1, cells = 0, per_sm = 0;
-    WarpKernel fn = nullptr;
-    size_t smem = 0;
-    for (int k = 2; k >= 0; --k) {
-        const int nw = 1 << k;
-        const size_t tables = (size_t)tabs[k].n_smem_ints * 4;
-        if (tables + per_cell > limit) continue;
-        int most = (int)((limit - tables) / per_cell), fit = 16 / nw < most ? 16 / nw : most;
-        if (k > 0 && fit < most && fit < share && fit < 16) continue;
-        v = k;
-        cells = fit < share ? fit : share;
-        break;
-    }
-    if (v < 0) return cudaErrorInvalidConfiguration;
-    fn = (method == METHOD_RKF) ? warp_kernel<METHOD_RKF>(v) : warp_kernel<METHOD_ALPHA_QSS>(v);
-    const int nw = 1 << v;
-    cudaError_t e = cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
-    if (e != cudaSuccess) return e;
-    smem = (size_t)tabs[v].n_smem_ints * 4 + per_cell * cells;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)fn, 32 * nw * cells, smem);
-    if (e != cudaSuccess) return e;
-    if (per_sm < 1) return cudaErrorInvalidConfiguration;
-    const int block = 32 * nw * cells;
-    long long want = ((long long)a.ncell + cells - 1) / cells;
-    long long grid = (long long)sm_count * per_sm;
-    if (want < grid) grid = want;
-    if (info) { info->grid = (int)grid; info->block = block; info->smem = (int)smem; info->blocks_per_sm = per_sm; }
-    fn<<<(unsigned)grid, block, smem, stream>>>(a, tabs[v], warp_doubles);
-    return cudaGetLastError();
+    WarpShape w;
+    const cudaError_t e = warp_shape(a.ncell, method, false, tabs, warp_doubles, sm_count, w);
+    return e == cudaSuccess ? launch_warp(a, w, tabs, warp_doubles, sm_count, nullptr, stream, info) : e;
 }
 
 #else

@@ -3,7 +3,7 @@ shared memory, changes no result; and factors that fill a table row, with coeffi
 too large for it.
 
 Slices of one cell up to a few cells per SM take four warps a cell, whole batches two (the acetylene mechanism) or one
-(small mechanisms with GDTK_CHEM_WARP_PER_CELL); every output is compared bit for bit, among them an invalid density
+(small mechanisms with GDTK_CHEM_WARP_PER_CELL, a slice of which takes two), longest first; every output is compared bit for bit, among them an invalid density
 and frozen cells."""
 import numpy as np
 import pytest
@@ -15,8 +15,8 @@ from test_gpu_parity import assert_parity, run_pair
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("name,n,flags,dt", [("c2h2", 1300, 3, 1.0e-7), ("park5", 4000, 3 | WARP_PER_CELL, 1.0e-6),
-                                             ("j92", 4000, 3 | WARP_PER_CELL, 1.0e-7)])
+@pytest.mark.parametrize("name,n,flags,dt", [("c2h2", 3100, 3, 1.0e-7), ("park5", 6200, 3 | WARP_PER_CELL, 1.0e-6),
+                                             ("j92", 6200, 3 | WARP_PER_CELL, 1.0e-7)])
 def test_number_of_warps_changes_no_result(name, n, flags, dt):
     import torch
     from gdtk_gb300.cells import ReactorCells
@@ -45,8 +45,9 @@ def test_number_of_warps_changes_no_result(name, n, flags, dt):
     ref = run(0, n)
     assert int(ref["status"][2]) == 5 and int((ref["status"] == 6).sum()) >= 1
     assert int((ref["status"] == 0).sum()) > 0.9 * n
-    for lo, m in ((0, 1), (1, 3), (0, 153), (7, 608), (2, 1217)):
-        got = run(lo, min(m, n - lo))
+    for lo, m in ((0, 1), (1, 3), (0, 153), (7, 608), (2, 1217), (1, 4000)):
+        m = min(m, n - lo)
+        got = run(lo, m)
         for k in ref:
             assert torch.equal(got[k], ref[k][..., lo:lo + m]), (lo, m, k)
     assert 4 in warps and max(warps) == 16   # one cell of four warps; a full block
