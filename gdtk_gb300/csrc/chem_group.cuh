@@ -155,9 +155,10 @@ __device__ __forceinline__ void grp_rate_constants(const GrpTab& tab, GrpCell& s
 #pragma unroll 1
         for (int f = gl; f < GDTK_NFALLOFF; f += L) {
             double M = 0.0;
+#pragma unroll 7
             for (int i = 0; i < GDTK_NSP; ++i) {
-                const double x = GRP_FALL_EFF[f * GDTK_NSP + i];
-                if (nonzero(x)) M = fma(x, c[i], M);
+                const double x = GRP_FALL_EFF[f * GDTK_NSP + i], y = fma(x, c[i], M);
+                M = nonzero(x) ? y : M;
             }
             G[GDTK_NSP + f] = M;
         }
@@ -285,15 +286,51 @@ __device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1
 }
 #endif
 
+// Lanes to a third-body sum: the L / G sums of a turn share its instructions, a sum's tree (grp_sum's) takes
+// 2 P2 / G - 1 of them in a lane and log2 G over its lanes.  The G of the fewest FP64 instructions; 3 sets of Park's 5
+// species with 32 lanes: 4 instructions where one sum after the other took 12 (4,096 cells 2.40 -> 2.04 ms).
+constexpr int set_cost(int L, int G) {
+    int lg = 0;
+    for (int x = 1; x < G; x <<= 1) ++lg;
+    return (GDTK_NSETS + L / G - 1) / (L / G) * (2 * (GRP_P2 / G) - 1 + lg);
+}
+constexpr int set_lanes(int L) {
+    int best = L < GRP_P2 ? L : GRP_P2;
+    for (int G = best; G >= 1 && GRP_P2 / G <= 4; G >>= 1)   // at most 4 values in a lane
+        if (set_cost(L, G) < set_cost(L, best)) best = G;
+    return best;
+}
+
 // q and L of every species at the concentrations c into S[GO_Q..], S[GO_L..] (gen_rhs).
 template <int L>
 __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, const double* c, int gl, bool act) {
     double* S = s.S;
+    constexpr int G = set_lanes(L);
+    if (G == L) {   // one sum after the other
 #pragma unroll 1
-    for (int m = 0; m < GDTK_NSETS; ++m) {
-        const double* ef = tab.eff + m * GDTK_NSP;
-        const double M = grp_sum<L>(gl, [&](int i) { return third_body(ef[i], c[i]); });
-        if (act && gl == 0) S[GO_M + m] = M;
+        for (int m = 0; m < GDTK_NSETS; ++m) {
+            const double* ef = tab.eff + m * GDTK_NSP;
+            const double M = grp_sum<L>(gl, [&](int i) { return third_body(ef[i], c[i]); });
+            if (act && gl == 0) S[GO_M + m] = M;
+        }
+    } else {
+        constexpr int KC = GRP_P2 / G;
+        const int base = (gl & (G - 1)) * KC;
+#pragma unroll 1
+        for (int m0 = 0; m0 < GDTK_NSETS; m0 += L / G) {
+            const int m = m0 + gl / G;
+            const double* ef = tab.eff + (m < GDTK_NSETS ? m : 0) * GDTK_NSP;
+            double v[KC];
+#pragma unroll
+            for (int k = 0; k < KC; ++k) v[k] = base + k < GDTK_NSP ? third_body(ef[base + k], c[base + k]) : 0.0;
+#pragma unroll
+            for (int w = 1; w < KC; w <<= 1)
+#pragma unroll
+                for (int k = 0; k < KC; k += 2 * w) v[k] += v[k + w];
+#pragma unroll
+            for (int x = 1; x < G; x <<= 1) v[0] += __shfl_xor_sync(GRP_FULL, v[0], x);
+            if (act && m < GDTK_NSETS && !(gl & (G - 1))) S[GO_M + m] = v[0];
+        }
     }
     __syncwarp(GRP_FULL);
     const double* K = S + GO_K;
