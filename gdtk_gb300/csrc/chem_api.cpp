@@ -149,7 +149,7 @@ struct ReactorObj {
     DevBuf<float> order_key;            // longest-first scheduling scratch
     DevBuf<int> order;
     DevBuf<int> order_hist;
-    // one warp per cell: for mechanisms beyond the thread-per-cell kernels' limits, or on request
+    // whole warps per cell: for mechanisms beyond the thread-per-cell kernels' limits, or on request
     bool large = false;                 // more than GDTK_MAX_SPECIES species or GDTK_MAX_REACTIONS reactions
     int warp_doubles = 0;
     DevBuf<int> wt_i;                   // warp-per-cell tables (WarpTables, chem_launch.h)
@@ -1010,7 +1010,7 @@ int chem_reactor_update_blocks(int cr_i, int nblock, const gdtk_cell_block* bloc
         if (flags & GDTK_CHEM_REFERENCE_ORDER)
             throw std::runtime_error("the block API runs the fast or the warp-per-cell kernel, not the reference-order one");
         cudaStream_t s = (cudaStream_t)stream;
-        if ((flags & GDTK_CHEM_WARP_PER_CELL) || r.large) {   // one warp per cell: one launch per block, in order
+        if ((flags & GDTK_CHEM_WARP_PER_CELL) || r.large) {   // whole warps per cell: one update per block, in order
             if (cell_counters)
                 throw std::runtime_error("per-cell counters of the block API need the thread-per-cell kernel");
             for (int k = 0; k < nblock; ++k) {

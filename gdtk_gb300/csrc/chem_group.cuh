@@ -1,9 +1,10 @@
 // chem_group.cuh -- the chemistry update with a group of L lanes per cell (L = 4, 8, 16, 32).
 //
-// Compiled by NVRTC after the generated prologue and chem_fast.cuh, whose arithmetic it shares: every cell's
-// result is bitwise the one-thread-per-cell kernel's, whatever L (sums over species take the same
-// zero-padded pairwise tree, gathers the same ascending order of reactions), so that the choice between
-// them, made from the batch's size, never shows in a result.
+// Compiled by NVRTC after the generated prologue and chem_fast.cuh, whose arithmetic it shares: a cell's
+// result does not depend on L, bit for bit (sums over species take the same zero-padded pairwise tree, gathers
+// the same ascending order of reactions), and for the Runge-Kutta method it is the one-thread-per-cell kernel's, so
+// that the choice among them, made from the batch's size, never shows in a result.  The alpha-QSS method, whose
+// q and L sums are rounded once here (grp_gather), takes a group for every size of batch.
 //
 // Why: an FP64 warp instruction costs 64 cycles (76 with all sub-partitions busy) however few of its lanes
 // are active, so with one cell per lane a step of the 13-species, 33-reaction H2-air mechanism takes

@@ -740,7 +740,7 @@ __global__ void order_scatter(const float* key, int n, int* hist, int* order) {
 
 
 #if GDTK_WARP_TU
-// ---------------------------------------------------------------- one warp per cell (large mechanisms)
+// ---------------------------------------------------------------- whole warps per cell (large mechanisms)
 // The reference-order update (chem_update_kernel above) with one, two or four warps (NW) integrating one cell: species
 // and reactions are spread over the lanes, and the cell's vectors live in its share of shared memory.  The
 // right-hand side reads compact tables (WarpTables) from shared memory: the reactions sorted by shape, so that the

@@ -27,7 +27,7 @@
 #define GDTK_MAX_SPECIES 32        // thread-per-cell kernels (fast, reference-order, surrogate, 2-T)
 #define GDTK_MAX_REACTIONS 128
 #define GDTK_MAX_SPECIES_ANY 128   // the reader; beyond GDTK_MAX_SPECIES / _REACTIONS the update runs one
-#define GDTK_MAX_REACTIONS_ANY 1024   // warp per cell
+#define GDTK_MAX_REACTIONS_ANY 1024   // whole warps per cell
 #define GDTK_MAX_SEGMENTS 4
 #define GDTK_MAX_EFFSETS 128
 #define GDTK_MAX_TERMS 4

@@ -43,12 +43,13 @@ enum gdtk_cell_status {
                                      the most expensive first, which shortens the tail; results
                                      do not depend on the order) */
 #define GDTK_CHEM_REFERENCE_ORDER 4 /* use the kernel that keeps the reference's operation order
-                                       (default: the mechanism-specialised kernel, which rearranges
-                                       the arithmetic to spend fewer FP64 operations) */
-#define GDTK_CHEM_WARP_PER_CELL 16  /* use the warp-per-cell kernel: the reference's operation order
-                                       with species and reactions spread over a warp's lanes.  It is
+                                       (default: the mechanism-specialised kernels, which rearrange
+                                       the arithmetic to spend fewer FP64 operations: a group of lanes
+                                       per cell or one thread per cell, by the batch's size) */
+#define GDTK_CHEM_WARP_PER_CELL 16  /* use the warp-per-cell kernel: the reference's update with species
+                                       and reactions spread over the lanes of one, two or four warps.  It is
                                        taken without the flag for mechanisms of more than 32 species or
-                                       128 reactions, which the thread-per-cell kernels do not take
+                                       128 reactions, which the specialised kernels do not take
                                        (the reader accepts up to 128 species and 1024 reactions) */
 
 /* ---- 1. libgas-compatible subset (gas_cwrap.d) ---------------------------------------- */
@@ -124,8 +125,8 @@ int chem_reactor_update_cells_ex(int cr_i, int ncell, const double* rho, const d
  * ordering the table by expected cost (most steps first) shortens the tail.  `first` is set
  * by the library.  The table is passed in the launch parameters: the call can be captured in a
  * CUDA graph and replayed.  cell_counters, when given, is int[6][total cells] in table order.
- * Mechanisms beyond 32 species / 128 reactions (or GDTK_CHEM_WARP_PER_CELL in flags) run one warp
- * per cell, one launch per block in table order (also capturable); cell_counters must then be NULL. */
+ * Mechanisms beyond 32 species / 128 reactions (or GDTK_CHEM_WARP_PER_CELL in flags) run whole warps
+ * per cell, one update per block in table order (also capturable); cell_counters must then be NULL. */
 typedef struct gdtk_cell_block {
     int ncell;
     int first;
@@ -212,10 +213,11 @@ int gdtk_exp_host(int n, const double* x, double* y);
  * copies the compiler log (register use) into log; 0 on success, -1 on a compile error. */
 int gdtk_compile_fast_source_check(const char* gas_file, const char* chem_file, int cc_major, int cc_minor,
                                    char* log, int n);
-/* Launch shape of the reactor's mechanism-specialised kernel: threads per block (a multiple of
- * 32) and resident blocks per SM it is compiled for (its register/shared-memory split).  0, 0
- * restores the default (largest block the shared-memory budget allows).  Compiles and loads the
- * variant now; later updates use it.  Used by the autotuner (gdtk_gb300/autotune.py). */
+/* Launch shape of the reactor's mechanism-specialised kernel of one thread per cell: threads per block
+ * (a multiple of 32) and resident blocks per SM it is compiled for (its register/shared-memory split);
+ * later updates run that kernel.  0, 0 restores the default: a group of lanes per cell or one thread
+ * (largest block that shared memory allows), by the batch's size.  Compiles and loads the
+ * variant now.  Used by the autotuner (gdtk_gb300/autotune.py). */
 int chem_reactor_configure(int cr_i, int block, int min_blocks);
 /* Work-queue refill of the mechanism-specialised kernel: with cells = 0 or 1 a warp takes, with one
  * atomic, exactly as many visit positions as it has lanes without a cell; with cells in 32..2^20 it
