@@ -1099,8 +1099,8 @@ cudaError_t launch_fast(FastKernel& k, FastArgs& a, int sm_count, cudaStream_t s
 // exceed `turns`: measured where two choices cross.  H2-air (13 species; ms with 4 / 8 / 16 / 32 lanes): 1,000 cells
 // 36 / 31 / 29 / 29, 12,000 63 / 52 / 48 / 54, 48,000 108 / 96 / 109 / 179, 262,147 364 / 437 / 575 / 975.  The
 // Runge-Kutta mechanisms are smaller (5 species) and their cells' step counts alike, so that no long tail
-// pays for lanes: 1,000 air cells 2.8 / 2.4 / 2.3 / 2.3, 4,000 2.7 / 2.3 / 2.9 / 3.5, 12,000 3.3 / 3.7 / 5.6 / 9.7;
-// one thread per cell takes 3.9 there and 4.9 at 30,000, where 4 lanes take 6.3.
+// pays for lanes: 1,000 air cells 2.6 / 1.9 / 1.7 / 1.8, 4,000 2.9 / 2.3 / 2.7 / 3.6, 12,000 3.5 / 4.3 / 5.8 / 9.6;
+// one thread per cell takes 4.2 there and 5.3 at 32,768, where 4 lanes take 8.3.
 int group_lanes(const FastKernel& k, long long total, int sm_count) {
     if (!k.group_function) return 0;
     const bool rkf = k.method == METHOD_RKF;
