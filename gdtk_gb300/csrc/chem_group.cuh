@@ -252,7 +252,8 @@ __device__ __forceinline__ double grp_ipow(double x, int n) {   // the order of 
 // The q and L sums of the alpha-QSS right-hand side on the integer pipe: a term takes about 22 cycles there, where
 // an FP64 addition takes 76 of the pipe that bounds the kernel (73% busy on the mixing layer), and the
 // terms do not wait for one another.  The terms, all >= 0, are aligned to the largest with 5 bits below its last
-// and the sum is rounded once, closer to the exact value than the chain of FP64 additions it replaces.
+// and the sum is rounded once, closer to the exact value than the chain of FP64 additions it replaces.  64 bits hold 64
+// terms of the largest one's size; a longer sum (128 reactions can give one 384 entries) is that chain.
 // 262,147 H2-air cells 400 -> 364 ms, 32,000 with 16 lanes 80.7 -> 72.0.  The tick rates' products stay FP64:
 // on the integer pipe, with its conversions, they took 391 to 517 ms.
 // sum of the entries' W 2^shift (index | shift << 16)
@@ -264,8 +265,9 @@ __device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1
         const unsigned x = ent[e];
         mx = max(mx, H[2 * (x & 0xffff)] + ((x >> 16) << 20));
     }
-    if (mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {   // a normal largest term, far from the range's ends
-        const int E6 = (int)(mx >> 20) + 6;
+    // at most 64 entries, and a normal largest term, far from the range's ends
+    if (e1 - e0 <= 64 && mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {
+        const int E6 = (int)(mx >> 20) + 6;   // the largest term's leading bit at 2^57
         uint64_t acc = 0;
 #pragma unroll 4
         for (int e = e0; e < e1; ++e) {
@@ -274,7 +276,7 @@ __device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1
             const int we = (int)(w >> 52), d = E6 - we - (int)(x >> 16);
             if (we != 0 && d < 64) acc += ((w << 11) | 0x8000000000000000ull) >> d;
         }
-        const int c = __clzll((long long)acc);   // 1..6
+        const int c = __clzll((long long)acc);   // 0..6
         acc <<= c;
         return __longlong_as_double((long long)((acc >> 11) + ((acc >> 10) & 1) + ((uint64_t)(unsigned)(E6 - c - 1) << 52)));
     }
