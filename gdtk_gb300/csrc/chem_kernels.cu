@@ -887,7 +887,8 @@ __device__ void w_rate_constants(const WarpCtx<NW>& w, double Tq, double* kf, do
 
 // The sum of a task's terms: W 2^shift of each entry.  The alpha-QSS sums are taken on the integer pipe, where a term
 // costs about 22 cycles beside the FP64 pipe that an addition would hold for 76 (chem_group.cuh's grp_gather): the
-// terms, all >= 0, are aligned to the largest with 5 bits below its last, and the sum is rounded once.
+// terms, all >= 0, are aligned to the largest with 5 bits below its last, and the sum is rounded once.  64 bits hold 64 terms
+// of the largest one's size; a part of more entries (from 8,193 entries of the mechanism on) is an FP64 chain.
 template <int METHOD, int NL>
 __device__ __forceinline__ double w_gather(const unsigned short* ent, int n, const double* W) {
     if (METHOD != METHOD_RKF) {
@@ -899,8 +900,9 @@ __device__ __forceinline__ double w_gather(const unsigned short* ent, int n, con
             mx = max(mx, H[2 * (x & 0x1fff)] + ((x >> 13) << 20));
         }
         if (mx == 0) return 0.0;   // absent species' rates: all terms below 2^-1054
-        if (mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {   // a normal largest term, far from the range's ends
-            const int E6 = (int)(mx >> 20) + 6;
+        // at most 64 entries, and a normal largest term, far from the range's ends
+        if (n <= 64 && mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {
+            const int E6 = (int)(mx >> 20) + 6;   // the largest term's leading bit at 2^57
             unsigned long long acc = 0;
 #pragma unroll 4
             for (int k = 0; k < n; ++k) {
@@ -909,7 +911,7 @@ __device__ __forceinline__ double w_gather(const unsigned short* ent, int n, con
                 const int ve = (int)(v >> 52), d = E6 - ve - (int)(x >> 13);
                 if (ve != 0 && d < 64) acc += ((v << 11) | 0x8000000000000000ull) >> d;
             }
-            const int c = __clzll((long long)acc);   // 1..6
+            const int c = __clzll((long long)acc);   // 0..6
             acc <<= c;
             return __longlong_as_double(
                 (long long)((acc >> 11) + ((acc >> 10) & 1) + ((unsigned long long)(unsigned)(E6 - c - 1) << 52)));

@@ -1,9 +1,10 @@
 """q and L sums of many terms of one size, against the oracle.
 
-The alpha-QSS kernel with a group of lanes per cell adds a sum's terms in 64-bit fixed point with room for 64 of the
-largest one (chem_group.cuh's grp_gather); longer sums are FP64 chains.  A mechanism with many copies of one reaction has
+The alpha-QSS kernels add a sum's terms in 64-bit fixed point with room for 64 of the largest one (chem_group.cuh's
+grp_gather, chem_kernels.cu's w_gather); longer sums are FP64 chains.  A mechanism with many copies of one reaction has
 sums of that many equal terms: 60, 62 (64 entries for one sum, 66 for another) and 100 copies, of a reaction with coefficients of 1
-and of one with a 2."""
+and of one with a 2, in the kernel with a group of lanes per cell; 990 copies of a reaction of six species in the one
+for large mechanisms, whose lanes then add parts of 94 terms."""
 import numpy as np
 import pytest
 
@@ -59,3 +60,15 @@ def test_copies_of_a_reaction(tmp_path, count, coeff):
     assert_parity(g, o)
     assert (g["status"] == 0).mean() > 0.95
 
+
+def test_a_thousand_copies_in_the_large_mechanism_kernel(tmp_path):
+    from gdtk_gb300.workloads import h2air_cells
+    text = open(mech("j92-chem.lua")).read()
+    # O + H2 + HO2 <=> H + O2 + H2O
+    text = _copies(text, 900, 990, 1.0e9, 0.0, 3.0e3, [(12, 1), (2, 1), (5, 1)], [(11, 1), (1, 1), (3, 1)])
+    rc, orc = _pair(tmp_path, "j92", text)
+    assert rc.nr > 1000
+    T, p, Y = h2air_cells(rc.species_names, rc.mol_masses, 192, seed=5, gas_file=rc.gmodel.file_name)
+    g, o, _, _ = run_pair(rc, orc, T, p, Y, 1.0e-7)
+    assert_parity(g, o)
+    assert (g["status"] == 0).mean() > 0.95
