@@ -259,14 +259,16 @@ __device__ __forceinline__ double grp_ipow(double x, int n) {   // the order of 
 // sum of the entries' W 2^shift (index | shift << 16)
 __device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1, const double* W) {
     const unsigned* H = reinterpret_cast<const unsigned*>(W) + 1;
-    unsigned mx = 0;
+    unsigned mx = 0, any = 0;
 #pragma unroll 4
     for (int e = e0; e < e1; ++e) {
-        const unsigned x = ent[e];
-        mx = max(mx, H[2 * (x & 0xffff)] + ((x >> 16) << 20));
+        const unsigned x = ent[e], h = H[2 * (x & 0xffff)];
+        mx = max(mx, h + ((x >> 16) << 20));
+        any |= h;
     }
-    // at most 64 entries, and a normal largest term, far from the range's ends
-    if (e1 - e0 <= 64 && mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {
+    // at most 64 entries, no sign (the scaling carries that of -inf or a NaN out of mx), and a normal largest term, so
+    // far from the range's ends that 64 of it have no infinite sum
+    if (e1 - e0 <= 64 && (int)any >= 0 && mx - 0x03600000u < 0x7f800000u - 0x03600000u) {
         const int E6 = (int)(mx >> 20) + 6;   // the largest term's leading bit at 2^57
         uint64_t acc = 0;
 #pragma unroll 4

@@ -893,15 +893,17 @@ template <int METHOD, int NL>
 __device__ __forceinline__ double w_gather(const unsigned short* ent, int n, const double* W) {
     if (METHOD != METHOD_RKF) {
         const unsigned* H = reinterpret_cast<const unsigned*>(W) + 1;
-        unsigned mx = 0;
+        unsigned mx = 0, any = 0;
 #pragma unroll 4
         for (int k = 0; k < n; ++k) {
-            const unsigned x = ent[k * NL];
-            mx = max(mx, H[2 * (x & 0x1fff)] + ((x >> 13) << 20));
+            const unsigned x = ent[k * NL], h = H[2 * (x & 0x1fff)];
+            mx = max(mx, h + ((x >> 13) << 20));
+            any |= h;
         }
-        if (mx == 0) return 0.0;   // absent species' rates: all terms below 2^-1054
-        // at most 64 entries, and a normal largest term, far from the range's ends
-        if (n <= 64 && mx - 0x03600000u < 0x7fe00000u - 0x03600000u) {
+        if (any == 0) return 0.0;   // absent species' rates: all terms below 2^-1042
+        // at most 64 entries, no sign (the scaling carries that of -inf or a NaN out of mx), and a normal largest term, so
+        // far from the range's ends that 64 of it have no infinite sum
+        if (n <= 64 && (int)any >= 0 && mx - 0x03600000u < 0x7f800000u - 0x03600000u) {
             const int E6 = (int)(mx >> 20) + 6;   // the largest term's leading bit at 2^57
             unsigned long long acc = 0;
 #pragma unroll 4
