@@ -228,7 +228,8 @@ std::string falloff_record(const ReactionHost& r, int ir) {
     };
     auto ln = [](double A) { return A > 0.0 ? std::log(A) : 0.0; };
     const bool troe = f.model == RATE_TROE, given = f.troe_flags & TROE_FCENT;
-    auto inv = [](double x) { return x != 0.0 ? -1.0 / x : 0.0; };
+    // -1 / x for exp(-T / x), which is 0 for x = 0: finite, so that it is a literal
+    auto inv = [](double x) { return std::max(-1.0e300, std::min(1.0e300, -1.0 / x)); };
     std::ostringstream o, sp, nu;
     int np = 0, nusum = 0;
     for (auto& pp : participants(r)) {
