@@ -116,6 +116,7 @@ SIGNATURES = {
                                                  ctypes.c_float, _v, _v]),
     "chem_surrogate_gradients": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _v, _v, _v, _v, _v, _v]),
     "chem_surrogate_predict": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _v, _v, _v]),
+    "chem_surrogate_predict_giving_up": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _v, _v, _v]),
     "chem_surrogate_set_gate": (ctypes.c_int, [ctypes.c_int, ctypes.c_double, ctypes.c_double, ctypes.c_double,
                                                ctypes.c_double]),
     "chem_surrogate_update_cells": (ctypes.c_int, [ctypes.c_int, ctypes.c_int, _v, _v, _v, _v, _v, _v, _v,

@@ -45,6 +45,7 @@ bool tcgen05_gemm_enabled();
 int tcgen05_gemm_set(int enable);                   // -1 leaves it; returns the previous setting
 unsigned long long tcgen05_gemm_launches();         // launches so far in this process
 cudaError_t tcgen05_gemm_error(int* error);         // not 0: a wait gave up (read and cleared)
+cudaError_t tcgen05_gemm_error_peek(int* error, cudaStream_t s);   // the same on a stream, not cleared
 cudaError_t launch_gemm_bf16_tcgen05(const GemmArgs& g, cudaStream_t s);
 
 // The network's inference in one launch (mlp_tcgen05.cu): layer sizes dims[0..nlayers], multiples of 8 up to 256,
@@ -60,6 +61,7 @@ struct FusedMlp {
     const float *X = nullptr, *xs = nullptr, *xd = nullptr;
     float* out = nullptr;
     const float *ys = nullptr, *yd = nullptr;
+    bool give_up = false;   // for testing: as after a wait that gave up
 };
 cudaError_t launch_mlp_fused(const FusedMlp& f, cudaStream_t s);
 

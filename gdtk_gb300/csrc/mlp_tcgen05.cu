@@ -34,7 +34,7 @@ namespace {
 constexpr int TC_M = 128;                           // rows per tile = TMEM lanes
 constexpr int EPI_WARPS = 16;                       // epilogue warps: 4 lane quarters x 4 column slices
 constexpr int TC_THREADS = 32 * (1 + EPI_WARPS);
-constexpr unsigned long long SPIN_LIMIT = 1ull << 22;   // mbarrier polls before a wait gives up
+constexpr unsigned SPIN_LIMIT = 1u << 22;   // mbarrier polls before a wait gives up
 
 __device__ int g_tc_error;
 
@@ -64,7 +64,7 @@ __device__ __forceinline__ void mbar_expect_tx(unsigned long long* bar, unsigned
 // Waits for the phase of parity `parity` to complete; false if it has not after SPIN_LIMIT polls.
 __device__ __forceinline__ bool mbar_wait(unsigned long long* bar, unsigned parity) {
     const unsigned a = smem_u32(bar);
-    for (unsigned long long i = 0; i < SPIN_LIMIT; ++i) {
+    for (unsigned i = 0; i < SPIN_LIMIT; ++i) {
         unsigned done;
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
@@ -364,6 +364,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 // 27 us; 4 x 128: 105 us, 2 x 64: 47 us.  What bounds it is shared memory: a tile's 256 x 256 layer reads 64 KB of
 // activations and 128 KB of weights for the MMAs and writes 128 KB and 64 KB, about 3,100 cycles of its 4,900; its
 // exponentials and reciprocals take 3,100 more, which the other slot's MMAs hide in part.
+//
+// A wait that gives up ends the CTA's work: the error flag is set, the rows that are not done become NaN (the surrogate
+// update sends such cells to the FP64 update), and what is in flight is waited for.  The rows are written out of line: in
+// the kernel's own code they cost the layers 1% (182.2 and 181.2 us).
 struct FusedArgs {
     int M, nlayers;
     int dims[FUSED_MAX_LAYERS + 1];          // nin_pad, width ..., nout_pad (multiples of 8)
@@ -374,6 +378,7 @@ struct FusedArgs {
     const float *X, *xs, *xd;                // raw rows: bf16((X - xs) / xd)
     float* out;                              // [M][nout_pad]: the output, or with ys: output * yd + ys
     const float *ys, *yd;
+    unsigned go;                             // 0, for testing: everything as after waits that gave up
 };
 struct FusedMaps {
     CUtensorMap w[FUSED_MAX_LAYERS];
@@ -429,6 +434,17 @@ __device__ __forceinline__ void store_out(const FusedArgs& g, unsigned row, int 
     o[1] = make_float4(f[4], f[5], f[6], f[7]);
 }
 
+// A warp's rows and columns of the CTA's tiles from number `j` on, every other one
+__device__ __noinline__ void nan_rows(float* out, int M, int nout, int j, int tiles, int r, int half) {
+    const int chunks = pad16(nout) / 16, c1 = 16 * ((half + 1) * chunks / 2);
+    for (; j < tiles; j += 2) {
+        const unsigned row = (blockIdx.x + j * gridDim.x) * TC_M + r;
+        if (row < (unsigned)M)
+            for (int c = 16 * (half * chunks / 2); c < c1 && c < nout; ++c)
+                out[(size_t)row * nout + c] = __int_as_float(0x7fffffff);
+    }
+}
+
 __global__ void __launch_bounds__(FUSED_THREADS, 1)
     mlp_fused_kernel(const __grid_constant__ FusedMaps maps, const __grid_constant__ FusedArgs g) {
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -469,17 +485,16 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
     tc_fence_after();
     const unsigned tmem = *tmem_slot;
     const int ntiles = (g.M - 1) / TC_M + 1;
-    int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
-    if (smem_u32(smem) & 1023u) {   // the swizzle is of shared addresses; the declaration asks for this alignment
-        if (threadIdx.x == 0) atomicExch(&g_tc_error, 6);
-        my_tiles = 0;
-    }
+    const int my_tiles = blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    // the swizzle is of shared addresses; the declaration asks for this alignment
+    const bool go = (smem_u32(smem) & 1023u) == 0 && g.go != 0;
+    if (!go && threadIdx.x == 0) atomicExch(&g_tc_error, 6);
     // tile j of this CTA is in slot j & 1; the layers of a pair of tiles alternate between the slots
 
     if (warp == 0 && lane == 0) {   // MMAs
         int stage = 0, failed = 0;
         unsigned wpar = 0, issued = 0;
-        for (int j0 = 0; j0 < my_tiles && !failed; j0 += 2)
+        for (int j0 = 0; go && j0 < my_tiles && !failed; j0 += 2)
             for (int l = 0; l < g.nlayers && !failed; ++l)
                 for (int s = 0; s < 2 && j0 + s < my_tiles && !failed; ++s) {
                     const unsigned seq = (unsigned)(j0 >> 1) * g.nlayers + l;
@@ -511,7 +526,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
     } else if (warp == 1 && lane == 0) {   // weights
         int stage = 0, failed = 0;
         unsigned par = 1, loads = 0;   // a first wait on the phase before the first passes
-        for (int j0 = 0; j0 < my_tiles && !failed; j0 += 2)
+        for (int j0 = 0; go && j0 < my_tiles && !failed; j0 += 2)
             for (int l = 0; l < g.nlayers && !failed; ++l)
                 for (int s = 0; s < 2 && j0 + s < my_tiles && !failed; ++s)
                     for (int k0 = 0; k0 < pad16(g.dims[l]); k0 += FUSED_KC) {
@@ -521,11 +536,10 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
                         ++loads;
                         if (++stage == g.stages) { stage = 0; par ^= 1; }
                     }
-        if (failed) {
-            atomicExch(&g_tc_error, failed);
-            for (unsigned q = loads > (unsigned)g.stages ? loads - g.stages : 0; q < loads; ++q)   // bounded: loads in flight
-                mbar_wait(&w_full[q % g.stages], (q / g.stages) & 1);
-        }
+        if (failed) atomicExch(&g_tc_error, failed);
+        // bounded: the loads in flight, also where it is the MMAs' thread that gave up
+        for (unsigned q = loads > (unsigned)g.stages ? loads - g.stages : 0; q < loads; ++q)
+            mbar_wait(&w_full[q % g.stages], (q / g.stages) & 1);
     } else if (warp >= 2) {
         const int s = (warp - 2) / FUSED_SLOT_WARPS, half = ((warp - 2) % FUSED_SLOT_WARPS) >> 2;
         const int r = (warp & 3) * 32 + lane;   // the TMEM lanes that a warp may read are those of its number mod 4
@@ -535,7 +549,8 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
         const unsigned trow = tmem + (unsigned)s * g.tmem_cols + ((unsigned)((warp & 3) * 32) << 16);
         const int nin = g.dims[0], nout = g.dims[g.nlayers];
         unsigned seq = 0;
-        bool ok = true;
+        bool ok = go;
+        int undone = ok ? my_tiles : s;   // the slot's first tile that is not done
         for (int j = s; j < my_tiles && ok; j += 2) {
             const unsigned row = (blockIdx.x + j * gridDim.x) * TC_M + r, M = g.M;
             // the input tile: the two warps of a lane quarter take every other K-group
@@ -573,6 +588,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
                 }
                 if (!ok) {
                     if (lane == 0) atomicExch(&g_tc_error, 4);
+                    undone = j;
                     break;
                 }
                 tc_fence_after();
@@ -614,6 +630,7 @@ __global__ void __launch_bounds__(FUSED_THREADS, 1)
                 }
             }
         }
+        if (undone < my_tiles) nan_rows(g.out, g.M, nout, undone, my_tiles, r, half);
     }
     tc_fence_before();
     __syncthreads();
@@ -691,6 +708,10 @@ cudaError_t tcgen05_gemm_error(int* error) {
     return cudaMemcpyToSymbol(g_tc_error, &zero, sizeof(int));
 }
 
+cudaError_t tcgen05_gemm_error_peek(int* error, cudaStream_t s) {
+    return cudaMemcpyFromSymbolAsync(error, g_tc_error, sizeof(int), 0, cudaMemcpyDeviceToHost, s);
+}
+
 bool tcgen05_gemm_eligible(const GemmArgs& g) {
     return !g.trans_a && g.trans_b && g.alpha == 1.f && g.beta == 0.f && g.splits == 1 &&
            (g.act == ACT_NONE || g.act == ACT_GELU) && g.K % 16 == 0 && g.K >= 16 && g.K <= 256 && g.N % 16 == 0 &&
@@ -765,6 +786,7 @@ cudaError_t launch_mlp_fused(const FusedMlp& f, cudaStream_t s) {
     if (a.stages > FUSED_MAX_STAGES) a.stages = FUSED_MAX_STAGES;
     const int smem = a.stages * a.stage_bytes + 2 * a.a_bytes + bar_bytes;
     a.Xh = f.Xh; a.X = f.X; a.xs = f.xs; a.xd = f.xd; a.out = f.out; a.ys = f.ys; a.yd = f.yd;
+    a.go = f.give_up ? 0 : 1;
     cudaError_t e = cudaFuncSetAttribute(mlp_fused_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     const int ntiles = (f.M - 1) / TC_M + 1, sms = sm_count();

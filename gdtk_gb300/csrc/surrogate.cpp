@@ -606,6 +606,18 @@ int chem_surrogate_predict(int sg, int n, const float* X, float* out, void* stre
     });
 }
 
+int chem_surrogate_predict_giving_up(int sg, int n, const float* X, float* out, void* stream) {
+    return guard([&] {
+        auto& S = surr(sg);
+        if (n <= 0) return 0;
+        FusedMlp f;
+        f.X = X; f.xs = S.d_xs.p; f.xd = S.d_xd.p; f.ys = S.d_ys.p; f.yd = S.d_yd.p;
+        f.give_up = true;
+        if (!S.net.fused(f, n, out, (cudaStream_t)stream)) throw std::runtime_error("the network does not run in one kernel");
+        return 0;
+    });
+}
+
 int chem_surrogate_set_gate(int sg, double elem_tol, double neg_tol, double T_tol, double max_dY) {
     return guard([&] {
         auto& S = surr(sg);
@@ -676,9 +688,15 @@ int chem_surrogate_update_cells(int sg, int ncell, const double* rho, const doub
         }
         int hc[2] = {0, 0};
         unsigned long long hcc[GATE_COUNT];
+        int gave_up = 0;
+        ck(tcgen05_gemm_error_peek(&gave_up, s), "D2H");
         ck(cudaMemcpyAsync(hc, cnt, sizeof hc, cudaMemcpyDeviceToHost, s), "D2H");
         ck(cudaMemcpyAsync(hcc, cc, sizeof hcc, cudaMemcpyDeviceToHost, s), "D2H");
         ck(cudaStreamSynchronize(s), "surrogate gate");
+        if (gave_up) {   // the rows are NaN, the gate has sent their cells to the FP64 update
+            ck(tcgen05_gemm_error(&gave_up), "surrogate network");
+            report_error("surrogate network: a launch gave up waiting (code " + std::to_string(gave_up) + "), its rows are NaN");
+        }
         const int n_rej = hc[0];
         int n_fail = 0;
         if (n_rej > 0) {

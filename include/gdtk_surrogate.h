@@ -89,8 +89,11 @@ int chem_surrogate_train_step(int sg, int batch, const float* X, const float* Y,
  * chem_surrogate_get_params), without an update. */
 int chem_surrogate_gradients(int sg, int batch, const float* X, const float* Y, const int* rows, float* grad,
                              float* loss_sum, void* stream);
-/* Raw predicted increments out[n][nout_pad] of raw features X[n][nin_pad]. */
+/* Raw predicted increments out[n][nout_pad] of raw features X[n][nin_pad].  The waits of a network that runs in one
+ * kernel are bounded; where one gives up, the rows that are not done are NaN and gdtk_mlp_tcgen05's error flag is set. */
 int chem_surrogate_predict(int sg, int n, const float* X, float* out, void* stream);
+/* For testing: that kernel as after waits that gave up at once (-1 for a network that does not run in one kernel). */
+int chem_surrogate_predict_giving_up(int sg, int n, const float* X, float* out, void* stream);
 /* Gate tolerances (defaults 1e-4, 1e-5, 1e-3, 5e-4). */
 int chem_surrogate_set_gate(int sg, double elem_tol, double neg_tol, double T_tol, double max_dY);
 /* The surrogate update with FP64 fallback.  Arguments as chem_reactor_update_cells; gate (may be
@@ -100,7 +103,8 @@ int chem_surrogate_set_gate(int sg, double elem_tol, double neg_tol, double T_to
  * is a multiple of monitor_stride with the FP64 update and writes to monitor (host, 4 doubles):
  * cells judged, the largest |dY| of the surrogate against the FP64 update, the largest relative
  * dT, and the mean of the per-cell largest |dY|.  Synchronises the stream (the number of
- * rejected cells is read back to size the fallback). */
+ * rejected cells is read back to size the fallback).  Rows of a network launch that gave up waiting are NaN: their cells
+ * are rejected, and the call says so on stderr and in gdtk_last_error. */
 int chem_surrogate_update_cells(int sg, int ncell, const double* rho, const double* u, double* T, double* p,
                                 double* massf, double* dt_chem, int* status, double t_interval, double T_frozen,
                                 int flags, void* stream, int* gate, long long* counts, int monitor_stride,
@@ -138,7 +142,7 @@ int gdtk_mlp_gemm(int M, int N, int K, const void* A, int lda, int trans_a, cons
  * enable 1 uses them where they apply, 0 uses the mma.sync kernel layer by layer everywhere, -1 leaves the setting (initially off only with GDTK_MLP_TCGEN05=0 in the environment).
  * Returns the previous setting; *launches (if not NULL) receives the tcgen05 launches so far and *error
  * (if not NULL, synchronising) the kernels' error flag, then cleared: 0, or 1 / 2 when a wait for its
- * loads / its MMAs gave up (3 to 5: a wait of the other warps, 6: unaligned shared memory). */
+ * loads / its MMAs gave up (3 to 5: a wait of the other warps, 6: unaligned shared memory, or the launch for testing). */
 int gdtk_mlp_tcgen05(int enable, unsigned long long* launches, int* error);
 
 #ifdef __cplusplus
