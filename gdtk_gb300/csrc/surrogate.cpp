@@ -338,7 +338,9 @@ struct Surrogate {
         // out = standardised prediction * y_scale + y_shift
         FusedMlp f;
         f.X = X; f.xs = d_xs.p; f.xd = d_xd.p; f.ys = d_ys.p; f.yd = d_yd.p;
-        if (net.fused(f, n, out, s)) return;
+        // features that rows of another block may be written over are gathered first
+        const bool over = out < X + (size_t)n * nin_pad && X < out + (size_t)n * nout_pad && !(out == X && nin_pad == nout_pad);
+        if (!over && net.fused(f, n, out, s)) return;
         const int chunk = std::min(n, 1 << 20);
         ensure_infer(chunk);
         for (int first = 0; first < n; first += chunk) {

@@ -89,8 +89,9 @@ int chem_surrogate_train_step(int sg, int batch, const float* X, const float* Y,
  * chem_surrogate_get_params), without an update. */
 int chem_surrogate_gradients(int sg, int batch, const float* X, const float* Y, const int* rows, float* grad,
                              float* loss_sum, void* stream);
-/* Raw predicted increments out[n][nout_pad] of raw features X[n][nin_pad].  The waits of a network that runs in one
- * kernel are bounded; where one gives up, the rows that are not done are NaN and gdtk_mlp_tcgen05's error flag is set. */
+/* Raw predicted increments out[n][nout_pad] of raw features X[n][nin_pad], which out may overlap for n up
+ * to 1,048,576.  The waits of a network that runs in one kernel are bounded; where one gives up, the rows that are not done
+ * are NaN and gdtk_mlp_tcgen05's error flag is set. */
 int chem_surrogate_predict(int sg, int n, const float* X, float* out, void* stream);
 /* For testing: that kernel as after waits that gave up at once (-1 for a network that does not run in one kernel). */
 int chem_surrogate_predict_giving_up(int sg, int n, const float* X, float* out, void* stream);
