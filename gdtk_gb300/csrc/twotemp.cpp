@@ -131,6 +131,7 @@ struct Reactor2TObj {
     Coupling2T* d_cpl = nullptr;
     int neff = 0, n_tab = 0, ncpl = 0;
     unsigned relaxing = 0;
+    bool big = false;   // coefficients beyond 126
     unsigned* d_counter = nullptr;   // work counter of the update's persistent launch
     int sm_count = 0;
     ~Reactor2TObj() {
@@ -229,9 +230,10 @@ extern "C" int chem_reactor2t_new(const char* gas_file, const char* chem_file, c
             for (int side = 0; side < 2; ++side)
                 for (unsigned k = 0; k < co[side] % 8; ++k) {
                     const int idx = x[(side ? RX_PROD_IDX : RX_REAC_IDX) + k], c = x[(side ? RX_PROD_COEFF : RX_REAC_COEFF) + k];
-                    if (c < 0 || c > 127) throw std::runtime_error("stoichiometric coefficient above 127");
                     sp[side] |= (unsigned)idx << (8 * k);
-                    co[side] |= (unsigned)c << (3 + 7 * k);
+                    const bool big = c < 0 || c > 126;
+                    r->big |= big;
+                    co[side] |= (unsigned)(big ? 127 : c) << (3 + 7 * k);
                 }
             tab.insert(tab.end(), {(int)sp[0], (int)sp[1], (int)co[0], (int)co[1], x[RX_COLLIDER] ? x[RX_EFFSET] : -1});
         }
@@ -334,7 +336,7 @@ extern "C" int chem_reactor2t_update_cells(int h, int ncell, const double* rho, 
         a.dt_chem = dt_chem; a.status = status; a.t_interval = t_interval; a.steps = steps;
         a.counter = r.d_counter;
         a.thermo = r.d_thermo; a.eff = r.d_eff; a.tab = r.d_tab; a.cpl = r.d_cpl;
-        a.neff = r.neff; a.n_tab = r.n_tab; a.ncpl = r.ncpl; a.relaxing = r.relaxing;
+        a.neff = r.neff; a.n_tab = r.n_tab; a.ncpl = r.ncpl; a.relaxing = r.relaxing; a.big = r.big;
         ck(launch_two_temperature_update(a, r.nsp, r.nr, r.sm_count, (cudaStream_t)stream), "two-temperature update launch");
         return 0;
     });

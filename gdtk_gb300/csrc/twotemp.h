@@ -57,15 +57,15 @@ struct TwoTArgs {
     const double* thermo;       // thermo table of cea_poly.cuh (fast_thermo_table)
     const double* eff;          // [neff][nsp] third-body efficiencies, 0 where absent
     const int* tab;             // per reaction: reactants, products (8 bits each), the number (3 bits) and coefficients
-                                // (7 bits each) of either, efficiency set or -1; first entry of each species; entries
-                                // (reaction, high word of the net coefficient)
+                                // (7 bits each, 127: see mech_i) of either, efficiency set or -1; first entry of each
+                                // species; entries (reaction, high word of the net coefficient)
     const Coupling2T* cpl;
     int neff, n_tab, ncpl;
     unsigned relaxing;          // species with Landau-Teller mechanisms, as bits
     double tol;     // RKF errTol (atol = rtol)
     int max_subcycles, max_attempts;
     int ncell;
-    int pad;
+    int big;                    // a coefficient of the table is 127
     const double* rho;
     double* T;
     double* Tve;

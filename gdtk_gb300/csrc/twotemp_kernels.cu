@@ -218,6 +218,8 @@ __device__ __forceinline__ double group_sum(double v) {
     return v;
 }
 
+// BIG: with coefficients beyond the reaction table's 126, which are read from the mechanism (the test for them costs 2.7%).
+template <bool BIG>
 __global__ void __launch_bounds__(UPDATE_BLOCK, 3) two_temperature_update_kernel(const TwoTArgs a) {
     extern __shared__ double smem[];
     MechView m;
@@ -275,11 +277,15 @@ __global__ void __launch_bounds__(UPDATE_BLOCK, 3) two_temperature_update_kernel
                 }
                 for (int k = 0; k < (x[2] & 7); ++k) {
                     const double v = y[(x[0] >> (8 * k)) & 255];
-                    for (int n = (x[2] >> (3 + 7 * k)) & 127; n > 0; --n) f *= v;
+                    int n = (x[2] >> (3 + 7 * k)) & 127;
+                    if (BIG && n == 127) n = m.rx(r)[RX_REAC_COEFF + k];
+                    for (; n > 0; --n) f *= v;
                 }
                 for (int k = 0; k < (x[3] & 7); ++k) {
                     const double v = y[(x[1] >> (8 * k)) & 255];
-                    for (int n = (x[3] >> (3 + 7 * k)) & 127; n > 0; --n) b *= v;
+                    int n = (x[3] >> (3 + 7 * k)) & 127;
+                    if (BIG && n == 127) n = m.rx(r)[RX_PROD_COEFF + k];
+                    for (; n > 0; --n) b *= v;
                 }
                 wf[r] = f;
                 wb[r] = b;
@@ -690,7 +696,8 @@ cudaError_t launch_two_temperature_update(const TwoTArgs& a, int nsp, int nr, in
     constexpr size_t LIMIT = 227 * 1024 - 2 * GDTK_EXP2_TABLE_SIZE * 8;
     const size_t tables = (size_t)(nsp * GDTK_TH_STRIDE + a.neff * nsp + (a.n_tab + 1) / 2) * 8;
     const size_t per_warp = (size_t)Layout2T(nsp, nr, a.ncpl).total * (32 / GL) * 8;
-    cudaError_t e = cudaFuncSetAttribute(two_temperature_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT);
+    const auto kernel = a.big ? two_temperature_update_kernel<true> : two_temperature_update_kernel<false>;
+    cudaError_t e = cudaFuncSetAttribute((const void*)kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LIMIT);
     if (e != cudaSuccess) return e;
     if (tables + per_warp > LIMIT) return cudaErrorInvalidConfiguration;
     const long long warps = ((long long)a.ncell + 32 / GL - 1) / (32 / GL);
@@ -700,7 +707,7 @@ cudaError_t launch_two_temperature_update(const TwoTArgs& a, int nsp, int nr, in
     if (fair < per_block) per_block = (int)fair;
     const size_t smem = tables + per_warp * per_block;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, two_temperature_update_kernel, 32 * per_block, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)kernel, 32 * per_block, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) return cudaErrorInvalidConfiguration;
     long long grid = (long long)sm_count * per_sm;
@@ -708,7 +715,7 @@ cudaError_t launch_two_temperature_update(const TwoTArgs& a, int nsp, int nr, in
     if (grid > want) grid = want;
     e = cudaMemsetAsync(a.counter, 0, sizeof(unsigned), s);
     if (e != cudaSuccess) return e;
-    two_temperature_update_kernel<<<(unsigned)grid, 32 * per_block, smem, s>>>(a);
+    kernel<<<(unsigned)grid, 32 * per_block, smem, s>>>(a);
     return cudaGetLastError();
 }
 
