@@ -249,16 +249,19 @@ const char* status_text(int st) {
     }
 }
 
-// Loads the mechanism-specialised kernels; false where they cannot be built (a large mechanism, shared memory).
+// Loads the mechanism-specialised kernels for a call that can do without them: false where they cannot be built, for good
+// where that is the mechanism's (a large one, shared memory), else until the next call (device memory, the cache
+// of compiled kernels).  gdtk_last_error has the reason.
 bool have_fast(ReactorObj& r) {
     if (r.fast) return true;
     if (r.large || r.no_fast) return false;
     try {
         r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
-    } catch (std::exception&) {
-        r.no_fast = true;
+    } catch (std::exception& e) {
+        r.no_fast = dynamic_cast<NoFastKernel*>(&e) != nullptr;
+        report(std::string("the reference-order kernel takes the call: ") + e.what());
     }
-    return !r.no_fast;
+    return r.fast != nullptr;
 }
 
 // Fast-kernel launch of an assembled FastArgs, longest-first unless GDTK_CHEM_INDEX_ORDER.

@@ -287,7 +287,7 @@ std::vector<double> fast_thermo_table(const GasModelHost& gm) {
             th[10 + k] = c.breaks[k] - 0.5 * c.blends[k - 1];
             th[13 + k] = c.breaks[k] + 0.5 * c.blends[k - 1];
             th[16 + k] = 1. / c.blends[k - 1];
-            if (!(th[10 + k] > 0.0)) throw std::runtime_error("thermo curve blend window below 0 K");
+            if (!(th[10 + k] > 0.0)) throw NoFastKernel("thermo curve blend window below 0 K");
         }
         for (int sg = 0; sg < c.nseg; ++sg) {
             const double* a = c.coeffs.data() + 9 * sg;
@@ -605,7 +605,7 @@ std::string group_tables(const GasModelHost& gm, const MechanismHost& mh, const 
 std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh, int block, int min_blocks,
                                  GroupShape* group_shape) {
     if (gm.n_species() > GDTK_MAX_SPECIES || (int)mh.reactions.size() > GDTK_MAX_REACTIONS)
-        throw std::runtime_error("the mechanism-specialised kernel takes up to " + std::to_string(GDTK_MAX_SPECIES) +
+        throw NoFastKernel("the mechanism-specialised kernel takes up to " + std::to_string(GDTK_MAX_SPECIES) +
                                  " species and " + std::to_string(GDTK_MAX_REACTIONS) +
                                  " reactions; larger mechanisms run one warp per cell");
     const int nsp = gm.n_species();
@@ -933,8 +933,9 @@ std::string compile_cubin(const std::string& src, int major, int minor, std::str
     while (!log.empty() && log.back() == '\0') log.pop_back();
     if (rc != NVRTC_SUCCESS) {
         nvrtcDestroyProgram(&prog);
-        throw std::runtime_error(std::string("NVRTC compilation of the mechanism kernel failed: ") +
-                                 nvrtcGetErrorString(rc) + "\n" + log);
+        const std::string why = std::string("NVRTC compilation of the mechanism kernel failed: ") + nvrtcGetErrorString(rc) + "\n" + log;
+        if (rc == NVRTC_ERROR_COMPILATION) throw NoFastKernel(why);
+        throw std::runtime_error(why);
     }
     size_t cn = 0;
     nvrtcGetCUBINSize(prog, &cn);
@@ -980,7 +981,7 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
     };
     int block = 256, min_blocks = 1;
     while (block > 32 && !fits(block, 1)) block -= 32;
-    if (!fits(block, 1)) throw std::runtime_error("mechanism too large for shared memory");
+    if (!fits(block, 1)) throw NoFastKernel("mechanism too large for shared memory");
     if (block <= 128 && fits(block, 2)) min_blocks = 2;
     if (req_block > 0) {   // an explicit launch shape (autotuning)
         if (req_block % 32 || req_block > 1024) throw std::runtime_error("block size must be a multiple of 32, <= 1024");
@@ -1026,14 +1027,14 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
             std::rename(tmp.c_str(), path.c_str());
         }
     }
-    {
-        std::lock_guard<std::mutex> lk(g_jit_mu);
-        g_cubins[key] = cubin;
-    }
     Driver& d = driver();
     CUmodule mod;
     cu_check(d.moduleLoadData(&mod, cubin.data()), "cuModuleLoadData");
     k->module = mod;
+    {   // one that loads
+        std::lock_guard<std::mutex> lk(g_jit_mu);
+        g_cubins[key] = cubin;
+    }
     CUfunction fn;
     cu_check(d.moduleGetFunction(&fn, mod, "gdtk_chem_fast"), "cuModuleGetFunction");
     k->function = fn;
@@ -1051,7 +1052,7 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
     cu_check(d.funcSetAttribute(cfn, CU_FUNC_ATTRIBUTE_MAX_DYNAMIC_SHARED_SIZE_BYTES, (int)smem_max),
              "cuFuncSetAttribute");
     cu_check(d.occupancy(&k->blocks_per_sm, fn, block, smem_max), "cuOccupancyMaxActiveBlocksPerMultiprocessor");
-    if (k->blocks_per_sm < 1) throw std::runtime_error("fast kernel cannot be resident (registers/shared memory)");
+    if (k->blocks_per_sm < 1) throw NoFastKernel("fast kernel cannot be resident (registers/shared memory)");
     if (k->group.cell_doubles) {
         CUfunction gfn;
         cu_check(d.moduleGetFunction(&gfn, mod, "gdtk_chem_group"), "cuModuleGetFunction");

@@ -2,6 +2,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <stdexcept>
 #include <string>
 #include <vector>
 
@@ -68,6 +69,10 @@ struct FastKernel {
     ~FastKernel();
 };
 
+// No mechanism-specialised kernel can be built for the mechanism, whatever the state of the machine.
+struct NoFastKernel : std::runtime_error {
+    using std::runtime_error::runtime_error;
+};
 // Thermo table of chem_fast.cuh (120 doubles per species).
 std::vector<double> fast_thermo_table(const GasModelHost& gm);
 // CUDA source of the generated prologue + kernel for one mechanism.
