@@ -251,16 +251,20 @@ const char* status_text(int st) {
 
 // Loads the mechanism-specialised kernels for a call that can do without them: false where they cannot be built, for good
 // where that is the mechanism's (a large one, shared memory), else until the next call (device memory, the cache
-// of compiled kernels).  gdtk_last_error has the reason.
+// of compiled kernels).  gdtk_last_error has the reason.  Allocating is allowed meanwhile, whatever other streams of
+// the thread or the process are being captured.
 bool have_fast(ReactorObj& r) {
     if (r.fast) return true;
     if (r.large || r.no_fast) return false;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
     try {
         r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
     } catch (std::exception& e) {
         r.no_fast = dynamic_cast<NoFastKernel*>(&e) != nullptr;
         report(std::string("the reference-order kernel takes the call: ") + e.what());
     }
+    check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
     return r.fast != nullptr;
 }
 

@@ -1068,10 +1068,16 @@ FastKernel* build_fast_kernel(const GasModelHost& gm, const MechanismHost& mh, i
     }
     std::vector<double> th = fast_thermo_table(gm);
     static const uint64_t etab[GDTK_EXP2_TABLE_SIZE] = GDTK_EXP2_TABLE_INIT;
-    if (cudaMalloc(&k->d_thermo, th.size() * 8) != cudaSuccess || cudaMalloc(&k->d_exp, sizeof etab) != cudaSuccess)
-        throw std::runtime_error("cudaMalloc failed");
-    cudaMemcpy(k->d_thermo, th.data(), th.size() * 8, cudaMemcpyHostToDevice);
-    cudaMemcpy(k->d_exp, etab, sizeof etab, cudaMemcpyHostToDevice);
+    // on a stream of its own: the default stream may not be used while another stream is captured
+    cudaStream_t copies = nullptr;
+    cudaError_t e = cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking);
+    if (e == cudaSuccess) e = cudaMalloc(&k->d_thermo, th.size() * 8);
+    if (e == cudaSuccess) e = cudaMalloc(&k->d_exp, sizeof etab);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(k->d_thermo, th.data(), th.size() * 8, cudaMemcpyHostToDevice, copies);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(k->d_exp, etab, sizeof etab, cudaMemcpyHostToDevice, copies);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(copies);
+    if (copies) cudaStreamDestroy(copies);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("tables of the mechanism kernel: ") + cudaGetErrorString(e));
     (void)sms;
     return k.release();
 }

@@ -1,6 +1,7 @@
-"""The first use of a mechanism's own kernels by calls that can do without them (source terms, the per-state update)
-when loading them fails for a reason that passes (a damaged file in the cache of compiled kernels stands for one):
-the next call loads them."""
+"""The first use of a mechanism's own kernels by calls that can do without them (source terms, the per-state update):
+while another stream is captured, and when loading them fails for a reason that passes (a damaged file in the cache of
+compiled kernels stands for one), after which the next call loads them."""
+import ctypes
 import os
 import subprocess
 import sys
@@ -24,6 +25,29 @@ def _cells(torch, rc, n=300):
 def _loaded(rc):
     from gdtk_gb300 import lib
     return lib().chem_reactor_update_cells_noalloc(rc.reactor.id, 0, *[None] * 7, 1.0, 0.0, 3, None) == 0   # which needs them loaded
+
+
+def test_source_terms_while_another_stream_is_captured():
+    import torch
+    from gdtk_gb300 import check, lib
+    from gdtk_gb300.cells import ReactorCells
+    rc = ReactorCells(mech("j92-gas.lua"), mech("j92-chem.lua"))
+    rho, T, Y = _cells(torch, rc)
+    out, x = torch.empty_like(Y), torch.zeros(8, device="cuda")
+    other = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    with torch.cuda.graph(graph, capture_error_mode="global"):
+        x += 1.0
+        check(lib().chem_reactor_source_terms_cells(rc.reactor.id, rho.shape[0], vp(rho), vp(T), vp(Y), vp(out), None,
+                                                    ctypes.c_void_p(other.cuda_stream)), "source terms")
+        x += 1.0
+    assert _loaded(rc)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert bool((x == 2.0).all())
+    assert torch.equal(out, rc.source_terms(rho, T, Y))
 
 
 CHILD = """
