@@ -459,9 +459,10 @@ int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, 
         a.counter = r.counter;
         a.cell_counters = cell_counters;
         a.totals = totals;
+        const int width = std::max(r.dev.host.nsp, r.dev.host.nr);
         // Longest cells first, where the cells take turns (6,007 acetylene cells 91 -> 75 ms); not while capturing: the
         // order's buffers would be the graph's, and a later batch may need larger ones.
-        if (!(flags & GDTK_CHEM_INDEX_ORDER) && ncell > chem_warp_resident(ncell, r.mh.method, r.wt, r.warp_doubles, cuda().sm_count)) {
+        if (!(flags & GDTK_CHEM_INDEX_ORDER) && ncell > chem_warp_resident(ncell, width, r.mh.method, r.wt, r.warp_doubles, cuda().sm_count)) {
             cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
             check(cudaStreamIsCapturing(s, &cap), "cudaStreamIsCapturing");
             if (cap == cudaStreamCaptureStatusNone) {
@@ -476,7 +477,7 @@ int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, 
                 a.order = r.order.p;
             }
         }
-        check(launch_chem_update_warp(a, r.mh.method, r.wt, r.warp_doubles, cuda().sm_count, s, &r.last),
+        check(launch_chem_update_warp(a, width, r.mh.method, r.wt, r.warp_doubles, cuda().sm_count, s, &r.last),
               "warp-per-cell update launch");
         return 0;
     }

@@ -1268,10 +1268,17 @@ __global__ void __launch_bounds__(512) chem_warp_kernel(ChemUpdateArgs a, WarpTa
     const int nsp = m.nsp;
     const unsigned ncell = (unsigned)a.ncell;
     const double tI = a.t_interval;
+    // The first cells are dealt over the SMs, so that the longest, which come first, do not share one (2,500 H2-air cells with a
+    // warp each 61 -> 43 ms); the rest come from the counter.
+    const unsigned dealt = gridDim.x * (blockDim.x / (32 * NW));
+    bool first = true;
     while (true) {
-        unsigned c = 0;
-        if (w.lane == 0) c = atomicAdd(a.counter, 1u);
-        c = (unsigned)w.bcast((double)c);
+        unsigned c = cell * gridDim.x + blockIdx.x;
+        if (!first) {
+            if (w.lane == 0) c = dealt + atomicAdd(a.counter, 1u);
+            c = (unsigned)w.bcast((double)c);
+        }
+        first = false;
         if (c >= ncell) break;
         if (!COST && a.order) c = (unsigned)a.order[c];
         const double rho = a.rho[c], u = a.u[c], T0 = a.T[c], p0 = a.p[c];
@@ -1501,12 +1508,15 @@ struct WarpShape {
 // turns of the cells that an SM then holds; beyond that as many as leave an SM the cells that shared memory holds.
 // Acetylene cells over 1e-6 s with one / two / four warps, in ms: 400 44.5 / 29.1 / 18.3, 1,000 49.4 / 32.7 / 23.2, 2,500
 // 56.2 / 42.7 / 37.8, 6,007 90.2 / 75.1 / 83.9; 20,000 over 1e-7 s 140 / 122 / 136.  The cost keys take one warp.
-cudaError_t warp_shape(int ncell, int method, bool cost, const WarpTables* tabs, int warp_doubles, int sm_count,
+// A small mechanism, which takes this kernel by a flag, leaves lanes of more warps idle: one up to 16 reactions and species,
+// two up to 32.  Park's air, 5 reactions, with one / two / four over 2e-7 s: 300 cells 2.0 / 2.0 / 2.2, 2,500 4.3 / 5.8 /
+// 9.4; Stanford's H2-air, 28, over 1e-7 s: 300 9.3 / 8.4 / 8.8, 2,500 13.0 / 12.2 / 14.8; 33: 20.3 with four, 22.8 with one.
+cudaError_t warp_shape(int ncell, int width, int method, bool cost, const WarpTables* tabs, int warp_doubles, int sm_count,
                        WarpShape& w) {
     const size_t limit = 227 * 1024, per_cell = (size_t)warp_doubles * 8;
     const int share = (ncell + sm_count - 1) / sm_count;   // cells for an SM
     w.v = -1;
-    for (int k = cost ? 0 : 2; k >= 0; --k) {
+    for (int k = cost || width <= 16 ? 0 : width <= 32 ? 1 : 2; k >= 0; --k) {
         const int nw = 1 << k;
         const size_t tables = (size_t)tabs[k].n_smem_ints * 4;
         if (tables + per_cell > limit) continue;
@@ -1539,24 +1549,24 @@ cudaError_t launch_warp(const ChemUpdateArgs& a, const WarpShape& w, const WarpT
 }
 }  // namespace
 
-int chem_warp_resident(int ncell, int method, const WarpTables* tabs, int warp_doubles, int sm_count) {
+int chem_warp_resident(int ncell, int width, int method, const WarpTables* tabs, int warp_doubles, int sm_count) {
     WarpShape w;
-    if (ncell <= 0 || warp_shape(ncell, method, false, tabs, warp_doubles, sm_count, w) != cudaSuccess) return 0;
+    if (ncell <= 0 || warp_shape(ncell, width, method, false, tabs, warp_doubles, sm_count, w) != cudaSuccess) return 0;
     return sm_count * w.per_sm * w.cells;
 }
 
 cudaError_t launch_chem_warp_cost(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
                                   int sm_count, float* key, cudaStream_t stream) {
     WarpShape w;
-    const cudaError_t e = warp_shape(a.ncell, method, true, tabs, warp_doubles, sm_count, w);
+    const cudaError_t e = warp_shape(a.ncell, 0, method, true, tabs, warp_doubles, sm_count, w);
     return e == cudaSuccess ? launch_warp(a, w, tabs, warp_doubles, sm_count, key, stream, nullptr) : e;
 }
 
-cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
+cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int width, int method, const WarpTables* tabs, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info) {
     if (a.ncell <= 0) return cudaSuccess;
     WarpShape w;
-    const cudaError_t e = warp_shape(a.ncell, method, false, tabs, warp_doubles, sm_count, w);
+    const cudaError_t e = warp_shape(a.ncell, width, method, false, tabs, warp_doubles, sm_count, w);
     return e == cudaSuccess ? launch_warp(a, w, tabs, warp_doubles, sm_count, nullptr, stream, info) : e;
 }
 

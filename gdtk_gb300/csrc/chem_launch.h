@@ -87,12 +87,13 @@ constexpr int RX_LONG = 1 << 30;
 constexpr int WARP_VARIANTS = 3;   // 1, 2, 4 warps per cell
 // Shared-memory doubles of one cell's vectors.
 int chem_warp_doubles(int nsp, int nr, int neff, int method, int npart);
-// Cells that are resident at once in a batch of ncell (0: the mechanism does not fit).
-int chem_warp_resident(int ncell, int method, const WarpTables* tabs, int warp_doubles, int sm_count);
+// Cells that are resident at once in a batch of ncell (0: the mechanism does not fit).  width: the larger of the mechanism's
+// numbers of species and reactions.
+int chem_warp_resident(int ncell, int width, int method, const WarpTables* tabs, int warp_doubles, int sm_count);
 // A cost key of each cell, for launch_bucket_order: about proportional to its steps.
 cudaError_t launch_chem_warp_cost(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
                                   int sm_count, float* key, cudaStream_t stream);
-cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int method, const WarpTables* tabs, int warp_doubles,
+cudaError_t launch_chem_update_warp(const ChemUpdateArgs& a, int width, int method, const WarpTables* tabs, int warp_doubles,
                                     int sm_count, cudaStream_t stream, LaunchInfo* info);
 // Cost buckets of the longest-first ordering: launch_bucket_order's hist scratch holds this many ints.
 constexpr int ORDER_BUCKETS = 256;
