@@ -54,6 +54,11 @@ __device__ __forceinline__ bool ge_nn(double a, double b) {
 __device__ __forceinline__ bool nonzero(double x) { return (dbits(x) & ABS_BITS) != 0; }
 // |x| as a double with the sign bit cleared (an integer operation)
 __device__ __forceinline__ double abs_bits(double x) { return __longlong_as_double(dbits(x) & ABS_BITS); }
+// fmax(|a|, |b|), any a, b
+__device__ __forceinline__ double larger_abs(double a, double b) {
+    const double x = abs_bits(a), y = abs_bits(b);
+    return (dbits(y) > dbits(x) && dbits(y) <= INF_BITS) || dbits(x) > INF_BITS ? y : x;
+}
 // ---------------------------------------------------------------- species thermo
 // Segment choice of cea_thermo_curves.d:150-182: coefficients sa blended towards sb by wb.
 // th[10] holds the segment count as integer bits; th[10 + i] and th[13 + i] the blend window

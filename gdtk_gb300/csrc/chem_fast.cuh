@@ -415,13 +415,16 @@ __device__ __forceinline__ void rkf_result(double K1, double K3, double K4, doub
                  b43 = 18575. / 48384., b44 = 13525. / 55296., b45 = 277. / 14336., b46 = 1.0 / 4.0;
     o = fma(h, fma(b56, K6, fma(b54, K4, fma(b53, K3, b51 * K1))), y0);
     const double o4 = fma(h, fma(b46, K6, fma(b45, K5, fma(b44, K4, fma(b43, K3, b41 * K1)))), y0);
-    e = gdtk_div(o - o4, fma(GDTK_ERRTOL, fmax(fabs(y0), fabs(o)), GDTK_ERRTOL));
+    e = gdtk_div(o - o4, fma(GDTK_ERRTOL, larger_abs(y0, o), GDTK_ERRTOL));
 }
-// the step-size factor of the scaled error norm; ok: the step is accepted
-__device__ __forceinline__ double rkf_scale(double errn, const uint64_t* etab, bool& ok) {
-    ok = errn <= 1.0;
-    if (ok) return (errn == 0.0) ? 10.0 : fmin(fmax(0.9 * gdtk_exp(-0.2 * gdtk_log(errn), etab), 0.2), 10.0);
-    return fmax(0.9 * gdtk_exp(-0.2 * gdtk_log(errn), etab), 0.2);
+// the step-size factor of the scaled error norm, from its square en2 (>= 0 or NaN): 0.9 norm^-0.2, at least 0.2, at most
+// 10 for an accepted step; ok: it is (the norm is at most 1, as is the rounded root of 1 + 2^-52).  Square root, minimum and
+// maximum would cost the FP64 pipe about 15 of a step's 590 instructions.
+__device__ __forceinline__ double rkf_scale(double en2, const uint64_t* etab, bool& ok) {
+    ok = (unsigned long long)dbits(en2) <= (unsigned long long)dbits(1.0) + 1;
+    if (!nonzero(en2)) return 10.0;
+    const double s = 0.9 * gdtk_exp(-0.1 * gdtk_log(en2), etab), t = gt_pos(s, 0.2) ? s : 0.2;
+    return ok ? min_pos(t, 10.0) : t;
 }
 #endif
 // GDTK_VEC (per-thread method vector, doubles) comes from the generator: the method's stage
@@ -543,7 +546,7 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
 #if GDTK_METHOD == 0
         // Runge-Kutta-Fehlberg with Cash-Karp coefficients, chemistry_update.d:404-478.
         // V holds k_1..k_6; all six right-hand sides share one call site.
-        double errn = 0.0;
+        double en2 = 0.0;
 #pragma unroll 1
         for (int s = 0; s < 6; ++s) {
             double q[GDTK_NSP], L[GDTK_NSP];
@@ -581,16 +584,16 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
                     yn[i] = fma(h, acc, y0[i]);
                 }
             } else {
-                errn = sqrt(sum_pairwise([&](int i) {
+                en2 = sum_pairwise([&](int i) {
                     double o, e;
                     rkf_result(V[i * ks], V[(2 * GDTK_NSP + i) * ks], V[(3 * GDTK_NSP + i) * ks], V[(4 * GDTK_NSP + i) * ks],
                                V[(5 * GDTK_NSP + i) * ks], h, y0[i], o, e);
                     yn[i] = o;
                     return __dmul_rn(e, e);
-                }) * (1.0 / GDTK_NSP));
+                }) * (1.0 / GDTK_NSP);
             }
         }
-        dtS = rkf_scale(errn, ETAB, ok) * h;
+        dtS = rkf_scale(en2, ETAB, ok) * h;
 #else
         // alpha-QSS, chemistry_update.d:533-655.  Iteration 0 is the predictor, 1..maxIters the
         // correctors; with q0 = q and p0 = p the corrector formula reduces to the predictor's, so

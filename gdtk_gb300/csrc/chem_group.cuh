@@ -291,13 +291,35 @@ __device__ __forceinline__ double grp_gather(const unsigned* ent, int e0, int e1
 }
 #endif
 
-// Lanes to a third-body sum: the L / G sums of a turn share its instructions, a sum's tree (grp_sum's) takes
-// 2 P2 / G - 1 of them in a lane and log2 G over its lanes.  The G of the fewest FP64 instructions; 3 sets of Park's 5
+// A third-body sum by G lanes (gl: the lane among them), in every lane: pairs of species with the second product fused, then
+// grp_sum's tree.  With one species to a lane both lanes of a pair form it.
+template <int G>
+__device__ __forceinline__ double third_body_sum(int gl, const double* ef, const double* c) {
+    constexpr int W = G < GRP_P2 ? G : GRP_P2, KC = GRP_P2 / W, KP = KC < 2 ? 1 : KC / 2;
+    const int base = (gl & (W - 1)) * KC & ~1;
+    double v[KP];
+#pragma unroll
+    for (int k = 0; k < KP; ++k) {
+        const int i = base + 2 * k;
+        v[k] = i < GDTK_NSP ? third_body(ef[i], c[i]) : 0.0;
+        if (i + 1 < GDTK_NSP) v[k] = fma(ef[i + 1], c[i + 1], v[k]);
+    }
+#pragma unroll
+    for (int w = 1; w < KP; w <<= 1)
+#pragma unroll
+        for (int k = 0; k < KP; k += 2 * w) v[k] += v[k + w];
+#pragma unroll
+    for (int x = KC < 2 ? 2 : 1; x < W; x <<= 1) v[0] += __shfl_xor_sync(GRP_FULL, v[0], x);
+    return v[0];
+}
+
+// Lanes to a third-body sum: the L / G sums of a turn share its instructions, of which a sum takes P2 / G for its pairs,
+// P2 / 2 G - 1 for its tree in a lane and log2 G over its lanes.  The G of the fewest FP64 instructions; 3 sets of Park's 5
 // species with 32 lanes: 4 instructions where one sum after the other took 12 (4,096 cells 2.40 -> 2.04 ms).
 constexpr int set_cost(int L, int G) {
     int lg = 0;
     for (int x = 1; x < G; x <<= 1) ++lg;
-    return (GDTK_NSETS + L / G - 1) / (L / G) * (2 * (GRP_P2 / G) - 1 + lg);
+    return (GDTK_NSETS + L / G - 1) / (L / G) * (GRP_P2 / G < 2 ? 1 + lg : GRP_P2 / G + GRP_P2 / (2 * G) - 1 + lg);
 }
 constexpr int set_lanes(int L) {
     int best = L < GRP_P2 ? L : GRP_P2;
@@ -315,26 +337,15 @@ __device__ __forceinline__ void grp_rhs(const GrpTab& tab, const GrpCell& s, con
 #pragma unroll 1
         for (int m = 0; m < GDTK_NSETS; ++m) {
             const double* ef = tab.eff + m * GDTK_NSP;
-            const double M = grp_sum<L>(gl, [&](int i) { return third_body(ef[i], c[i]); });
+            const double M = third_body_sum<L>(gl, ef, c);
             if (act && gl == 0) S[GO_M + m] = M;
         }
     } else {
-        constexpr int KC = GRP_P2 / G;
-        const int base = (gl & (G - 1)) * KC;
 #pragma unroll 1
         for (int m0 = 0; m0 < GDTK_NSETS; m0 += L / G) {
             const int m = m0 + gl / G;
-            const double* ef = tab.eff + (m < GDTK_NSETS ? m : 0) * GDTK_NSP;
-            double v[KC];
-#pragma unroll
-            for (int k = 0; k < KC; ++k) v[k] = base + k < GDTK_NSP ? third_body(ef[base + k], c[base + k]) : 0.0;
-#pragma unroll
-            for (int w = 1; w < KC; w <<= 1)
-#pragma unroll
-                for (int k = 0; k < KC; k += 2 * w) v[k] += v[k + w];
-#pragma unroll
-            for (int x = 1; x < G; x <<= 1) v[0] += __shfl_xor_sync(GRP_FULL, v[0], x);
-            if (act && m < GDTK_NSETS && !(gl & (G - 1))) S[GO_M + m] = v[0];
+            const double M = third_body_sum<G>(gl & (G - 1), tab.eff + (m < GDTK_NSETS ? m : 0) * GDTK_NSP, c);
+            if (act && m < GDTK_NSETS && !(gl & (G - 1))) S[GO_M + m] = M;
         }
     }
     __syncwarp(GRP_FULL);
@@ -606,7 +617,6 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
             }
         };
 #if GDTK_METHOD == 0
-        double errn = 0.0;
 #pragma unroll 1
         for (int st = 0; st < 6; ++st) {
             grp_rhs<L>(tab, s, st == 0 ? Y0 : C, gl, act);
@@ -634,8 +644,7 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
         }
         {
             const double err2 = grp_sum<L>(gl, [&](int i) { return W[i]; });
-            errn = sqrt(err2 * (1.0 / GDTK_NSP));
-            if (act) s.dtS = rkf_scale(errn, tab.ETAB, ok) * s.h;
+            if (act) s.dtS = rkf_scale(err2 * (1.0 / GDTK_NSP), tab.ETAB, ok) * s.h;
         }
 #else
         {

@@ -324,12 +324,17 @@ int rhs_fence() {
     return (e && *e) ? std::max(0, std::atoi(e)) : 4;
 }
 
-// A sum over the species as the zero-padded pairwise tree of chem_fast.cuh's sum_pairwise.
-std::string tree_sum(const std::vector<std::string>& leaf, int lo, int n) {
-    if (n == 1) return leaf[lo];
-    const std::string a = tree_sum(leaf, lo, n / 2);
+// A third-body sum over the species (leaf: the efficiency, 0 where absent) as chem_group.cuh's third_body_sum: pairs with the
+// second product fused, then the zero-padded pairwise tree of chem_fast.cuh's sum_pairwise.
+std::string third_body_sum(const std::vector<double>& leaf, int lo, int n) {
+    auto c = [](int i) { return "c[" + std::to_string(i) + "]"; };
+    auto product = [&](int i) { return leaf[i] == 0.0 ? std::string() : leaf[i] == 1.0 ? c(i) : "__dmul_rn(" + lit(leaf[i]) + ", " + c(i) + ")"; };
+    if (n == 1) return product(lo);
+    if (n == 2 && lo + 1 < (int)leaf.size() && leaf[lo] != 0.0 && leaf[lo + 1] != 0.0 && leaf[lo + 1] != 1.0)
+        return "fma(" + lit(leaf[lo + 1]) + ", " + c(lo + 1) + ", " + product(lo) + ")";
+    const std::string a = third_body_sum(leaf, lo, n / 2);
     std::string b;
-    if (lo + n / 2 < (int)leaf.size()) b = tree_sum(leaf, lo + n / 2, n / 2);
+    if (lo + n / 2 < (int)leaf.size()) b = third_body_sum(leaf, lo + n / 2, n / 2);
     if (a.empty() || b.empty()) return a.empty() ? b : a;
     return "(" + a + " + " + b + ")";
 }
@@ -841,14 +846,11 @@ std::string generate_fast_source(const GasModelHost& gm, const MechanismHost& mh
         set_of[ir] = f;
     }
     for (size_t s = 0; s < sets.size(); ++s) {
-        std::vector<std::string> leaf(nsp);
-        for (auto& e : sets[s]) {
-            const std::string cc = "c[" + std::to_string(e.first) + "]";
-            leaf[e.first] = e.second == 1.0 ? cc : "__dmul_rn(" + lit(e.second) + ", " + cc + ")";
-        }
+        std::vector<double> leaf(nsp, 0.0);
+        for (auto& e : sets[s]) leaf[e.first] = e.second;
         int p2 = 1;
         while (p2 < nsp) p2 *= 2;
-        const std::string sum = tree_sum(leaf, 0, p2);
+        const std::string sum = third_body_sum(leaf, 0, p2);
         o << "  const double M" << s << " = " << (sum.empty() ? "0.0" : sum) << ";\n";
     }
     std::vector<bool> qset(nsp, false), lset(nsp, false);

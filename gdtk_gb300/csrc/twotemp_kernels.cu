@@ -191,13 +191,8 @@ __constant__ double CK_A[5][5] = {
 using gdtk_fast::abs_bits;
 using gdtk_fast::ge_pos;
 using gdtk_fast::gt_pos;
+using gdtk_fast::larger_abs;
 using gdtk_fast::lt_pos;
-// fmax(|a|, |b|), on the integer pipe
-__device__ __forceinline__ double larger_abs(double a, double b) {
-    const double x = abs_bits(a), y = abs_bits(b);
-    using namespace gdtk_fast;
-    return (dbits(y) > dbits(x) && dbits(y) <= INF_BITS) || dbits(x) > INF_BITS ? y : x;
-}
 
 // offsets of a cell's vectors in its slice, in doubles
 struct Layout2T {
