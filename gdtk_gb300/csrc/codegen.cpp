@@ -1109,12 +1109,13 @@ cudaError_t launch_fast(FastKernel& k, FastArgs& a, int sm_count, cudaStream_t s
 // exceed `turns`: measured where two choices cross.  H2-air (13 species; ms with 4 / 8 / 16 / 32 lanes): 1,000 cells
 // 36 / 31 / 29 / 29, 12,000 63 / 52 / 48 / 54, 48,000 108 / 96 / 109 / 179, 262,147 364 / 437 / 575 / 975.  The
 // Runge-Kutta mechanisms are smaller (5 species) and their cells' step counts alike, so that no long tail
-// pays for lanes: 1,000 air cells 2.6 / 1.9 / 1.7 / 1.8, 4,000 2.9 / 2.3 / 2.7 / 3.6, 12,000 3.5 / 4.3 / 5.8 / 9.6;
-// one thread per cell takes 4.2 there and 5.3 at 32,768, where 4 lanes take 8.3.
+// pays for lanes: 1,000 air cells 2.6 / 1.9 / 1.7 / 1.8, 4,000 2.9 / 2.3 / 2.7 / 3.6, 12,000 3.5 / 4.3 / 5.8 / 9.6.
+// Against one thread per cell 4 lanes lie ahead for one turn, 19,456 cells: over 2e-7 s 2.9 and 4.1 at 12,000, 3.8 and 4.1 at
+// 16,384, 3.9 and 4.0 at 19,000 (Gupta's air 11.6 and 12.5), 8.3 and 4.3 at 32,768.
 int group_lanes(const FastKernel& k, long long total, int sm_count) {
     if (!k.group_function) return 0;
     const bool rkf = k.method == METHOD_RKF;
-    const double turns[4] = {rkf ? 0.78 : 1e30, rkf ? 0.65 : 7.0, rkf ? 0.44 : 6.5, rkf ? 0.3 : 1.6};
+    const double turns[4] = {rkf ? 1.0 : 1e30, rkf ? 0.65 : 7.0, rkf ? 0.44 : 6.5, rkf ? 0.3 : 1.6};
     for (int lv = 3; lv >= 0; --lv) {
         const double resident = (double)sm_count * k.group_warps[lv] * (8 >> lv);
         if ((double)total <= turns[lv] * resident) return 4 << lv;
