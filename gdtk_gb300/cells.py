@@ -149,8 +149,8 @@ class ReactorCells:
         return F[0] * kc + F[1] * rhs + F[2] * steps + F[3] * corr + F[4] * newton
 
     def set_lane_stats(self, stats):
-        """Diagnostics (chem_reactor_set_lane_stats): a cuda int64 tensor of 24 slots that later fast-kernel
-        launches add to -- per phase k, warp executions [2k], active lanes [2k + 1], and with a kernel
+        """Diagnostics (chem_reactor_set_lane_stats) of the one-thread-per-cell kernel, which updates run while
+        they are on: a cuda int64 tensor of 24 slots that later launches add to -- per phase k, warp executions [2k], active lanes [2k + 1], and with a kernel
         generated under GDTK_PHASE_CLOCKS=1 the SM cycles [16 + k].  None turns it off."""
         if stats is not None:
             import torch

@@ -285,6 +285,7 @@ void run_fast(ReactorObj& r, FastArgs& a, int flags, cudaStream_t s) {
     if (lanes) {
         check(launch_group(*r.fast, a, lanes, cuda().sm_count, s, &r.last.grid, &r.last.block, &r.last.smem),
               "chemistry update launch");
+        r.last.blocks_per_sm = 1;
         return;
     }
     check(launch_fast(*r.fast, a, cuda().sm_count, s, &r.last.grid, &r.last.block, &r.last.smem),
@@ -513,7 +514,6 @@ int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, 
     b.t_interval = t_interval;
     b.rho = rho; b.u = u; b.T = T; b.p = p; b.massf = massf; b.dt_chem = dt_chem; b.status = status;
     run_fast(r, a, flags, s);
-    r.last.blocks_per_sm = r.fast->blocks_per_sm;
     return 0;
 }
 

@@ -45,7 +45,8 @@ enum gdtk_cell_status {
 #define GDTK_CHEM_REFERENCE_ORDER 4 /* use the kernel that keeps the reference's operation order
                                        (default: the mechanism-specialised kernels, which rearrange
                                        the arithmetic to spend fewer FP64 operations: a group of lanes
-                                       per cell or one thread per cell, by the batch's size) */
+                                       per cell or one thread per cell, by the batch's size, which
+                                       changes no result) */
 #define GDTK_CHEM_WARP_PER_CELL 16  /* use the warp-per-cell kernel: the reference's update with species
                                        and reactions spread over the lanes of one, two or four warps.  It is
                                        taken without the flag for mechanisms of more than 32 species or
@@ -216,15 +217,19 @@ int gdtk_compile_fast_source_check(const char* gas_file, const char* chem_file, 
 /* Launch shape of the reactor's mechanism-specialised kernel of one thread per cell: threads per block
  * (a multiple of 32) and resident blocks per SM it is compiled for (its register/shared-memory split);
  * later updates run that kernel.  0, 0 restores the default: a group of lanes per cell or one thread
- * (largest block that shared memory allows), by the batch's size.  Compiles and loads the
+ * (largest block that shared memory allows), by the batch's size.  For alpha-QSS mechanisms the two kernels'
+ * results agree to rounding (the q and L sums of a group are rounded once); for Runge-Kutta ones, and among the
+ * numbers of lanes, they are the same bits.  Compiles and loads the
  * variant now.  Used by the autotuner (gdtk_gb300/autotune.py). */
 int chem_reactor_configure(int cr_i, int block, int min_blocks);
 /* Work-queue refill of the mechanism-specialised kernel: with cells = 0 or 1 a warp takes, with one
  * atomic, exactly as many visit positions as it has lanes without a cell; with cells in 32..2^20 it
  * reserves that many consecutive positions per atomic and hands them out to its own lanes before
- * taking another chunk.  Only scheduling changes, never a cell's result.  Autotuner dimension. */
+ * taking another chunk.  Only scheduling changes, never a cell's result.  Autotuner dimension.  The kernel of one
+ * thread per cell alone has it: updates that take a group of lanes per cell run as without. */
 int chem_reactor_set_refill_chunk(int cr_i, int cells);
-/* Diagnostics: when stats (device, unsigned long long[24]) is set, later fast-kernel launches
+/* Diagnostics of the kernel of one thread per cell, which updates run while stats is set, also where they would take a
+ * group of lanes per cell: when stats (device, unsigned long long[24]) is set, later launches
  * add, for each phase k (0 iteration, 1 rate constants, 2 right-hand side, 3 step control,
  * 4 Newton iteration, 5 cell completion, 6 refill, 7 the alpha-QSS update after a right-hand
  * side), the number of warp executions in stats[2k] and of active lanes in them in stats[2k+1].
