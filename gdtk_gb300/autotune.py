@@ -8,7 +8,7 @@ integrates at once (32, one per thread; or 1, with species and reactions over th
 tuner times a sample of the caller's own cells under
   (threads per block, blocks per SM) x (longest-first | index order), (0, 0) standing for the
   library's own choice (a group of lanes per cell or one thread per cell, by the batch's size),
-  then refill chunks on the best of those, then one warp per cell,
+  then refill chunks on the best of those (if it is a shape: only one thread per cell has them), then one warp per cell,
 keeps the fastest, and records the choice in a versioned JSON file keyed by mechanism, device
 and workload tag, so later runs reuse it without timing.
 """
@@ -19,7 +19,7 @@ import time
 
 from . import lib, check
 
-CACHE_VERSION = 3
+CACHE_VERSION = 4
 SHAPES = [(0, 0), (256, 1), (224, 1), (192, 1), (160, 1), (128, 1), (128, 2), (96, 2), (64, 2), (64, 3)]
 ORDERS = {"longest-first": 0, "index": 8}
 CHUNKS = [128, 1024]          # refill chunks tried on the best shape (0: exactly the lanes that need a cell)
@@ -116,7 +116,7 @@ def tune(rc, sample, t_interval, tag="default", repeats=1, use_cache=True, flags
         if results:
             best = min(results, key=lambda r: r["ms"])
             check_shape(rc, best["block"], best["min_blocks"])
-            for cells in CHUNKS:
+            for cells in CHUNKS if best["block"] else []:   # the library's own choice is mostly a kernel without chunks
                 set_refill_chunk(rc, cells)
                 ms = _time(rc, sample, t_interval, flags | ORDERS[best["order"]], repeats)
                 results.append(dict(best, refill_chunk=cells, ms=ms))

@@ -64,3 +64,17 @@ def test_refill_chunk_changes_no_result(shaped, chunk):
     assert last["grid"] * last["block"] < n and int((outs[0][-1] == 0).sum()) > 0.95 * n
     for a, b in zip(*outs):
         assert torch.equal(a, b)
+
+
+def test_autotuner_times_no_refill_chunk_of_the_librarys_choice(tmp_path, monkeypatch):
+    from gdtk_gb300 import autotune
+    torch = torch_cuda()
+    monkeypatch.setenv("GDTK_JIT_CACHE", str(tmp_path))
+    monkeypatch.setattr(autotune, "SHAPES", [(0, 0)])
+    rc, _ = pair("park5")
+    T, p, Y = _cells("park5", rc, 512, seed=7)
+    dT, dp, dY = to_dev(torch, T, p, Y)
+    rho, u = rc.thermo_from_pT(dp, dT, dY)
+    sample = dict(rho=rho, u=u, T=dT, p=dp, massf=dY, dt_chem=torch.full((512,), -1.0, dtype=torch.float64, device="cuda"))
+    _, _, results = autotune.tune(rc, sample, 1.0e-7, tag="test", allow_warp=False)
+    assert [(r["order"], r["refill_chunk"]) for r in results] == [(name, 0) for name in autotune.ORDERS]
