@@ -143,6 +143,7 @@ struct ReactorObj {
     LaunchInfo last{};
     std::unique_ptr<FastKernel> fast;   // mechanism-specialised kernel, compiled on first use
     bool no_fast = false;               // they cannot be built for this mechanism
+    std::mutex fast_mu;                 // of these two: source terms may be asked for by several threads
     int req_block = 0, req_min_blocks = 0;   // launch shape chosen by chem_reactor_configure
     int refill_chunk = 0;                    // chem_reactor_set_refill_chunk
     unsigned long long* lane_stats = nullptr;   // when set, the fast kernel counts lane occupancy
@@ -254,6 +255,7 @@ const char* status_text(int st) {
 // of compiled kernels).  gdtk_last_error has the reason.  Allocating is allowed meanwhile, whatever other streams of
 // the thread or the process are being captured.
 bool have_fast(ReactorObj& r) {
+    std::lock_guard<std::mutex> lk(r.fast_mu);
     if (r.fast) return true;
     if (r.large || r.no_fast) return false;
     cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
@@ -265,6 +267,17 @@ bool have_fast(ReactorObj& r) {
         report(std::string("the reference-order kernel takes the call: ") + e.what());
     }
     check(cudaThreadExchangeStreamCaptureMode(&mode), "cudaThreadExchangeStreamCaptureMode");
+    return r.fast != nullptr;
+}
+
+// The same for a call that cannot.
+void load_fast(ReactorObj& r) {
+    std::lock_guard<std::mutex> lk(r.fast_mu);
+    if (!r.fast) r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
+}
+
+bool fast_loaded(ReactorObj& r) {
+    std::lock_guard<std::mutex> lk(r.fast_mu);
     return r.fast != nullptr;
 }
 
@@ -499,7 +512,7 @@ int launch_update(ReactorObj& r, int ncell, const double* rho, const double* u, 
         check(launch_chem_update(a, r.mh.method, r.scratch, cuda().sm_count, s, &r.last), "chemistry update launch");
         return 0;
     }
-    if (!r.fast) r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
+    load_fast(r);
     FastArgs a{};
     a.nblocks = 1;
     a.total = ncell;
@@ -549,7 +562,7 @@ int update_cells_with_scratch(int cr_i, int ncell, const double* rho, const doub
     return guarded([&] {
         auto& r = reactor(cr_i);
         if (!cuda().ok) throw std::runtime_error(cuda().why);
-        if (!r.fast)
+        if (!fast_loaded(r))
             throw std::runtime_error("chem_reactor_update_cells_noalloc: the reactor's mechanism kernel is not loaded "
                                      "yet; one chem_reactor_update_cells call on this reactor (which may allocate) "
                                      "loads it");
@@ -1030,7 +1043,7 @@ int chem_reactor_update_blocks(int cr_i, int nblock, const gdtk_cell_block* bloc
             }
             return 0;
         }
-        if (!r.fast) r.fast.reset(build_fast_kernel(model(r.gm).gm, r.mh, r.req_block, r.req_min_blocks));
+        load_fast(r);
         if (!r.counter) check(cudaMalloc(&r.counter, sizeof(unsigned)), "cudaMalloc");
         long long done_cells = 0;
         for (int b0 = 0; b0 < nblock; b0 += FAST_MAX_BLOCKS) {   // one launch per 128 blocks
@@ -1114,7 +1127,7 @@ int chem_reactor_source_terms_cells(int cr_i, int ncell, const double* rho, cons
         // the mechanism-specialised kernel (600,011 H2-air cells in 1.6 ms, where the reference-order service takes
         // 15.1); a large mechanism has none, and a capture cannot load one
         cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-        if (!r.large && !r.fast) check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
+        if (!r.large && !fast_loaded(r)) check(cudaStreamIsCapturing(s, &capturing), "cudaStreamIsCapturing");
         if (capturing == cudaStreamCaptureStatusNone && have_fast(r)) {
             check(launch_source(*r.fast, ncell, rho, T, massf, source, status, cuda().sm_count, s), "source terms launch");
             return 0;
@@ -1186,6 +1199,7 @@ int chem_reactor_configure(int cr_i, int block, int min_blocks) {
         auto& r = reactor(cr_i);
         require_cuda();
         std::unique_ptr<FastKernel> k(build_fast_kernel(model(r.gm).gm, r.mh, block, min_blocks));
+        std::lock_guard<std::mutex> lk(r.fast_mu);
         r.req_block = block;
         r.req_min_blocks = min_blocks;
         r.fast = std::move(k);

@@ -1,5 +1,5 @@
 """The first use of a mechanism's own kernels by calls that can do without them (source terms, the per-state update):
-while another stream is captured, and when loading them fails for a reason that passes (a damaged file in the cache of
+while another stream is captured, by several threads at once, and when loading them fails for a reason that passes (a damaged file in the cache of
 compiled kernels stands for one), after which the next call loads them."""
 import ctypes
 import os
@@ -48,6 +48,37 @@ def test_source_terms_while_another_stream_is_captured():
     torch.cuda.synchronize()
     assert bool((x == 2.0).all())
     assert torch.equal(out, rc.source_terms(rho, T, Y))
+
+
+def test_source_terms_by_several_threads():
+    import threading
+    import torch
+    from gdtk_gb300 import lib
+    from gdtk_gb300.cells import ReactorCells
+    vp = lambda t: ctypes.c_void_p(t.data_ptr())
+    for name in ("j92", "j92", "j92"):   # a fresh reactor each time
+        rc = ReactorCells(mech(name + "-gas.lua"), mech(name + "-chem.lua"))
+        rho, T, Y = _cells(torch, rc)
+        n = 6
+        outs, streams, rcs = [torch.empty_like(Y) for _ in range(n)], [torch.cuda.Stream() for _ in range(n)], [None] * n
+        torch.cuda.synchronize()
+        gate = threading.Barrier(n)
+
+        def call(k):
+            gate.wait()
+            for _ in range(20):
+                rcs[k] = lib().chem_reactor_source_terms_cells(rc.reactor.id, rho.shape[0], vp(rho), vp(T), vp(Y), vp(outs[k]), None,
+                                                               ctypes.c_void_p(streams[k].cuda_stream))
+        threads = [threading.Thread(target=call, args=(k,)) for k in range(n)]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        torch.cuda.synchronize()
+        assert rcs == [0] * n
+        want = rc.source_terms(rho, T, Y)
+        for out in outs:
+            assert torch.equal(out, want)
 
 
 CHILD = """
