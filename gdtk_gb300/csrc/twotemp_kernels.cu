@@ -171,7 +171,7 @@ __device__ void coupling(const Eem2T& e, double rT, double rTv, double& ga, doub
 // 5,900 FP64 instructions per attempt and warp (32 cells), most of them over tables that every lane walked for
 // itself, with 13 of 32 lanes active and a warp waiting for its longest cell; eight lanes issue about 930 for
 // 4 cells, a cell's attempt takes a fifth of the time, and cells are handed out as groups come free.
-// 65,536 non-equilibrium air cells over 2e-7 s: 181 -> 64 ms; one cell 14.4 -> 3.0 ms.  FP64 issue (60% busy at
+// 65,536 non-equilibrium air cells over 2e-7 s: 181 -> 64 ms; one cell 14.4 -> 3.0 ms.  FP64 issue (69% busy at
 // 16,384 cells) and instruction fetch bound it.
 // All groups of a warp stay in step: every sync and shuffle is over the whole warp, in loops uniform over it.
 // The operations per cell are those of the subcycle and attempt loops of
@@ -687,7 +687,8 @@ int grid_for_cells(int n, int block, int sm_count) {
 cudaError_t launch_two_temperature_update(const TwoTArgs& a, int nsp, int nr, int sm_count, cudaStream_t s) {
     if (a.ncell <= 0) return cudaSuccess;
     if (a.neem > MAX_EEM || !a.counter) return cudaErrorInvalidValue;
-    // one block per SM, with as many warps (four cells each) as fit, spread over the SMs
+    // as many blocks per SM as are resident (three of 256 threads), each with as many warps (four cells each) as fit, or
+    // as a share of the batch needs
     constexpr size_t LIMIT = 227 * 1024 - 2 * GDTK_EXP2_TABLE_SIZE * 8;
     const size_t tables = (size_t)(nsp * GDTK_TH_STRIDE + a.neff * nsp + (a.n_tab + 1) / 2) * 8;
     const size_t per_warp = (size_t)Layout2T(nsp, nr, a.ncpl).total * (32 / GL) * 8;
