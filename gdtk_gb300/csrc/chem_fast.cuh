@@ -520,6 +520,9 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
         if (!__any_sync(FULL, alive || have)) break;
         if (have) {
         lane_stat(a.lane_stats, 0);
+        // The third bodies of pressure-dependent rates are those of the input's mass fractions, also of negative ones
+        // (rate_constant.d:114-121); the concentrations are clipped after them.
+        const bool fresh = GDTK_NFALLOFF && phase == -1;
         if (phase == -1) {   // (re)start from the stored input state
             const CellBlock& B = BLK[b];
             T = B.T[ci]; p = B.p[ci]; dtS = dtS0; t = 0.0; err = 0;
@@ -527,7 +530,7 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
 #pragma unroll
             for (int i = 0; i < GDTK_NSP; ++i) {
                 double v = B.massf[(size_t)i * B.ncell + ci] * rho * GDTK_RM[i];
-                y0[i] = (v < MIN_MOLES) ? 0.0 : v;
+                y0[i] = (!GDTK_NFALLOFF && v < MIN_MOLES) ? 0.0 : v;
             }
             need_kc = true;
             phase = 0;
@@ -538,6 +541,10 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
             rate_constants(TH, T, lnT, K, ks, ETAB, V, &err);
             ++n_kc;
             need_kc = false;
+            if (fresh) {
+#pragma unroll
+                for (int i = 0; i < GDTK_NSP; ++i) y0[i] = (y0[i] < MIN_MOLES) ? 0.0 : y0[i];
+            }
         }
         __syncwarp(hm);
         ++n_steps;
@@ -769,7 +776,8 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_c
 // over the interval: 40 x^0.4.  Against the step counts of the update (rank correlation over cells of the H2-air
 // batch, the mixing layer with carried step sizes, and methane at 1e-6 s) the growth limit alone gives 0.78, 0.04
 // and 0.50, x 0.91, 0.95 and 0.92, with 83 to 98% of the longest hundredth in the first twentieth (5%, 4%, 33%).
-// The rates cost about a 500th of an update.
+// The rates cost 0.23 of 123 ms for 65,536 fresh H2-air cells over 1e-6 s, 0.36 of 17 to 20 ms on a 131,072-cell mixing layer
+// with carried steps, and 0.22 of 0.74 ms for 65,536 cells whose carried step covers the interval.
 extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS) gdtk_chem_cost(const __grid_constant__ FastArgs a,
                                                                                      float* key) {
     extern __shared__ double smem[];
@@ -845,11 +853,15 @@ extern "C" __global__ void __launch_bounds__(GDTK_BLOCK, GDTK_MIN_BLOCKS)
 #pragma unroll
             for (int i = 0; i < GDTK_NSP; ++i) {
                 const double v = massf[(size_t)i * n + g] * r * GDTK_RM[i];
-                y[i] = (v < MIN_MOLES) ? 0.0 : v;
+                y[i] = (!GDTK_NFALLOFF && v < MIN_MOLES) ? 0.0 : v;   // clipped after the third bodies, as in the update
             }
             const double Tc = T[g];
             if (GDTK_NFALLOFF) gen_falloff_M(y, V + GDTK_NSP * ks, ks);
             rate_constants(TH, Tc, gdtk_log(Tc), K, ks, ETAB, V, &err);
+            if (GDTK_NFALLOFF) {
+#pragma unroll
+                for (int i = 0; i < GDTK_NSP; ++i) y[i] = (y[i] < MIN_MOLES) ? 0.0 : y[i];
+            }
             gen_rhs(y, q, L, K, ks);
 #pragma unroll
             for (int i = 0; i < GDTK_NSP; ++i) source[(size_t)i * n + g] = (q[i] - L[i]) * GDTK_M[i];

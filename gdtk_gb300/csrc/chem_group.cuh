@@ -250,7 +250,7 @@ __device__ __forceinline__ double grp_ipow(double x, int n) {   // the order of 
 
 #if GDTK_METHOD != 0
 // The q and L sums of the alpha-QSS right-hand side on the integer pipe: a term takes about 22 cycles there, where
-// an FP64 addition takes 76 of the pipe that bounds the kernel (73% busy on the mixing layer), and the
+// an FP64 addition takes 76 of the pipe that bounds the kernel (74% busy with 65,536 cells), and the
 // terms do not wait for one another.  The terms, all >= 0, are aligned to the largest with 5 bits below its last
 // and the sum is rounded once, closer to the exact value than the chain of FP64 additions it replaces.  64 bits hold 64
 // terms of the largest one's size; a longer sum (128 reactions can give one 384 entries) is that chain.
@@ -566,14 +566,16 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
         double* const LO = S + GO_L;
         double* const W = S + GO_W;
         double* const V = S + GO_V;
-        if (__any_sync(GRP_FULL, s.have && s.phase == -1)) {   // (re)start from the stored input state
-            if (s.have && s.phase == -1) {
+        // as in gdtk_chem_fast, the third bodies of pressure-dependent rates see the input's concentrations unclipped
+        const bool start = s.have && s.phase == -1, fresh = GDTK_NFALLOFF && start;
+        if (__any_sync(GRP_FULL, start)) {   // (re)start from the stored input state
+            if (start) {
                 const CellBlock& B = a.blocks[s.b];
                 s.T = B.T[s.ci]; s.p = B.p[s.ci]; s.dtS = s.dtS0; s.t = 0.0; s.err = 0;
                 s.lnT = gdtk_log(s.T);
                 for (int i = gl; i < GDTK_NSP; i += L) {
                     const double v = B.massf[(size_t)i * B.ncell + s.ci] * s.rho * GDTK_RM[i];
-                    Y0[i] = (v < MIN_MOLES) ? 0.0 : v;
+                    Y0[i] = (!GDTK_NFALLOFF && v < MIN_MOLES) ? 0.0 : v;
                 }
                 s.need_kc = true;
                 s.phase = 0;
@@ -585,6 +587,11 @@ __device__ __forceinline__ bool grp_loop(const FastArgs& a, const GrpTab& tab, G
             if (__any_sync(GRP_FULL, k)) {
                 grp_rate_constants<L>(tab, s, gl, k);
                 if (k) { ++s.n_kc; s.need_kc = false; }
+            }
+            if (GDTK_NFALLOFF && __any_sync(GRP_FULL, fresh)) {
+                if (fresh)
+                    for (int i = gl; i < GDTK_NSP; i += L) Y0[i] = (Y0[i] < MIN_MOLES) ? 0.0 : Y0[i];
+                __syncwarp(GRP_FULL);
             }
         }
         const bool act = s.have;
