@@ -441,8 +441,8 @@ __global__ void __launch_bounds__(UPDATE_BLOCK, 3) two_temperature_update_kernel
                 h = dt_suggest > tI ? tI : dt_suggest <= 0.0 ? fmax(fmin(1.0e-3 * md, 1.0e-10), 1.0e-15) : dt_suggest;
                 phase = 1;
             }
-            if (setup) {   // partial pressures, number densities, Y (e_ve(T) - e_ve(T_ve))
-                const double rmol = gdtk_rcp(mol) * (p * (1.0 / P_atm));
+            if (setup) {   // mole fractions, number densities, Y (e_ve(T) - e_ve(T_ve))
+                const double rmol = gdtk_rcp(mol);
                 for (int i = gl; i < nsp; i += GL) {
                     const double n_i = Y[i] * (R(i) * R_INV);
                     xa[i] = n_i * rmol;
@@ -458,15 +458,16 @@ __global__ void __launch_bounds__(UPDATE_BLOCK, 3) two_temperature_update_kernel
             __syncwarp(FULL);
             double lt = 0.0;
             if (setup) {
-                const double small = SMALL_MOLE_FRACTION * (p * (1.0 / P_atm));
+                const double patm = p * (1.0 / P_atm);
                 const double htc2 = sqrtT * (50e3 * rT) * (50e3 * rT);
                 for (int k = gl; k < a.neem; k += GL) {
                     const Eem2T& e = a.eem[k];
                     if (e.kind == EEM_LANDAU_TELLER) {   // relaxation_time.d:27-175; a rare collider has none
-                        if (gt_pos(xa[e.q], small)) {
-                            double tau = gdtk_div(ex(fma(e.a, T13, -e.b)), xa[e.q]);   // xa: partial pressure in atm
+                        if (gt_pos(xa[e.q], SMALL_MOLE_FRACTION)) {
+                            double tau = gdtk_div(ex(fma(e.a, T13, -e.b)), xa[e.q] * patm);   // the partial pressure in atm
                             if (e.rt != RT_MILLIKAN_WHITE) tau += gdtk_rcp(e.sigma * xb[e.q] * (e.rt == RT_PARK_HTC ? sqrtT : htc2));
-                            lt += gdtk_div(de[e.p], tau);
+                            // a negative time or none (at T <= 0) relaxes nothing
+                            if ((unsigned long long)__double_as_longlong(tau) <= 0x7ff0000000000000ull) lt += gdtk_div(de[e.p], tau);
                         }
                     } else {
                         double g0, g1;
