@@ -1086,8 +1086,8 @@ def main():
     ap.add_argument("--no-surrogate", action="store_true", help="leave out the surrogate + fallback object")
     ap.add_argument("--no-blocks", action="store_true", help="leave out the 64-block batch object")
     ap.add_argument("--lane-stats", action="store_true",
-                    help="after the timed region, one more update with the kernel's lane statistics attached; "
-                         "with GDTK_PHASE_CLOCKS=1 in the environment the line also gets each phase's share of "
+                    help="after the timed region, one more update with lane statistics attached, by the kernel of one "
+                         "thread per cell, which alone has them; with GDTK_PHASE_CLOCKS=1 in the environment the line also gets each phase's share of "
                          "warp time")
     args = ap.parse_args()
     # the timed kernel is never the phase-clock build: that one is generated only for the untimed
